@@ -638,8 +638,8 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
     // that the lane-per-row writes spread over the banks) and leaves with one TMA store, which
     // also clips at M and N.
     const int q = warp & 3;  // tensor-memory lane quarter this warp may read
-    const float scale_a = p.alpha * (p.ga ? __ldg(p.ga) : 1.0f);
-    const float scale_ab = scale_a * ((p.gb && p.gb_group == 0) ? __ldg(p.gb) : 1.0f);
+    const float scale_a = p.alpha * (p.ga ? load_f32(p.ga) : 1.0f);
+    const float scale_ab = scale_a * ((p.gb && p.gb_group == 0) ? load_f32(p.gb) : 1.0f);
     const uint32_t lead_acc_empty0 = mapa_u32(acc_empty_bar(0), 0);
     const uint32_t lead_acc_empty1 = mapa_u32(acc_empty_bar(1), 0);
     const uint32_t on = elect_one();
@@ -729,12 +729,12 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
 #pragma unroll
           for (int g = 0; g < 8; ++g)
             bb[g] = col0 + g * 8 < p.N
-                        ? __ldg(reinterpret_cast<const uint4*>(p.bias + col0 + g * 8))
+                        ? load_u32x4(p.bias + col0 + g * 8)
                         : make_uint4(0, 0, 0, 0);
         }
         // stacked weights: the tensor scale of the weight this group's columns belong to
         const float scale = (p.gb_group > 0 && col0 < p.N)
-                                ? scale_a * __ldg(p.gb + col0 / p.gb_group) : scale_ab;
+                                ? scale_a * load_f32(p.gb + col0 / p.gb_group) : scale_ab;
         if (!p.c) {
           // the previous store must have finished reading the slab
           asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
@@ -771,8 +771,8 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
             for (int e = 0; e < 4; ++e) v[e] = gelu_tanh2(v[e]);
           }
           if (p.gate && in_n) {
-            const float4 g0 = __ldg(reinterpret_cast<const float4*>(p.gate + col0 + g * 8));
-            const float4 g1 = __ldg(reinterpret_cast<const float4*>(p.gate + col0 + g * 8 + 4));
+            const float4 g0 = load_f32x4(p.gate + col0 + g * 8);
+            const float4 g1 = load_f32x4(p.gate + col0 + g * 8 + 4);
             v[0] = f2_mul(v[0], make_float2(g0.x, g0.y));
             v[1] = f2_mul(v[1], make_float2(g0.z, g0.w));
             v[2] = f2_mul(v[2], make_float2(g1.x, g1.y));

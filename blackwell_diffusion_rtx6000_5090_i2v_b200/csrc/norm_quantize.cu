@@ -80,7 +80,7 @@ struct NormArgs {
 __device__ __forceinline__ void load16(const float* p, float2 (&d)[8]) {
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(p) + q);
+    const float4 a = load_f32x4(p + 4 * q);
     d[2 * q] = make_float2(a.x, a.y);
     d[2 * q + 1] = make_float2(a.z, a.w);
   }
@@ -274,7 +274,7 @@ norm_mod_kernel(const NormArgs p) {
   grid_dependency_wait();
   float s_enc = 0.0f;
   if (kQuantize) {
-    s_enc = global_encode_scale(__ldg(p.amax_in));
+    s_enc = global_encode_scale(load_f32(p.amax_in));
     const float s_dec = __fdiv_rn(1.0f, s_enc);
     if (p.gscale_out && blockIdx.x == 0 && threadIdx.x == 0) *p.gscale_out = s_dec;
     // the encode scale depends on the block only through its scale byte: tabulate it
@@ -328,7 +328,7 @@ norm_mod_kernel(const NormArgs p) {
 #pragma unroll
     for (int r = 0; r < kR; ++r) {
       const int64_t rr = base + r < p.rows ? base + r : base;
-      const float2 st = __ldg(reinterpret_cast<const float2*>(p.stats) + rr);
+      const float2 st = load_f32x2(p.stats + 2 * rr);
       mean_n[r] = st.x;
       rstd_n[r] = st.y;
     }

@@ -176,6 +176,43 @@ __device__ __forceinline__ uint32_t quad_transpose(uint32_t w) {
   return __byte_perm(w, __shfl_xor_sync(0xffffffffu, w, 2), (lane & 2) ? 0x3276u : 0x5410u);
 }
 
+// A kernel launched by launch_dependent() may start while the kernel before it in its stream is still
+// finishing.  This waits until everything before it has completed and is visible; what a kernel
+// does ahead of it (barriers, tensor-memory allocation, index arithmetic) touches no global memory
+// that another kernel writes or reads.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Loads for such a kernel.  Not __ldg and the like: those are non-coherent loads, for memory that
+// stays read-only from the kernel's start to its end, which a predecessor's output is not, and nothing
+// keeps them behind the wait.  These are ordinary loads, and as volatile statements they stay in
+// order with it.  (`_once`: data with no second reader.)
+__device__ __forceinline__ uint32_t load_u32(const void* p) {
+  uint32_t v;
+  asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float load_f32(const float* p) { return __uint_as_float(load_u32(p)); }
+__device__ __forceinline__ float2 load_f32x2(const void* p) {
+  float2 v;
+  asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float4 load_f32x4(const void* p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint4 load_u32x4(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint4 load_u32x4_once(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.cs.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
 // 32 bytes of x that are read once: one 256-bit load where the address allows, else two of 128.
 __device__ __forceinline__ void load_block_once(const uint4* src, bool wide, uint32_t (&x)[8]) {
   if (wide) {
@@ -183,20 +220,14 @@ __device__ __forceinline__ void load_block_once(const uint4* src, bool wide, uin
                  : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]), "=r"(x[7])
                  : "l"(src));
   } else {
-    const uint4 a = __ldcs(src), b = __ldcs(src + 1);
+    const uint4 a = load_u32x4_once(src), b = load_u32x4_once(src + 1);
     x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
     x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
   }
 }
 
-// A kernel launched by launch_dependent() may start while the kernel before it in its stream is still
-// finishing.  This waits until everything before it has completed and is visible; what a kernel
-// does ahead of it (barriers, tensor-memory allocation, index arithmetic) touches no global memory
-// that another kernel writes or reads.
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // Launch with programmatic stream serialization: the launch latency and the prologue of `kernel`
-// overlap the tail of its predecessor.  The kernel calls grid_dependency_wait().  `cluster`: CTAs per
+// overlap the tail of its predecessor.  The kernel calls grid_dependency_wait() and loads as above.  `cluster`: CTAs per
 // cluster along x.  Amax + pack of [27280, 3072] 67.7 -> 64.0 us, norm + quantize 98.0 -> 94.5 us, RoPE
 // 127.8 -> 126.2 us, a [4095, 5120] x 5120 GEMM 67.8 -> 66.3 us, each called back to back.
 template <typename... Params, typename... Args>

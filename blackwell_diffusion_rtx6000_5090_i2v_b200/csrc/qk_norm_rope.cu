@@ -96,7 +96,7 @@ __device__ __forceinline__ uint4 norm_rotate(const uint4& v, float2 r2, const fl
   if (gain) {
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-      const float4 t = __ldg(reinterpret_cast<const float4*>(gain) + q);
+      const float4 t = load_f32x4(gain + 4 * q);
       g[2 * q] = make_float2(t.x, t.y);
       g[2 * q + 1] = make_float2(t.z, t.w);
     }
@@ -143,12 +143,12 @@ __global__ void __launch_bounds__(kThreads, 2) rope_warp_kernel(const RopeArgs p
 #pragma unroll
     for (int j = 0; j < kN; ++j) {
       const int c = lane + j * 32;
-      v[j] = c < chunks ? __ldcs(src + c) : make_uint4(0, 0, 0, 0);
+      v[j] = c < chunks ? load_u32x4_once(src + c) : make_uint4(0, 0, 0, 0);
     }
     float4 cs[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
     if (rotate && one_entry) {
-      cs[0] = __ldg(table + 2 * (lane % per_head));
-      cs[1] = __ldg(table + 2 * (lane % per_head) + 1);
+      cs[0] = load_f32x4(table + 2 * (lane % per_head));
+      cs[1] = load_f32x4(table + 2 * (lane % per_head) + 1);
     }
     float rstd = 0.0f;
     if (which < 2) {
@@ -173,8 +173,8 @@ __global__ void __launch_bounds__(kThreads, 2) rope_warp_kernel(const RopeArgs p
       if (c >= chunks) break;
       if (which < 2) {
         if (rotate && !one_entry) {
-          cs[0] = __ldg(table + 2 * (c % per_head));
-          cs[1] = __ldg(table + 2 * (c % per_head) + 1);
+          cs[0] = load_f32x4(table + 2 * (c % per_head));
+          cs[1] = load_f32x4(table + 2 * (c % per_head) + 1);
         }
         v[j] = norm_rotate(v[j], r2, gain ? gain + 8 * c : nullptr, rotate, cs);
       }
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(512) rope_cta_kernel(const RopeArgs p) {
     const float4* table = reinterpret_cast<const float4*>(p.cos_sin + row * half_hd);
     uint4 v[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = dst[k] ? __ldcs(src + threadIdx.x + k * T) : make_uint4(0, 0, 0, 0);
+    for (int k = 0; k < 4; ++k) v[k] = dst[k] ? load_u32x4_once(src + threadIdx.x + k * T) : make_uint4(0, 0, 0, 0);
     float rstd = 0.0f;
     if (which < 2) {
       float2 s2 = make_float2(0.0f, 0.0f);
@@ -239,8 +239,8 @@ __global__ void __launch_bounds__(512) rope_cta_kernel(const RopeArgs p) {
       if (which < 2) {
         float4 cs[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
         if (rotate) {
-          cs[0] = __ldg(table + 2 * (c % per_head));
-          cs[1] = __ldg(table + 2 * (c % per_head) + 1);
+          cs[0] = load_f32x4(table + 2 * (c % per_head));
+          cs[1] = load_f32x4(table + 2 * (c % per_head) + 1);
         }
         v[k] = norm_rotate(v[k], r2, gain ? gain + 8 * c : nullptr, rotate, cs);
       }

@@ -22,23 +22,23 @@ constexpr int kBlocksPerThread = 2;  // two 16-element scale blocks (64 B of inp
 // ---------------------------------------------------------------- amax ----
 
 // kPartial: every CTA leaves its own maximum in out[blockIdx.x] for the packing kernel to combine,
-// so that no slot has to be zeroed first; else one atomic per CTA on the zeroed slot.
+// so that no slot has to be zeroed first, and launched by launch_dependent(); else one atomic per CTA
+// on the zeroed slot.
 template <bool kPartial>
-__global__ void __launch_bounds__(kThreads) amax_bf16_kernel(const uint4* __restrict__ x,
-                                                             int64_t n_vec,
-                                                             const __nv_bfloat16* __restrict__ tail,
-                                                             int n_tail, unsigned* __restrict__ out) {
+__global__ void __launch_bounds__(kThreads) amax_bf16_kernel(const uint4* x, int64_t n_vec,
+                                                             const __nv_bfloat16* tail, int n_tail,
+                                                             unsigned* out) {
   __nv_bfloat162 m2[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) m2[j] = __nv_bfloat162(__float2bfloat16(0.f), __float2bfloat16(0.f));
-  grid_dependency_wait();
+  if (kPartial) grid_dependency_wait();
   const int64_t stride = (int64_t)gridDim.x * kThreads;
   int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
   // four independent 16-byte loads in flight per thread
   for (; i + 3 * stride < n_vec; i += 4 * stride) {
     uint4 v[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = __ldg(x + i + j * stride);
+    for (int j = 0; j < 4; ++j) v[j] = load_u32x4(x + i + j * stride);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v[j]);
@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(kThreads) amax_bf16_kernel(const uint4* __rest
     }
   }
   for (; i < n_vec; i += stride) {
-    uint4 v = __ldg(x + i);
+    uint4 v = load_u32x4(x + i);
     const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v);
 #pragma unroll
     for (int k = 0; k < 4; ++k) m2[k] = __hmax2(m2[k], __habs2(p[k]));
@@ -81,7 +81,6 @@ quantize_bf16_kernel(const uint4* __restrict__ x, uint32_t n_blocks, uint32_t kb
                      uint2* __restrict__ packed, uint8_t* __restrict__ sf_lin,
                      uint8_t* __restrict__ sf_swz, uint32_t k_atoms,
                      float* __restrict__ global_scale_out) {
-  grid_dependency_wait();
   const float amax_g = amax_ptr ? __ldg(amax_ptr) : amax_val;
   const float s_enc = global_encode_scale(amax_g);
   const float s_dec = __fdiv_rn(1.0f, s_enc);
@@ -181,7 +180,7 @@ __global__ void __launch_bounds__(kPackThreads, 4) pack_rows_kernel(const PackAr
   float amax_g;
   if (p.partial) {
     unsigned m = 0u;
-    for (int i = threadIdx.x; i < p.n_partial; i += blockDim.x) m = max(m, __ldg(p.partial + i));
+    for (int i = threadIdx.x; i < p.n_partial; i += blockDim.x) m = max(m, load_u32(p.partial + i));
     m = __reduce_max_sync(0xffffffffu, m);
     if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = m;
     __syncthreads();
@@ -189,7 +188,7 @@ __global__ void __launch_bounds__(kPackThreads, 4) pack_rows_kernel(const PackAr
     amax_g = __uint_as_float(m);
     if (scribe) *p.amax_out = amax_g;
   } else {
-    amax_g = p.amax ? __ldg(p.amax) : p.amax_val;
+    amax_g = p.amax ? load_f32(p.amax) : p.amax_val;
   }
   const float s_enc = global_encode_scale(amax_g);
   const float s_dec = __fdiv_rn(1.0f, s_enc);
@@ -252,7 +251,7 @@ constexpr int64_t kSmallMax = (int64_t)kSmallCtas * kSmallThreads * kSmallBlocks
 
 template <int kB>
 __global__ void __launch_bounds__(kSmallThreads)
-quantize_small_kernel(const uint4* __restrict__ x, uint32_t n_blocks, uint32_t kb_per_row, int wide_x,
+quantize_small_kernel(const uint4* x, uint32_t n_blocks, uint32_t kb_per_row, int wide_x,
                       float* __restrict__ amax_out, uint2* __restrict__ packed,
                       uint8_t* __restrict__ sf_lin, uint8_t* sf_swz, uint32_t swz_vecs,
                       uint32_t k_atoms, float* __restrict__ gscale_out) {

@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(kThreads, 4) quantize_transposed_kernel(const 
   __shared__ __align__(16) uint32_t tile[kTileRows * kTileCols / 2];
   __shared__ float enc_tab[128];
   grid_dependency_wait();
-  const float s_enc = global_encode_scale(__ldg(p.amax));
+  const float s_enc = global_encode_scale(load_f32(p.amax));
   const float s_dec = __fdiv_rn(1.0f, s_enc);
   if (p.gscale_out && blockIdx.x == 0 && threadIdx.x == 0) *p.gscale_out = s_dec;
   fill_encode_table(enc_tab, s_dec);
@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(kThreads, 4) quantize_transposed_kernel(const 
     for (int j = 0; j < 4; ++j) {
       const int i = threadIdx.x + j * kThreads;            // 16-byte piece of the tile
       const int64_t r = row0 + (i >> 3), c = col0 + (i & 7) * 8;
-      v[j] = r < p.rows && c < p.cols ? __ldg(reinterpret_cast<const uint4*>(p.x + (r * p.cols + c) * 2))
+      v[j] = r < p.rows && c < p.cols ? load_u32x4(p.x + (r * p.cols + c) * 2)
                                       : make_uint4(0, 0, 0, 0);
     }
     __syncthreads();     // the previous tile has been read
