@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import contextlib
 import ctypes as C
+import functools
 import os
 
 import torch
@@ -96,14 +97,16 @@ def device_guard(device: torch.device):
     return _nothing if device.index == torch._C._cuda_getDevice() else torch.cuda.device(device)
 
 
+# The library's own answers, remembered for the last shapes: the layout has one definition, and a call
+# that runs every step does not cross into the library for it.
+@functools.lru_cache(maxsize=1024)
 def linear_workspace_bytes(rows: int, cols: int) -> int:
-    """``nvfp4_linear_workspace_bytes`` without the call."""
-    return (rows * cols // 2 + 255) // 256 * 256 + swizzled_scale_bytes(rows, cols) + 256 + 4 * AMAX_PARTIALS
+    return lib.nvfp4_linear_workspace_bytes(rows, cols)
 
 
+@functools.lru_cache(maxsize=1024)
 def swizzled_scale_bytes(rows: int, cols: int) -> int:
-    """``nvfp4_swizzled_scale_bytes`` without the call."""
-    return ((rows + 255) // 256 * 2) * ((cols // 16 + 15) // 16 * 4) * 512
+    return lib.nvfp4_swizzled_scale_bytes(rows, cols)
 
 
 def ptr(t: torch.Tensor | None):

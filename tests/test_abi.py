@@ -40,6 +40,26 @@ def test_swizzled_bytes_formula():
     assert f(300, 320) == 4 * 8 * 512
 
 
+def test_sizes_have_one_definition():
+    """Buffers that a call without a size argument fills: the sizes that Python allocates are the
+    library's, for any shape and any change of layout there."""
+    from unittest import mock
+    from blackwell_diffusion_rtx6000_5090_i2v_b200 import _native
+    L = _native.lib
+    for rows in (1, 2, 127, 128, 129, 255, 256, 257, 4095, 27280):
+        for cols in (16, 32, 48, 240, 256, 272, 3072, 3088, 14336):
+            assert _native.swizzled_scale_bytes(rows, cols) == L.nvfp4_swizzled_scale_bytes(rows, cols)
+            assert _native.linear_workspace_bytes(rows, cols) == L.nvfp4_linear_workspace_bytes(rows, cols)
+    with mock.patch.object(_native, "lib", mock.Mock()) as fake:
+        fake.nvfp4_swizzled_scale_bytes.return_value = 7
+        fake.nvfp4_linear_workspace_bytes.return_value = 8
+        assert _native.swizzled_scale_bytes(3, 16 * 1000003) == 7
+        assert _native.linear_workspace_bytes(3, 32 * 1000003) == 8
+    _native.swizzled_scale_bytes.cache_clear()
+    _native.linear_workspace_bytes.cache_clear()
+    assert f"#define NVFP4_AMAX_PARTIALS {_native.AMAX_PARTIALS}\n" in open(HEADER).read()
+
+
 def test_argument_validation_without_device():
     from blackwell_diffusion_rtx6000_5090_i2v_b200 import _native
     L = _native.lib
