@@ -49,14 +49,6 @@ def quantized_weight(weight: torch.Tensor) -> FP4Tensor:
     return q
 
 
-def _known_weight_amax(weight: torch.Tensor) -> Optional[torch.Tensor]:
-    """max|weight| of the packed copy, if there is one of this version of the tensor."""
-    hit = _weight_cache.get(id(weight))
-    if hit is not None and hit[0]() is weight and hit[1] == weight._version and hit[2] == weight.data_ptr():
-        return hit[3].global_amax()
-    return None
-
-
 def _transposable(t: torch.Tensor) -> bool:
     # what the transposing quantizer reads in place; the rest goes through a transposed copy
     return t.is_contiguous() and t.numel() > 0 and t.size(1) % 8 == 0 and t.data_ptr() % 16 == 0
@@ -256,13 +248,14 @@ def backward(grad_output: torch.Tensor, input: torch.Tensor, weight: torch.Tenso
         if one_dw:
             grad_weight = torch.empty((out_features, in_features), dtype=torch.bfloat16, device=dev)
         k = weight.size(1) if one_dx else in_features
-        w_amax = _known_weight_amax(weight) if one_dx else None
         with N.device_guard(dev):
             ws = torch.empty(N.lib.nvfp4_linear_backward_workspace_bytes(m, out_features, k),
                              dtype=torch.uint8, device=dev)
+            # the maximum of the weight is taken here, not from the forward's packed copy: a write
+            # through weight.data would leave that one behind
             N.check(N.lib.nvfp4_linear_backward_bf16(
                 go.data_ptr(), x2.data_ptr() if one_dw else None, weight.data_ptr() if one_dx else None,
-                N.ptr(w_amax), m, out_features, k, N.ptr(grad_input), N.ptr(grad_weight), ws.data_ptr(),
+                None, m, out_features, k, N.ptr(grad_input), N.ptr(grad_weight), ws.data_ptr(),
                 N.status_word(dev).data_ptr(), N.stream_ptr()), "[linear] backward")
         if one_dx:
             grad_input = grad_input.reshape(input.shape)

@@ -50,3 +50,8 @@ def test_gradients_equal_the_products_on_copies(m, n, k):
     w.mul_(3)
     dx3 = lc.backward(go, x, w, one, one, one, True, False, False)[0]
     assert torch.equal(dx3, lc.gemm(go, w.t().contiguous()))
+    # also when the change went past the version count
+    lc.quantized_weight(w)
+    w.data.mul_(4)
+    dx12 = lc.backward(go, x, w, one, one, one, True, False, False)[0]
+    assert torch.equal(dx12, lc.gemm(go, w.t().contiguous()))
