@@ -14,19 +14,17 @@
 // The two query tiles alternate on the tensor pipe: while the threads of one tile run the
 // softmax, the MMAs of the other tile execute.
 //
-// The reference m of a row is the exact maximum of its first key tile and from then on follows the
-// row sums instead of a maximum of every tile: any reference gives the same quotient, as long as
-// nothing overflows (bf16 and fp32 reach 2^127) and the row's largest terms do not vanish.  A thread
-// leaves its sum over a key tile in shared memory; at the next tile both threads of the row see
-// both sums -- no barrier of their own: each wrote before it handed over P, which precedes the S
-// they then wait for -- and where one exceeds 2^8 both raise m by the same amount and
-// rescale their halves of O, which is at rest then: the S tile they hold was committed after the
-// previous P V product of the same query tile had completed.  A sum above 2^100 within ONE
-// tile (logits 69 nats above everything before them), or an O that overflowed all the same (values
-// of v beyond 2^20 beside such a leap), ends the attempt: the CTA runs a second time with the exact
-// maximum of every tile.
-// [27280, 24, 128]: 7123 -> 6649 us (1284 -> 1375 TFLOP/s); [32760, 5, 128]: 2554 -> 2386 us; q, k and v
-// from a Student-t(4), [27280, 24, 128]: 7.07 -> 6.72 ms (8.0 ms with the line drawn at 2^32).
+// The reference m of a row is its running maximum, raised only when a tile exceeds it by more than
+// 2^8; the two threads of a row exchange the maxima of their halves at every tile.  (A reference that
+// follows the row sums of earlier tiles needs neither the maximum nor the exchange: 6.75 against 7.05
+// ms at [27280, 24, 128] with N(0, 1) inputs.  But a key far above all before it then weighs 2^x rounded
+// to bf16 where it should weigh exactly 1, or overflows and sends the CTA through all keys again: with
+// q, k and v from a Student-t(4) distribution 8.7 against 7.5 ms, and an error of 2.3e-3.)
+// The row sum adds the probabilities as they are rounded for the product, so that numerator and
+// denominator agree; adding a bf16 to an fp32 is one instruction.  Against the sum of the unrounded
+// ones, relative error against 64 bits with Student-t(4) inputs 1.82e-3 -> 1.67e-3, with N(0, 1) 2.35e-3
+// either way.  The four partial sums of a thread are joined at the end, not at every tile:
+// [27280, 24, 128] 7.21 -> 7.05 ms (1320 TFLOP/s), [32760, 5, 128] 2.6 ms either way.
 //
 // Tensor memory (512 columns): S0/P0 at 0, S1/P1 at 128, O0 at 256, O1 at 384.
 // Shared memory: Q0, Q1 (32 KiB each), a ring of four 32 KiB K/V tiles (K0 V0 K1 V1 ...),
@@ -60,16 +58,11 @@ constexpr int kDataBytes = (kQTiles + kKvSlots) * kTileBytes;
 constexpr int kSmemBytes = kDataBytes + 1024 /*align slack*/ + 256 /*barriers*/ + 4096 /*row exchange*/;
 constexpr int kSoftmaxWarps = 16;         // eight per query tile
 constexpr int kLoaderWarp = 16, kIssuerWarp = 17;
-// 18 warps and no more: 65536 registers are 112 for each thread then, which the softmax needs (64
-// logits and what it keeps beside them); 20 warps would leave 96 and spill.
-constexpr int kThreads = 576;
+constexpr int kThreads = 576;             // 96 registers each, no spills
 constexpr int kXchgBytes = kQTiles * 2 * 2 * kBQ * 4;   // [tile][parity][half][row] floats
 constexpr int kTmemCols = 512;
 constexpr int kColS = 0, kColO = 256;     // + 128 * tile
-constexpr float kRescaleStep = 8.f;       // exact mode: raise the running maximum only past 2^8
-constexpr float kRaiseSum = 256.f;        // raise the reference when a tile's sum exceeds 2^8
-constexpr float kRedoLog2 = 100.f;        // a term or sum above 2^100 is left to the exact mode
-constexpr float kRedoSum = 1.2676506e30f;
+constexpr float kRescaleStep = 8.f;       // raise the running maximum only past 2^8
 #ifndef NVFP4_ATTN_FMA_EXP_EVERY
 #define NVFP4_ATTN_FMA_EXP_EVERY 4
 #endif
@@ -256,6 +249,14 @@ __device__ __forceinline__ float2 exp2_fma(float2 x) {
   return y;
 }
 
+// acc + the two bf16 of a word, in fp32 (mixed-precision add, sm_100)
+__device__ __forceinline__ float2 add_bf16x2(uint32_t w, float2 acc) {
+  asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %2;\n\t"
+      "add.f32.bf16 %0, lo, %0;\n\tadd.f32.bf16 %1, hi, %1;\n\t}"
+      : "+f"(acc.x), "+f"(acc.y) : "r"(w));
+  return acc;
+}
+
 // Shared-memory matrix descriptors, 128-byte swizzle (layout code 2, descriptor version 1).
 // K-major operand (Q, K: rows of 64 contraction elements = 128 bytes): 8-row groups 1024 bytes
 // apart (stride offset); the leading offset is unused.
@@ -288,7 +289,6 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   const uint32_t bar_base = smem_base + kDataBytes;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + kDataBytes + 248);
-  volatile int* redo_flag = reinterpret_cast<volatile int*>(smem_gen + kDataBytes + 244);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_gen + kDataBytes + 252);
   auto q_smem = [&](int t) { return smem_base + (uint32_t)t * kTileBytes; };
   auto kv_smem = [&](int s) { return smem_base + (uint32_t)(kQTiles + s) * kTileBytes; };
@@ -298,7 +298,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   auto s_full = [&](int t) { return bar_base + 8u * (1 + 2 * kKvSlots + t); };
   auto p_full = [&](int t) { return bar_base + 8u * (3 + 2 * kKvSlots + t); };
   auto o_full = [&](int t) { return bar_base + 8u * (5 + 2 * kKvSlots + t); };
-  static_assert(8 * (7 + 2 * kKvSlots) <= 244, "barriers overrun their area");
+  static_assert(8 * (7 + 2 * kKvSlots) <= 248, "barriers overrun their area");
   float* xchg = reinterpret_cast<float*>(smem_gen + kDataBytes + 256);
   static_assert(kXchgBytes <= 4096, "row exchange overruns its area");
 
@@ -320,7 +320,6 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       mbar_init(o_full(t), 1);
     }
     *abort_flag = 0;
-    *redo_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -347,245 +346,194 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   auto xslot = [&](int parity, int h) -> volatile float* { return xchg + ((t * 2 + parity) * 2 + h) * kBQ + r; };
   float l = 0.f;
   bool ok = true;
-  // pass 0 follows the sums, pass 1 (rare) takes the exact maximum of every tile
-#pragma unroll 1
-  for (int pass = 0;; ++pass) {
-    const int kv0 = pass * 2 * n, tile0 = pass * n;   // the ring and the barriers count on
-    if (warp == kLoaderWarp) {
-      // --------------------------------------------------------- loader ----
-      const uint32_t on = elect_one();
-      if (pass == 0) {
-        mbar_expect_tx(q_full(), kQTiles * kTileBytes, on);
-        for (int qt = 0; qt < kQTiles; ++qt)
-          for (int h = 0; h < 2; ++h)
-            tma_load_3d(&map_q, q_full(), q_smem(qt) + h * kHalfBytes, h * 64, head,
-                        (int)(q0 + qt * kBQ), on);
-      }
-      for (int j = 0; j < 2 * n; ++j) {
-        const int i = kv0 + j;
-        const int s = i & (kKvSlots - 1);
-        if (i >= kKvSlots) {
-          ok = mbar_wait(kv_empty(s), (uint32_t)((i / kKvSlots) + 1) & 1u, abort_flag, p.status,
-                         kErrBase + 0x30 + s);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-        }
-        const CUtensorMap* map = (j & 1) ? &map_v : &map_k;
-        mbar_expect_tx(kv_full(s), kTileBytes, on);
-        for (int h = 0; h < 2; ++h)
-          tma_load_3d(map, kv_full(s), kv_smem(s) + h * kHalfBytes, h * 64, head, (j >> 1) * kBKV, on);
-      }
-      if (!ok) {
-        // let copies already in flight land before the CTA's memory is released
-        const long long t0 = clock64();
-        while (clock64() - t0 < 2000000LL) {
-        }
-      }
-    } else if (warp == kIssuerWarp) {
-      // ----------------------------------------------------- MMA issuer ----
-      const uint32_t on = elect_one();
-      const uint32_t idesc_s = make_idesc(false);
-      const uint32_t idesc_pv = make_idesc(true);
-      auto issue_s = [&](int qt, int slot) {
-        // S = Q K^T: eight steps of 16 contraction elements (32 bytes inside the swizzled row,
-        // the second 64 elements one half tile further)
-#pragma unroll
-        for (int ks = 0; ks < kD / 16; ++ks) {
-          const uint32_t off = (uint32_t)(ks >> 2) * kHalfBytes + (uint32_t)(ks & 3) * 32u;
-          tc_mma_ss(tmem_base + kColS + qt * 128, desc_kmajor(q_smem(qt) + off),
-                    desc_kmajor(kv_smem(slot) + off), idesc_s, ks > 0, on);
-        }
-        tc_commit(s_full(qt), on);
-      };
-      const int s0 = kv0 & (kKvSlots - 1);
-      ok = mbar_wait(q_full(), 0, abort_flag, p.status, kErrBase + 0x10);
-      if (ok) ok = mbar_wait(kv_full(s0), (uint32_t)(kv0 / kKvSlots) & 1u, abort_flag, p.status, kErrBase + 0x20);
-      ok = __all_sync(0xffffffffu, ok);
-      if (ok) {
-        tc_fence_after();
-        issue_s(0, s0);
-        issue_s(1, s0);
-        tc_commit(kv_empty(s0), on);
-      }
-      for (int j = 0; ok && j < n; ++j) {
-        const int iv = kv0 + 2 * j + 1, ik = kv0 + 2 * j + 2;
-        const int sv = iv & (kKvSlots - 1), sk = ik & (kKvSlots - 1);
-        const bool has_next = j + 1 < n;
-        ok = mbar_wait(kv_full(sv), (uint32_t)(iv / kKvSlots) & 1u, abort_flag, p.status,
-                       kErrBase + 0x20 + sv);
-        if (ok && has_next)
-          ok = mbar_wait(kv_full(sk), (uint32_t)(ik / kKvSlots) & 1u, abort_flag, p.status,
-                         kErrBase + 0x20 + sk);
+  if (warp == kLoaderWarp) {
+    // --------------------------------------------------------- loader ----
+    const uint32_t on = elect_one();
+    mbar_expect_tx(q_full(), kQTiles * kTileBytes, on);
+    for (int qt = 0; qt < kQTiles; ++qt)
+      for (int h = 0; h < 2; ++h)
+        tma_load_3d(&map_q, q_full(), q_smem(qt) + h * kHalfBytes, h * 64, head,
+                    (int)(q0 + qt * kBQ), on);
+    for (int i = 0; i < 2 * n; ++i) {
+      const int s = i & (kKvSlots - 1);
+      if (i >= kKvSlots) {
+        ok = mbar_wait(kv_empty(s), (uint32_t)((i / kKvSlots) + 1) & 1u, abort_flag, p.status,
+                       kErrBase + 0x30 + s);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        for (int qt = 0; qt < kQTiles; ++qt) {
-          ok = mbar_wait(p_full(qt), (uint32_t)(tile0 + j) & 1u, abort_flag, p.status, kErrBase + 0x50 + qt);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-          tc_fence_after();
-          // O += P V: sixteen keys per step = eight 32-bit columns of P (the first four steps' at the
-          // start of the first half of S, the others' at the start of the second), two 8-key
-          // groups of V
-#pragma unroll
-          for (int ks = 0; ks < kBKV / 16; ++ks)
-            tc_mma_ts(tmem_base + kColO + qt * 128,
-                      tmem_base + kColS + qt * 128 + (ks >> 2) * 64 + (ks & 3) * 8,
-                      desc_mnmajor(kv_smem(sv) + (uint32_t)ks * 2048u), idesc_pv, (j > 0 || ks > 0), on);
-          if (has_next)
-            issue_s(qt, sk);
-          else
-            tc_commit(o_full(qt), on);
-        }
-        if (!ok) break;
-        tc_commit(kv_empty(sv), on);
-        if (has_next) tc_commit(kv_empty(sk), on);
       }
-    } else {
-      // ------------------------------------------------------- softmax ----
-      const float c = p.scale_log2;
-      float m_ref = 0.f, own_sum = 0.f;
-      bool lost = false;                       // a term or sum of this thread went past 2^100
-      l = 0.f;
-      for (int j = 0; j < n; ++j) {
-        ok = mbar_wait(s_full(t), (uint32_t)(tile0 + j) & 1u, abort_flag, p.status, kErrBase + 0x40 + t);
-        ok = __all_sync(0xffffffffu, ok);
-        const bool meet = pass > 0 || j == 0;  // the two threads of a row exchange exact maxima
-        if (!ok) {
-          // The partner warp may have seen this barrier flip a moment before the abort flag went
-          // up and be on its way to this key tile's meeting point, which has no time limit of its
-          // own: arrive there without waiting, so that it gets through.  It cannot reach the next
-          // meeting point of the walk: the next S needs this warp's probabilities, which never come.
-          if (meet) asm volatile("bar.arrive %0, %1;" ::"r"(pair_bar), "n"(64) : "memory");
-          break;
-        }
-        tc_fence_after();
-        // keys past the end of the sequence (their K rows were read as zeros) get no weight
-        const int valid = j == n - 1 ? (int)(p.kv_len - (int64_t)j * kBKV) - half * 64 : 64;
-        float m_new;
-        bool raise;
-        if (meet) {
-          float mx = -INFINITY;
-#pragma unroll 1
-          for (int g = 0; g < 64; g += 8) {
-            uint32_t v[8];
-            tc_ld8(s_addr + g, v);
-            tc_wait_ld();
-#pragma unroll
-            for (int e = 0; e < 8; ++e)
-              if (g + e < valid) mx = fmaxf(mx, __uint_as_float(v[e]));
-          }
-          *xslot(j & 1, half) = mx;
-          asm volatile("bar.sync %0, %1;" ::"r"(pair_bar), "n"(64) : "memory");
-          mx = fmaxf(mx, *xslot(j & 1, half ^ 1));
-          m_new = mx * c;
-          raise = j > 0 && m_new - m_ref > kRescaleStep;
-          if (j == 0) m_ref = m_new;
-        } else {
-          // both threads' sums over the previous tile; by the exponent of the larger one, so that
-          // both threads of the row compute the same
-          const float seen = fmaxf(own_sum, *xslot(j & 1, half ^ 1));
-          raise = seen > kRaiseSum;
-          m_new = m_ref + (float)((__float_as_int(seen) >> 23) - 127);
-        }
-        if (__any_sync(0xffffffffu, raise)) {
-          // the previous P V of this tile completed before this S was committed: O is at rest
-          const float alpha = raise ? ex2(m_ref - m_new) : 1.f;
-          if (raise) m_ref = m_new;
-          l *= alpha;
-#pragma unroll 1
-          for (int g = 0; g < 64 / 8; ++g) {
-            uint32_t o[8];
-            tc_ld8(o_addr + g * 8, o);
-            tc_wait_ld();
-#pragma unroll
-            for (int e = 0; e < 8; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
-            tc_st8(o_addr + g * 8, o);
-          }
-        }
-        uint32_t s[64];
-        tc_ld32(s_addr, s);
-        tc_ld32(s_addr + 32, s + 32);
-        tc_wait_ld();
-        if (valid < 64) {
-#pragma unroll
-          for (int e = 0; e < 64; ++e)
-            if (e >= valid) s[e] = 0xFF800000u;   // -inf
-        }
-        // p = exp2(s*c - m); the row sum in fp32 before the rounding to bf16; bf16 pairs go back
-        // over this thread's own half of S (32 packed columns)
-        const float2 c2 = make_float2(c, c);
-        const float2 nm2 = make_float2(-m_ref, -m_ref);
-        float2 sum0 = make_float2(0.f, 0.f), sum1 = make_float2(0.f, 0.f);
-        // three sweeps rather than one loop, so that consecutive exponentials do not depend on one
-        // another's results: the special-function unit takes one warp instruction every 8 cycles
-        // and a sum or a pack right behind each would stall on it
-#pragma unroll
-        for (int e = 0; e < 32; ++e) {
-          const float2 x = f2_fma(make_float2(__uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1])), c2, nm2);
-          s[2 * e] = __float_as_uint(x.x);
-          s[2 * e + 1] = __float_as_uint(x.y);
-        }
-        // the exponent the FMA-pipe form adds must not leave its field: the largest such input (the
-        // special-function unit's results overflow to infinity by themselves and show in the sum)
-        float top = 0.f;
-        if (kFmaExpEvery > 0) {
-#pragma unroll
-          for (int e = 0; e < 32; e += (kFmaExpEvery > 0 ? kFmaExpEvery : 1))
-            top = max3(top, __uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1]));
-        }
-#pragma unroll
-        for (int e = 0; e < 32; ++e) {
-          float2 x = make_float2(__uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1]));
-          if (kFmaExpEvery > 0 && e % (kFmaExpEvery > 0 ? kFmaExpEvery : 1) == 0) {
-            x = exp2_fma(x);
-          } else {
-            x.x = ex2(x.x);
-            x.y = ex2(x.y);
-          }
-          s[2 * e] = __float_as_uint(x.x);
-          s[2 * e + 1] = __float_as_uint(x.y);
-        }
-#pragma unroll
-        for (int e = 0; e < 32; ++e) {
-          const float2 x = make_float2(__uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1]));
-          if (e & 1) sum1 = f2_add(sum1, x); else sum0 = f2_add(sum0, x);
-          s[e] = f2_to_bf16x2(x);      // s[e] is dead by now: 2e, 2e+1 >= e
-        }
-        own_sum = (sum0.x + sum0.y) + (sum1.x + sum1.y);
-        l += own_sum;
-        // a sum that is not a number counts, too
-        lost = lost || !(own_sum <= kRedoSum) || top > kRedoLog2;
-        // read by the partner at the next tile, written again two tiles on (the slot the exact
-        // maxima of tile 0 met in is the other one)
-        *xslot((j + 1) & 1, half) = own_sum;
-        tc_st32(s_addr, s);
-        tc_wait_st();
-        tc_fence_before();
-        mbar_arrive(p_full(t));
-      }
-      if (ok) {
-        ok = mbar_wait(o_full(t), (uint32_t)pass & 1u, abort_flag, p.status, kErrBase + 0x60 + t);
-        ok = __all_sync(0xffffffffu, ok);
-      }
-      if (pass == 0 && ok) {
-        tc_fence_after();
-        uint32_t most = 0u;                    // largest |O| of this thread, as float bits
-#pragma unroll 1
-        for (int g = 0; g < 64; g += 8) {
-          uint32_t o[8];
-          tc_ld8(o_addr + g, o);
-          tc_wait_ld();
-#pragma unroll
-          for (int e = 0; e < 8; ++e) most = max(most, o[e] & 0x7FFFFFFFu);
-        }
-        if (lost || most >= 0x7F800000u) *redo_flag = 1;
+      const CUtensorMap* map = (i & 1) ? &map_v : &map_k;
+      mbar_expect_tx(kv_full(s), kTileBytes, on);
+      for (int h = 0; h < 2; ++h)
+        tma_load_3d(map, kv_full(s), kv_smem(s) + h * kHalfBytes, h * 64, head, (i >> 1) * kBKV, on);
+    }
+    if (!ok) {
+      // let copies already in flight land before the CTA's memory is released
+      const long long t0 = clock64();
+      while (clock64() - t0 < 2000000LL) {
       }
     }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    if (pass > 0 || *redo_flag == 0 || *abort_flag != 0) break;
+  } else if (warp == kIssuerWarp) {
+    // ----------------------------------------------------- MMA issuer ----
+    const uint32_t on = elect_one();
+    const uint32_t idesc_s = make_idesc(false);
+    const uint32_t idesc_pv = make_idesc(true);
+    auto issue_s = [&](int qt, int slot) {
+      // S = Q K^T: eight steps of 16 contraction elements (32 bytes inside the swizzled row,
+      // the second 64 elements one half tile further)
+#pragma unroll
+      for (int ks = 0; ks < kD / 16; ++ks) {
+        const uint32_t off = (uint32_t)(ks >> 2) * kHalfBytes + (uint32_t)(ks & 3) * 32u;
+        tc_mma_ss(tmem_base + kColS + qt * 128, desc_kmajor(q_smem(qt) + off),
+                  desc_kmajor(kv_smem(slot) + off), idesc_s, ks > 0, on);
+      }
+      tc_commit(s_full(qt), on);
+    };
+    ok = mbar_wait(q_full(), 0, abort_flag, p.status, kErrBase + 0x10);
+    if (ok) ok = mbar_wait(kv_full(0), 0, abort_flag, p.status, kErrBase + 0x20);
+    ok = __all_sync(0xffffffffu, ok);
+    if (ok) {
+      tc_fence_after();
+      issue_s(0, 0);
+      issue_s(1, 0);
+      tc_commit(kv_empty(0), on);
+    }
+    for (int j = 0; ok && j < n; ++j) {
+      const int iv = 2 * j + 1, ik = 2 * j + 2;
+      const int sv = iv & (kKvSlots - 1), sk = ik & (kKvSlots - 1);
+      const bool has_next = j + 1 < n;
+      ok = mbar_wait(kv_full(sv), (uint32_t)(iv / kKvSlots) & 1u, abort_flag, p.status,
+                     kErrBase + 0x20 + sv);
+      if (ok && has_next)
+        ok = mbar_wait(kv_full(sk), (uint32_t)(ik / kKvSlots) & 1u, abort_flag, p.status,
+                       kErrBase + 0x20 + sk);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      for (int qt = 0; qt < kQTiles; ++qt) {
+        ok = mbar_wait(p_full(qt), (uint32_t)j & 1u, abort_flag, p.status, kErrBase + 0x50 + qt);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        // O += P V: sixteen keys per step = eight 32-bit columns of P (the first four steps' at the
+        // start of the first half of S, the others' at the start of the second), two 8-key
+        // groups of V
+#pragma unroll
+        for (int ks = 0; ks < kBKV / 16; ++ks)
+          tc_mma_ts(tmem_base + kColO + qt * 128,
+                    tmem_base + kColS + qt * 128 + (ks >> 2) * 64 + (ks & 3) * 8,
+                    desc_mnmajor(kv_smem(sv) + (uint32_t)ks * 2048u), idesc_pv, (j > 0 || ks > 0), on);
+        if (has_next)
+          issue_s(qt, sk);
+        else
+          tc_commit(o_full(qt), on);
+      }
+      if (!ok) break;
+      tc_commit(kv_empty(sv), on);
+      if (has_next) tc_commit(kv_empty(sk), on);
+    }
+  } else {
+    // ------------------------------------------------------- softmax ----
+    const float c = p.scale_log2;
+    float m_ref = 0.f;
+    float2 sum0 = make_float2(0.f, 0.f), sum1 = make_float2(0.f, 0.f);   // together the thread's row sum
+    for (int j = 0; j < n; ++j) {
+      ok = mbar_wait(s_full(t), (uint32_t)j & 1u, abort_flag, p.status, kErrBase + 0x40 + t);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) {
+        // The partner warp may have seen this barrier flip a moment before the abort flag went
+        // up and be on its way to this key tile's meeting point, which has no time limit of its
+        // own: arrive there without waiting, so that it gets through.  It cannot reach the next
+        // meeting point of the walk: the next S needs this warp's probabilities, which never come.
+        asm volatile("bar.arrive %0, %1;" ::"r"(pair_bar), "n"(64) : "memory");
+        break;
+      }
+      tc_fence_after();
+      // keys past the end of the sequence (their K rows were read as zeros) get no weight
+      const int valid = j == n - 1 ? (int)(p.kv_len - (int64_t)j * kBKV) - half * 64 : 64;
+      uint32_t s[64];
+      tc_ld32(s_addr, s);
+      tc_ld32(s_addr + 32, s + 32);
+      tc_wait_ld();
+      if (valid < 64) {
+#pragma unroll
+        for (int e = 0; e < 64; ++e)
+          if (e >= valid) s[e] = 0xFF800000u;   // -inf
+      }
+      float mx0 = -INFINITY, mx1 = -INFINITY;
+#pragma unroll
+      for (int e = 0; e < 64; e += 4) {
+        mx0 = max3(mx0, __uint_as_float(s[e]), __uint_as_float(s[e + 1]));
+        mx1 = max3(mx1, __uint_as_float(s[e + 2]), __uint_as_float(s[e + 3]));
+      }
+      float mx = fmaxf(mx0, mx1);
+      *xslot(j & 1, half) = mx;
+      asm volatile("bar.sync %0, %1;" ::"r"(pair_bar), "n"(64) : "memory");
+      mx = fmaxf(mx, *xslot(j & 1, half ^ 1));
+      const float m_new = mx * c;
+      const bool raise = j > 0 && m_new - m_ref > kRescaleStep;
+      if (j == 0) m_ref = m_new;
+      if (__any_sync(0xffffffffu, raise)) {
+        // the previous P V of this tile completed before this S was committed: O is at rest
+        const float alpha = raise ? ex2(m_ref - m_new) : 1.f;
+        if (raise) m_ref = m_new;
+        sum0 = f2_mul(sum0, make_float2(alpha, alpha));
+        sum1 = f2_mul(sum1, make_float2(alpha, alpha));
+#pragma unroll 1
+        for (int g = 0; g < 64 / 8; ++g) {
+          uint32_t o[8];
+          tc_ld8(o_addr + g * 8, o);
+          tc_wait_ld();
+#pragma unroll
+          for (int e = 0; e < 8; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+          tc_st8(o_addr + g * 8, o);
+        }
+      }
+      // p = exp2(s*c - m); bf16 pairs and the row sum of what they hold; the pairs go back
+      // over this thread's own half of S (32 packed columns)
+      const float2 c2 = make_float2(c, c);
+      const float2 nm2 = make_float2(-m_ref, -m_ref);
+      // three sweeps rather than one loop, so that consecutive exponentials do not depend on one
+      // another's results: the special-function unit takes one warp instruction every 8 cycles
+      // and a sum or a pack right behind each would stall on it
+#pragma unroll
+      for (int e = 0; e < 32; ++e) {
+        const float2 x = f2_fma(make_float2(__uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1])), c2, nm2);
+        s[2 * e] = __float_as_uint(x.x);
+        s[2 * e + 1] = __float_as_uint(x.y);
+      }
+#pragma unroll
+      for (int e = 0; e < 32; ++e) {
+        float2 x = make_float2(__uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1]));
+        if (kFmaExpEvery > 0 && e % (kFmaExpEvery > 0 ? kFmaExpEvery : 1) == 0) {
+          x = exp2_fma(x);
+        } else {
+          x.x = ex2(x.x);
+          x.y = ex2(x.y);
+        }
+        s[2 * e] = __float_as_uint(x.x);
+        s[2 * e + 1] = __float_as_uint(x.y);
+      }
+#pragma unroll
+      for (int e = 0; e < 32; ++e) {
+        const float2 x = make_float2(__uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1]));
+        float2& sum = (e & 1) ? sum1 : sum0;
+        s[e] = f2_to_bf16x2(x);      // s[e] is dead by now: 2e, 2e+1 >= e
+        sum = add_bf16x2(s[e], sum);
+      }
+      tc_st32(s_addr, s);
+      tc_wait_st();
+      tc_fence_before();
+      mbar_arrive(p_full(t));
+    }
+    l = (sum0.x + sum0.y) + (sum1.x + sum1.y);
+    if (ok) {
+      ok = mbar_wait(o_full(t), 0, abort_flag, p.status, kErrBase + 0x60 + t);
+      ok = __all_sync(0xffffffffu, ok);
+    }
   }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
   if (warp < kSoftmaxWarps) {
     // ----------------------------------------------------------- epilogue ----
     // nobody gives up any more: all warps with a result agree on it (ok), and a warp without one
