@@ -342,7 +342,9 @@ quantize_small_kernel(const uint4* x, uint32_t n_blocks, uint32_t kb_per_row, in
 // results, so each CTA tabulates them once (low bytes, then high bytes, of the eight bf16 values
 // of a scale byte: one 16-byte shared-memory read per block) and an element costs byte selections
 // instead of a decode, a multiply and a conversion, a block no division.  [14336, 3072]: 47.1 -> 24.2 us
-// through to_bfloat16() (2.4 -> 4.7 TB/s), the call's host part included.
+// through to_bfloat16() (2.4 -> 4.7 TB/s), the call's host part included.  A thread with few blocks in
+// all (`direct`) makes its own entries instead, and the first loads are on their way meanwhile: small
+// tensors are all latency ([64, 3072], replayed from a graph: 2.4 us with the table, 2.0 without).
 constexpr int kDequantBlocks = 2;    // scale blocks in flight per thread
 
 __device__ __forceinline__ void decode4(uint32_t codes, const uint4& t, uint32_t signs, uint32_t& o0,
@@ -354,27 +356,26 @@ __device__ __forceinline__ void decode4(uint32_t codes, const uint4& t, uint32_t
   o1 = __byte_perm(lo, hi, 0x7362) ^ (((codes & 0x8800u) * 0x10010u) & signs);
 }
 
+__device__ __forceinline__ uint4 dequant_entry(uint32_t sf, float s_enc) {
+  const float d = __fdiv_rn(e4m3_to_f32((uint8_t)sf), s_enc);
+  const float mag[8] = {0.0f, 0.5f, 1.0f, 1.5f, 2.0f, 3.0f, 4.0f, 6.0f};
+  uint32_t v[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    v[k] = f2_to_bf16x2(make_float2(__fmul_rn(mag[2 * k], d), __fmul_rn(mag[2 * k + 1], d)));
+  return make_uint4(__byte_perm(v[0], v[1], 0x6420), __byte_perm(v[2], v[3], 0x6420),
+                    __byte_perm(v[0], v[1], 0x7531), __byte_perm(v[2], v[3], 0x7531));
+}
+
 __global__ void __launch_bounds__(kThreads)
 dequantize_bf16_kernel(const uint32_t* __restrict__ packed, const uint8_t* __restrict__ sf_lin,
                        int64_t n_blocks, const float* __restrict__ amax_ptr, float amax_val,
-                       uint4* __restrict__ out, int word2, int wide_out) {
+                       uint4* __restrict__ out, int word2, int wide_out, int direct) {
   __shared__ uint4 table[256];
-  const float s_enc = global_encode_scale(amax_ptr ? __ldg(amax_ptr) : amax_val);
-  for (int i = threadIdx.x; i < 256; i += kThreads) {
-    const float d = __fdiv_rn(e4m3_to_f32((uint8_t)i), s_enc);
-    const float mag[8] = {0.0f, 0.5f, 1.0f, 1.5f, 2.0f, 3.0f, 4.0f, 6.0f};
-    uint32_t v[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      v[k] = f2_to_bf16x2(make_float2(__fmul_rn(mag[2 * k], d), __fmul_rn(mag[2 * k + 1], d)));
-    table[i] = make_uint4(__byte_perm(v[0], v[1], 0x6420), __byte_perm(v[2], v[3], 0x6420),
-                          __byte_perm(v[0], v[1], 0x7531), __byte_perm(v[2], v[3], 0x7531));
-  }
-  __syncthreads();
   const int64_t stride = (int64_t)gridDim.x * kThreads;
-  for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n_blocks; i += kDequantBlocks * stride) {
-    uint2 p[kDequantBlocks];
-    uint32_t sf[kDequantBlocks];
+  uint2 p[kDequantBlocks];
+  uint32_t sf[kDequantBlocks];
+  auto load = [&](int64_t i) {
 #pragma unroll
     for (int j = 0; j < kDequantBlocks; ++j) {
       const int64_t b = i + j * stride;
@@ -384,11 +385,20 @@ dequantize_bf16_kernel(const uint32_t* __restrict__ packed, const uint8_t* __res
         sf[j] = __ldcs(sf_lin + b);
       }
     }
+  };
+  int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  load(i);       // on their way while the table is made: a small tensor is all latency
+  const float s_enc = global_encode_scale(amax_ptr ? __ldg(amax_ptr) : amax_val);
+  if (!direct) {
+    for (int b = threadIdx.x; b < 256; b += kThreads) table[b] = dequant_entry(b, s_enc);
+    __syncthreads();
+  }
+  for (; i < n_blocks; i += kDequantBlocks * stride) {
 #pragma unroll
     for (int j = 0; j < kDequantBlocks; ++j) {
       const int64_t b = i + j * stride;
       if (b < n_blocks) {
-        const uint4 t = table[sf[j]];
+        const uint4 t = direct ? dequant_entry(sf[j], s_enc) : table[sf[j]];
         const uint32_t signs = (sf[j] & 127u) == 127u ? 0u : 0x80008000u;   // a NaN scale: one NaN
         uint32_t o[8];
         decode4(p[j].x & 0xFFFFu, t, signs, o[0], o[1]);
@@ -406,6 +416,7 @@ dequantize_bf16_kernel(const uint32_t* __restrict__ packed, const uint8_t* __res
         }
       }
     }
+    load(i + kDequantBlocks * stride);
   }
 }
 
@@ -629,13 +640,15 @@ static int dequantize_impl(const uint8_t* packed, const uint8_t* scales, int64_t
   int rc = check_device_sm100();
   if (rc != NVFP4_OK) return rc;
   const int64_t n_blocks = n / kBlock;
-  const int64_t want = (n_blocks + kThreads * kDequantBlocks - 1) / (kThreads * kDequantBlocks);
+  const int direct = n_blocks <= (int64_t)sm_count() * kThreads;
+  const int per_thread = direct ? 1 : kDequantBlocks;
+  const int64_t want = (n_blocks + kThreads * per_thread - 1) / (kThreads * per_thread);
   const int64_t resident = (int64_t)sm_count() * 8;       // 2048 threads per SM
   dequantize_bf16_kernel<<<(unsigned)(want < resident ? want : resident), kThreads, 0,
                            reinterpret_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<const uint32_t*>(packed), scales, n_blocks, amax_dev, amax_val,
       reinterpret_cast<uint4*>(out), (reinterpret_cast<uintptr_t>(packed) & 7u) == 0,
-      (reinterpret_cast<uintptr_t>(out) & 31u) == 0);
+      (reinterpret_cast<uintptr_t>(out) & 31u) == 0, direct);
   return launch_status();
 }
 
