@@ -248,6 +248,10 @@ constexpr int kSmallThreads = 512;
 constexpr int kSmallCtas = 8;            // the portable cluster size
 constexpr int kSmallBlocks = 8;          // most blocks per thread
 constexpr int64_t kSmallMax = (int64_t)kSmallCtas * kSmallThreads * kSmallBlocks;
+// Most bytes of swizzled scales, which the cluster zeroes: a few long rows are mostly pad, and a memset
+// has the whole GPU for it ([1, 65536], 1 MB: 9.7 us with memsets and two kernels, 5.0 here; [1, 262144],
+// 4 MB: 10.3 and 12.7; [1, 524288], 8 MB: 10.4 and 23).
+constexpr int64_t kSmallPad = 2 << 20;
 
 template <int kB>
 __global__ void __launch_bounds__(kSmallThreads)
@@ -585,7 +589,8 @@ int nvfp4_amax_quantize_bf16(const void* x, int64_t rows, int64_t cols, float* a
   if (!amax_dev) return NVFP4_ERR_BAD_ARG;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int64_t n_blocks = rows * cols / kBlock;
-  if (n_blocks > 0 && n_blocks <= kSmallMax && aligned16(scales_swizzled)) {
+  if (n_blocks > 0 && n_blocks <= kSmallMax && aligned16(scales_swizzled) &&
+      (!scales_swizzled || sf_swizzled_bytes(rows, cols) <= kSmallPad)) {
     // as few blocks per thread as the cluster allows: latency is what counts here
     int ctas = 1;
     while (ctas < kSmallCtas && n_blocks > (int64_t)ctas * kSmallThreads) ctas *= 2;

@@ -21,6 +21,7 @@ def _check(oracle, x, t):
 @pytest.mark.parametrize("rows,cols", [
     (1, 16), (1, 18432), (2, 8192), (33, 512), (128, 64),                  # one CTA to eight
     (31, 16896), (32, 16384), (33, 15888),                                 # around 524288 elements
+    (1, 131072), (1, 131088), (3, 131088), (1, 524288),                    # mostly pad: 2 MB of it, and past that
     (31, 17408), (32, 16912), (40, 13840), (200, 3072), (171, 3088),       # past it: flat / rows
     (1000, 1520), (1000, 1536), (1000, 1552), (4096, 144), (70000, 16)])   # narrow rows
 def test_forms_against_the_oracle(oracle, rows, cols):
