@@ -81,6 +81,7 @@ class PackedBuffers:
             self.amax = torch.empty(1, dtype=torch.float32, device=self.device)
             self.gscale = torch.empty(1, dtype=torch.float32, device=self.device)
             self.stats = torch.empty(rows, 2, dtype=torch.float32, device=self.device)   # fused norm
+            self.partials = torch.empty(N.AMAX_PARTIALS, dtype=torch.float32, device=self.device)  # quantizer
         self.device = self.data.device       # with its index, as tensors report it
 
     def matches(self, rows: int, cols: int, device) -> bool:
@@ -164,7 +165,8 @@ class FP4Tensor:
                                     if swizzled_scales and rows * cols > 0 else None)
             st = N.stream_ptr()
             if amax is None and amax_hook is None and rows * cols > 0:
-                part = torch.empty(N.AMAX_PARTIALS, dtype=torch.float32, device=dev)
+                part = (out.partials if out is not None
+                        else torch.empty(N.AMAX_PARTIALS, dtype=torch.float32, device=dev))
                 N.check(N.lib.nvfp4_amax_quantize_bf16(N.ptr(x), rows, cols, N.ptr(self._amax),
                                                        N.ptr(self._data), N.ptr(self._scales),
                                                        N.ptr(self._scales_swz), N.ptr(self._gscale),

@@ -66,3 +66,20 @@ def test_c_entry_without_partials_and_with_odd_scale_pointers(oracle, offset, wi
         assert np.array_equal(lin[offset:offset + scales.size].cpu().numpy(), scales.reshape(-1))
         assert np.array_equal(swz[offset:offset + n].cpu().numpy(), oracle.swizzle_scales(scales, cols))
         assert bool((swz[offset + n:] == 0xAA).all()) and bool((swz[:offset] == 0xAA).all())
+
+
+@pytest.mark.parametrize("rows,cols", [(33, 512), (600, 1024), (1000, 1536), (700, 4096)])
+def test_given_buffers_nothing_is_allocated(rows, cols):
+    from blackwell_diffusion_rtx6000_5090_i2v_b200 import nvfp4 as nv
+    x = student_t_bf16((rows, cols), 7, device="cuda")
+    b = nv.PackedBuffers(rows, cols, "cuda", linear_scales=True)
+    want = nv.FP4Tensor.from_bfloat16(x)
+    count = lambda: torch.cuda.memory_stats()["allocation.all.allocated"]  # noqa: E731
+    before = count()
+    t = nv.FP4Tensor.from_bfloat16(x, out=b)
+    nv.FP4Tensor.from_bfloat16(x, amax=t.global_amax(), out=b)
+    nv.FP4Tensor.from_norm_mod(x, out=b)
+    t = nv.FP4Tensor.from_bfloat16(x, out=b)
+    assert count() == before
+    assert torch.equal(t.quantized_data(), want.quantized_data())
+    assert torch.equal(t.scale_factors_swizzled(), want.scale_factors_swizzled())
