@@ -496,7 +496,13 @@ int quantize_impl(const void* x, int64_t rows, int64_t cols, const float* amax_d
   if (rc != NVFP4_OK || n_blocks == 0) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   int threads;
-  if (rows_form(rows, cols, sf_swz != nullptr, &threads)) {
+  // With the maximum known the flat form is one kernel where the layout has no pad, and then the rows
+  // form (its table, a CTA's idle lanes) pays only for long tensors and nearly full CTAs.  Replayed from a
+  // graph, us flat and rows: [256, 3072] 2.4 and 2.9, [4096, 3072] 6.1 and 6.1, [16384, 3072] 19.9 and
+  // 18.8, [16384, 1280] 8.9 and 9.2; with a pad, and so a memset, [170, 3072] 3.9 and 2.8.
+  const bool pads = sf_swz && (rows % 256 != 0 || cols / kBlock % kSfKbPad != 0);
+  if (rows_form(rows, cols, sf_swz != nullptr, &threads) &&
+      (pads || (n_blocks >= (1 << 20) && cols / kBlock * 8 >= (int64_t)threads * 7))) {
     PackArgs a{};
     a.x = reinterpret_cast<const uint4*>(x);
     a.rows = rows;

@@ -42,6 +42,20 @@ def test_input_on_a_16_byte_boundary_only(oracle, rows, cols):
     _check(oracle, x.cpu(), nv.FP4Tensor.from_bfloat16(x))
 
 
+@pytest.mark.parametrize("rows,cols", [(2049, 1152), (5000, 1280), (5120, 1280), (300, 3072), (5376, 3072), (5632, 3072),
+                                       (257, 2048)])
+def test_known_maximum_fills_a_poisoned_buffer(oracle, rows, cols):
+    """The packing kernel alone, through the entry point that takes the maximum: every byte of the
+    swizzled layout is written, whichever form packs."""
+    from blackwell_diffusion_rtx6000_5090_i2v_b200 import nvfp4 as nv
+    x = student_t_bf16((rows, cols), 9)
+    b = nv.PackedBuffers(rows, cols, "cuda", linear_scales=True)
+    for t in (b.data, b.scales, b.scales_swz):
+        t.fill_(0xAA)
+    amax = x.float().abs().max().reshape(1).cuda()
+    _check(oracle, x, nv.FP4Tensor.from_bfloat16(x.cuda(), amax=amax, out=b))
+
+
 @pytest.mark.parametrize("offset", [0, 1])
 @pytest.mark.parametrize("with_partials", [False, True])
 def test_c_entry_without_partials_and_with_odd_scale_pointers(oracle, offset, with_partials):
