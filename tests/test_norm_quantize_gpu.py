@@ -66,6 +66,20 @@ def test_fused_norm_quantize(oracle, rows, cols, rms, affine, mod):
     assert float((h != ref).float().mean()) < 0.02
 
 
+@pytest.mark.parametrize("rows,cols", [(1, 3072), (129, 3072), (255, 256), (300, 512), (511, 3088), (257, 5120)])
+def test_pad_of_the_swizzled_scales_is_written(oracle, rows, cols):
+    """Rows up to the next 256 and K-blocks up to the next 16 pad the layout: zeros over whatever the
+    buffer held."""
+    from blackwell_diffusion_rtx6000_5090_i2v_b200 import nvfp4 as nv
+    x = student_t_bf16((rows, cols), 3, device="cuda")
+    b = nv.PackedBuffers(rows, cols, "cuda")
+    b.scales_swz.fill_(0xAA)
+    t, h = nv.FP4Tensor.from_norm_mod(x, out=b, return_normed=True)
+    _, scales, _ = oracle.quantize(bits_of(h))
+    assert t.scale_factors_swizzled().data_ptr() == b.scales_swz.data_ptr()
+    assert np.array_equal(b.scales_swz.cpu().numpy(), oracle.swizzle_scales(scales, cols))
+
+
 def test_fused_norm_feeds_the_gemm(oracle):
     """norm -> modulation -> QKV linear, fused against unfused, through the GEMM."""
     from blackwell_diffusion_rtx6000_5090_i2v_b200 import nvfp4 as nv

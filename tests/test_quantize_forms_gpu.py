@@ -23,6 +23,7 @@ def _check(oracle, x, t):
     (31, 16896), (32, 16384), (33, 15888),                                 # around 524288 elements
     (1, 131072), (1, 131088), (3, 131088), (1, 524288),                    # mostly pad: 2 MB of it, and past that
     (31, 17408), (32, 16912), (40, 13840), (200, 3072), (171, 3088),       # past it: flat / rows
+    (1000, 1136), (1000, 1152), (1000, 1280), (1000, 1488),                # the narrowest rows of that form
     (1000, 1520), (1000, 1536), (1000, 1552), (4096, 144), (70000, 16)])   # narrow rows
 def test_forms_against_the_oracle(oracle, rows, cols):
     from blackwell_diffusion_rtx6000_5090_i2v_b200 import nvfp4 as nv
@@ -33,7 +34,8 @@ def test_forms_against_the_oracle(oracle, rows, cols):
     _check(oracle, x, nv.FP4Tensor.from_bfloat16(x.cuda(), amax=t.global_amax()))
 
 
-@pytest.mark.parametrize("rows,cols", [(40, 512), (700, 1024)])
+# small, flat and, past 524288 elements and with 96 threads or more a row, rows form
+@pytest.mark.parametrize("rows,cols", [(40, 512), (700, 1024), (1000, 1552), (200, 3072)])
 def test_input_on_a_16_byte_boundary_only(oracle, rows, cols):
     from blackwell_diffusion_rtx6000_5090_i2v_b200 import nvfp4 as nv
     buf = student_t_bf16((rows * cols + 8,), 5).cuda()
@@ -60,7 +62,7 @@ def test_known_maximum_fills_a_poisoned_buffer(oracle, rows, cols):
 @pytest.mark.parametrize("with_partials", [False, True])
 def test_c_entry_without_partials_and_with_odd_scale_pointers(oracle, offset, with_partials):
     from blackwell_diffusion_rtx6000_5090_i2v_b200 import _native as N
-    for rows, cols in ((3, 256), (600, 1024)):
+    for rows, cols in ((3, 256), (600, 1024), (1000, 1152), (1000, 1280), (1000, 1552), (200, 3072)):
         x = student_t_bf16((rows, cols), 6)
         xd = x.cuda()
         swz = torch.full((N.lib.nvfp4_swizzled_scale_bytes(rows, cols) + 16,), 0xAA, dtype=torch.uint8, device="cuda")
