@@ -907,23 +907,36 @@ int g_tiling_mode = 0;
 // Columns per tile.  256-wide tiles take in the fewest operand bytes per flop, and under a sustained
 // load that is what counts ([4095, 5120] x 5120: 66 us, 72 us with 192-wide tiles that would save a
 // sixth of the waves).  Narrower ones are for grids that leave the GPU idle: at most two waves of
-// 256-wide tiles, and an estimate (waves times a tile's cost) at least a tenth lower.  A narrow tile
-// costs more than its share because the A rows and their scales are taken in whole.  Replayed from a
-// graph, us uniform -> chosen: 256 x 3072 x 3072 (M, N, K) 10.6 -> 8.6 (64 columns), 512 x 3072 x 4096 11.8 ->
-// 10.2 (128), 1760 x 3072 x 3072 15.9 -> 14.3 and x 14336 42.7 -> 38.2 (192), 2048 x 3072 x 3072 15.9 -> 14.4;
-// a single row, where there is no epilogue to share out, 1 x 3072 x 3072 9.8 -> 10.2.
-int tile_width(int64_t m_tiles, int64_t N) {
+// 256-wide tiles.  The choice is the least waves times a tile's cost; the costs are what one wave of a
+// width takes beside one of 256, rounded (replayed from a graph, us at 256 / 192 / 128 / 64 columns: 256 x
+// 3072 x 3072 (M, N, K) 10.9 / 10.3 / 9.5 / 9.0, 256 x 3072 x 14336 24.8 / 23.5 / 22.0 / 21.1, 1760 x 3072 x
+// 14336, two waves of both, 42.8 / 39.0).
+//
+// Few rows: then every CTA pair fetches the same few lines of A for every stage, and the more pairs do the
+// longer they queue.  What narrower tiles gained turns into a loss where there are many of them or the
+// contraction is long (1 x 3072 x 14336 24.3 / 23.1 / 22.9 / 27.1; 1 x 3072 x 3072 10.3 / 9.9 / 9.6 / 10.6;
+// 1 x 9216 x 3072, 72 tiles of 128, 12.7 / - / 12.9; 1 x 5120 x 13824, 40 of 128, 25.1 / - / 27.6; 32 x 13824 x
+// 5120, 72 of 192, 15.8 / 16.2), but stays one where there are few (1 x 1024 x 1024 8.0 / 7.9 / 6.8 / 6.8, 8 x
+// 5120 x 5120, 40 of 128, 13.9 / - / 12.7).
+int tile_width(int64_t m_tiles, int64_t M, int64_t N, int64_t K) {
   const int64_t pairs = sm_count() / 2;
   static const int width[4] = {256, 192, 128, 64};
-  static const int cost[4] = {100, 88, 76, 64};      // of a tile, in hundredths of a 256-wide one
-  const int64_t waves = (m_tiles * ((N + 255) / 256) + pairs - 1) / pairs;
-  if (waves > 2) return 256;
+  static const int cost[4] = {100, 93, 88, 84};      // of a wave, in hundredths of a 256-wide one
+  if ((m_tiles * ((N + 255) / 256) + pairs - 1) / pairs > 2) return 256;
+  auto queues = [&](int w, int64_t tiles) {
+    switch (w) {
+      case 192: return M < 64;
+      case 128: return M < 32 && (tiles * 3 > pairs * 2 || tiles * K > 350000);
+      case 64: return M < 32 && tiles * 3 > pairs;
+      default: return false;
+    }
+  };
   int best = 256;
-  int64_t best_time = waves * 90;
-  for (int i = 1; i < 4; ++i) {
+  int64_t best_time = INT64_MAX;
+  for (int i = 0; i < 4; ++i) {
     const int64_t tiles = m_tiles * ((N + width[i] - 1) / width[i]);
     const int64_t time = (tiles + pairs - 1) / pairs * cost[i];
-    if (time < best_time) {
+    if (time < best_time && !queues(width[i], tiles)) {
       best = width[i];
       best_time = time;
     }
@@ -976,7 +989,7 @@ int gemm_impl(const uint8_t* a_packed, const uint8_t* b_packed, const uint8_t* a
   if (rc != NVFP4_OK) return rc;
 
   const int64_t m_tiles = (M + 2 * gemm::BM - 1) / (2 * gemm::BM);     // 256-row pair tiles
-  const int width = g_tiling_mode == 0 ? tile_width(m_tiles, N) : gemm::BN;
+  const int width = g_tiling_mode == 0 ? tile_width(m_tiles, M, N, K) : gemm::BN;
   const bool narrow = width < gemm::BN, alt = g_tiling_mode == 2;
   const int narrow_w = narrow ? width : gemm::kAltNarrow;
 

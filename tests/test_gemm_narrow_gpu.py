@@ -9,7 +9,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("M,N,K", [
-    (1, 8, 32), (1, 64, 256), (3, 200, 512), (512, 3072, 1024), (512, 3080, 4096), (257, 1096, 2048),
+    (1, 8, 32), (1, 64, 256), (3, 200, 512), (1, 3072, 512), (31, 1536, 512), (31, 1600, 512), (32, 1600, 512),
+    (31, 6272, 256), (31, 6400, 256), (32, 6400, 256), (63, 13824, 256), (64, 13824, 256), (8, 5120, 8192), (512, 3072, 1024), (512, 3080, 4096), (257, 1096, 2048),
     (1760, 3072, 512), (1760, 9216, 256), (1760, 14336, 256), (2048, 1032, 14336), (900, 5120, 96),
     (4095, 5120, 288)])
 @pytest.mark.parametrize("epilogue", [False, True])
