@@ -11,15 +11,17 @@
 // tensor can be carried along untouched so that q, k and v land in one packed
 // [tokens, heads, 3 * head_dim] buffer ready for a head/sequence exchange.
 //
-// Bound: HBM, 8 B per element of q and k.  A row is reduced and then rewritten, so it has to be
-// held: one warp holds a row of up to 5120 elements in registers, a lane taking every 32nd 8-element
-// chunk, all its loads in flight together; nothing is staged in shared memory and no barrier is met.
-// Longer rows take a CTA.  The rotation-table entries of a lane are the same for all its chunks when
-// 32 chunks are whole heads (they were fetched once per chunk before, the largest stall), and the
-// gains come from L1.  The sum of squares is added in one fixed order whoever holds the chunks: W
-// groups of 32 lanes (W = warps that four chunks per thread need), four chunks each, lanes by halving,
-// then groups in pairs.
-// [27280, 3 x 3072], L2 flushed: 160.7 -> 125.0 us (two CTAs per SM; three at 80 registers: 135).
+// Bound: HBM, 8 B per element of q and k.  A row is reduced and then rewritten, so it has to be held.
+// Two forms, neither of which stages it in shared memory:
+//   CTA    a row per CTA, four 8-element chunks per thread, the next row's loads on their way while this one
+//          is reduced and written
+//   warp   a row per warp, a lane taking every 32nd chunk, all its loads in flight together and no barrier met
+// The rotation-table entries of a thread are the same for all its chunks when a warp's (a CTA's) chunks
+// are whole heads, and the gains come from L1.  The sum of squares is added in one fixed order whoever
+// holds the chunks: W groups of 32 lanes (W = warps that four chunks per thread need), four chunks each,
+// lanes by halving, then groups in pairs.
+// [27280, 3 x 3072], L2 flushed: 160.7 us with the row staged, 125.0 a row per warp (two CTAs per SM; three
+// at 80 registers: 135).  Which form when, and what each takes: warp_form().
 // blockIdx.y selects the tensor: 0 = q, 1 = k, 2 = v (copy only).
 #include "exchange_sync.cuh"
 #include "nvfp4_common.cuh"
@@ -117,7 +119,7 @@ __device__ __forceinline__ uint4 norm_rotate(const uint4& v, float2 r2, const fl
   return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
-// One warp per row of at most 4 W groups of 32 chunks.
+// Warp form: one warp per row of at most 4 W groups of 32 chunks.
 template <int W>
 __global__ void __launch_bounds__(kThreads, 2) rope_warp_kernel(const RopeArgs p) {
   constexpr int kN = 4 * W, kRowsPerCta = kThreads / 32;
@@ -186,8 +188,9 @@ __global__ void __launch_bounds__(kThreads, 2) rope_warp_kernel(const RopeArgs p
   if (p.signal) xsync::signal_when_grid_done(p.peers, 0, gridDim.x * gridDim.y, false);
 }
 
-// One CTA per row, four chunks per thread.
-__global__ void __launch_bounds__(512) rope_cta_kernel(const RopeArgs p) {
+// CTA form.  64 registers, so that 1024 threads of any CTA width fit an SM.
+__global__ void __launch_bounds__(512, 2) rope_cta_kernel(const RopeArgs p) {
+  extern __shared__ uint8_t* dst_tab[];
   __shared__ __align__(16) float red[2][16];
   const int which = blockIdx.y;
   const int lane = threadIdx.x & 31;
@@ -198,22 +201,33 @@ __global__ void __launch_bounds__(512) rope_cta_kernel(const RopeArgs p) {
   const bool rotate = which < 2 && p.cos_sin != nullptr;
   const int64_t half_hd = p.head_dim >> 1;
   const float dim_f = (float)p.dim;
-  uint8_t* dst[4];
+  for (int c = threadIdx.x; c < chunks; c += T) dst_tab[c] = chunk_dst(p, which, c, per_head);
+  uint4 v[4], next[4];
+  auto load = [&](int64_t row, uint4 (&d)[4]) {
+    const uint4* src = reinterpret_cast<const uint4*>(in + row * p.in_row_bytes);
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int c = threadIdx.x + k * T;
-    dst[k] = c < chunks ? chunk_dst(p, which, c, per_head) : nullptr;
-  }
+    for (int k = 0; k < 4; ++k) {
+      const int c = threadIdx.x + k * T;
+      d[k] = c < chunks ? load_u32x4_once(src + c) : make_uint4(0, 0, 0, 0);
+    }
+  };
   if (threadIdx.x < 32) (&red[0][0])[threadIdx.x] = 0.0f;
   __syncthreads();
   grid_dependency_wait();
+  const bool one_entry = T % per_head == 0;      // as in the kernel above
   int parity = 0;
+  if (blockIdx.x < p.rows) load(blockIdx.x, next);
   for (int64_t row = blockIdx.x; row < p.rows; row += gridDim.x, parity ^= 1) {
-    const uint4* src = reinterpret_cast<const uint4*>(in + row * p.in_row_bytes);
     const float4* table = reinterpret_cast<const float4*>(p.cos_sin + row * half_hd);
-    uint4 v[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = dst[k] ? load_u32x4_once(src + threadIdx.x + k * T) : make_uint4(0, 0, 0, 0);
+    for (int k = 0; k < 4; ++k) v[k] = next[k];
+    // the next row is on its way while this one is reduced and written
+    if (row + gridDim.x < p.rows) load(row + gridDim.x, next);
+    float4 cs[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+    if (rotate && one_entry) {
+      cs[0] = load_f32x4(table + 2 * (threadIdx.x % per_head));
+      cs[1] = load_f32x4(table + 2 * (threadIdx.x % per_head) + 1);
+    }
     float rstd = 0.0f;
     if (which < 2) {
       float2 s2 = make_float2(0.0f, 0.0f);
@@ -235,16 +249,15 @@ __global__ void __launch_bounds__(512) rope_cta_kernel(const RopeArgs p) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int c = threadIdx.x + k * T;
-      if (!dst[k]) break;
+      if (c >= chunks) break;
       if (which < 2) {
-        float4 cs[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
-        if (rotate) {
+        if (rotate && !one_entry) {
           cs[0] = load_f32x4(table + 2 * (c % per_head));
           cs[1] = load_f32x4(table + 2 * (c % per_head) + 1);
         }
         v[k] = norm_rotate(v[k], r2, gain ? gain + 8 * c : nullptr, rotate, cs);
       }
-      *reinterpret_cast<uint4*>(dst[k] + out_row) = v[k];
+      *reinterpret_cast<uint4*>(dst_tab[c] + out_row) = v[k];
     }
   }
   if (p.signal) xsync::signal_when_grid_done(p.peers, 0, gridDim.x * gridDim.y, false);
@@ -263,17 +276,27 @@ int launch_warp(const RopeArgs& a, int tensors, cudaStream_t st) {
                           (size_t)(a.dim / 8) * sizeof(uint8_t*), 1, st, a);
 }
 
+// The warp form wins where every warp has one row at most and the SMs are nearly full of them (its 16 warps
+// per SM; for rows of one group from the first row on), and at three groups for many rows.  Replayed
+// from a graph, us warp / CTA: [512, 6 heads of 128] 3.1 / 3.7, [1024, 12] 4.7 / 5.1, [1024, 24] 7.2 / 7.9,
+// [32760, 24] 144 / 150, [32760, 20] 123 / 132; but [512, 24] 6.6 / 5.0, [1760, 24] 12.0 / 10.5, [8192, 12] 20.7 /
+// 22.3, [32760, 12] 84 / 80, [32760, 6] 53 / 42.  Four or five groups, where a lane holds 16 or 20 chunks: [64,
+// 40] 10.2 / 4.0, [1760, 40] 20.4 / 16.6, [32760, 32] 207 / 189, [32760, 40] 252 / 250.
+bool warp_form(int W, int64_t rows) {
+  const int64_t slots = (int64_t)sm_count() * 2 * (kThreads / 32);
+  if (W > 3) return false;
+  if (rows <= slots) return W == 1 || rows * 5 > slots * 4;
+  return W == 3 && rows >= slots * 10;
+}
+
 int launch_rope(const RopeArgs& a, int tensors, cudaStream_t st) {
   const int W = ((a.dim / 8 + 3) / 4 + 31) / 32;
-  switch (W) {
-    case 1: return launch_warp<1>(a, tensors, st);
-    case 2: return launch_warp<2>(a, tensors, st);
-    case 3: return launch_warp<3>(a, tensors, st);
-    case 4: return launch_warp<4>(a, tensors, st);
-    case 5: return launch_warp<5>(a, tensors, st);
-  }
+  if (warp_form(W, a.rows * tensors))
+    return W == 1 ? launch_warp<1>(a, tensors, st) : W == 2 ? launch_warp<2>(a, tensors, st)
+                                                            : launch_warp<3>(a, tensors, st);
   const int64_t gx = grid_x(a.rows, 1, 1024 / (32 * W), tensors);
-  return launch_dependent(rope_cta_kernel, dim3((unsigned)gx, (unsigned)tensors), 32 * W, 0, 1, st, a);
+  return launch_dependent(rope_cta_kernel, dim3((unsigned)gx, (unsigned)tensors), 32 * W,
+                          (size_t)(a.dim / 8) * sizeof(uint8_t*), 1, st, a);
 }
 
 }  // namespace

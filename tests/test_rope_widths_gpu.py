@@ -1,5 +1,5 @@
-"""q/k RMSNorm + rotation for every number of warps that share a row, and for heads whose width does not
-divide a team's: against the torch ops it replaces."""
+"""q/k RMSNorm + rotation in both forms (a row per warp, a row per CTA), for every number of warps that
+share a row and for heads whose width does not divide a team's: against the torch ops it replaces."""
 import pytest
 import torch
 
@@ -10,7 +10,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("rows,heads,D", [
     (5, 1, 16), (9, 1, 128), (33, 24, 128), (65, 25, 128), (1, 40, 128), (130, 48, 128), (17, 49, 128),
-    (3, 128, 128), (20, 10, 48), (11, 70, 80), (700, 3, 128)])
+    (3, 128, 128), (20, 10, 48), (11, 70, 80), (700, 3, 128),
+    (1300, 3, 128), (1000, 12, 128), (1000, 24, 128), (1000, 30, 80), (1185, 12, 128), (12000, 20, 128)])   # rows at which the form changes
 @pytest.mark.parametrize("gains", [True, False])
 def test_widths_against_torch_ops(rows, heads, D, gains):
     from blackwell_diffusion_rtx6000_5090_i2v_b200 import dit
