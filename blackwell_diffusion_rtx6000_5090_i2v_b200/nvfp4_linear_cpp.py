@@ -144,7 +144,7 @@ def linear(input: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
     if gate is not None:
         ep["gate"] = gate
     if residual is not None:
-        ep["C"] = residual.reshape(-1, n)
+        ep["C"] = r2
     if out is not None:
         ep["out"] = out.reshape(-1, n)
     if n % 8 != 0 and ep:
@@ -157,7 +157,7 @@ def linear(input: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
         if gate is not None:
             y = y * gate.to(y.dtype)
         if residual is not None:
-            y = y + residual.reshape(-1, n)
+            y = y + r2
         return y.reshape(batch_dims + [n])
     beta = 1.0 if residual is not None else 0.0
     _check_pair(x2, weight)

@@ -47,3 +47,20 @@ def test_operands_for_the_general_path():
         y = lc.linear(x, w)
     torch.cuda.current_stream().wait_stream(side)
     assert torch.equal(y, lc.gemm(x, w))
+
+
+def test_a_strided_residual_is_copied_once():
+    from blackwell_diffusion_rtx6000_5090_i2v_b200 import nvfp4_linear_cpp as lc
+    x, w = randn_bf16((4, 10, 64), 1, device="cuda"), randn_bf16((48, 64), 2, device="cuda")
+    res = randn_bf16((10, 4, 48), 3, device="cuda").transpose(0, 1)
+    out = torch.empty(4, 10, 48, dtype=torch.bfloat16, device="cuda")
+
+    def allocations(r):
+        before = torch.cuda.memory_stats()["allocation.all.allocated"]
+        lc.linear(x, w, residual=r, out=out)
+        return torch.cuda.memory_stats()["allocation.all.allocated"] - before
+    lc.linear(x, w, residual=res, out=out)
+    want = out.clone()
+    plain = res.contiguous()
+    assert allocations(res) == allocations(plain) + 1
+    assert torch.equal(lc.linear(x, w, residual=res.contiguous()), want)
