@@ -505,7 +505,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       const int sfa_atom = (2 * tl.mt + (int)rank) * p.k_atoms;
       const int sfb_atom0 = (tl.n0 >> 7) * p.k_atoms;
       const int sfb_atom1 = sfb_atom0 + p.k_atoms;
-      // this CTA's half of the tile's B rows; the narrow tiles use a 96-row box
+      // this CTA's half of the tile's B rows; narrower tiles use a box of half their width
       const bool narrow = kAlt && (tl.buf == 1 || p.tile_w > 0);
       const int b_row = tl.n0 + (int)rank * (tl.w >> 1);
       const CUtensorMap* mb = narrow ? &map_b_narrow : &map_b;

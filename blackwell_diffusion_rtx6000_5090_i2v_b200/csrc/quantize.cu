@@ -458,10 +458,13 @@ int zero_swizzle_padding(uint8_t* swz, int64_t rows, int64_t cols, cudaStream_t 
   return NVFP4_OK;
 }
 
-// The rows form takes rows that one CTA spans with at least three quarters of its threads, and
-// enough of them for kRows at a time.  Wider rows stay with the flat form, whose CTAs read one
-// contiguous piece each: amax + pack of [27280, 14336] 291 us against 302-350 us with five CTAs side
-// by side on a row; of [27280, 3072] 77.8 us (flat, two memsets) against 71.7 us (rows).
+// The rows form takes rows that one CTA of kPackThreads spans with at least three quarters of its threads
+// (1152 to 3072 columns), and enough of them for kRows at a time: [27280, 3072] amax + pack 77.8 us flat with
+// its two memsets, 71.7 rows.  Much wider rows are better off in the flat form, whose CTAs read one contiguous
+// piece each ([27280, 14336] 291 us, 302-350 with five CTAs side by side on a row).  Where the line should
+// lie in between is open: CTAs of 320 threads would take 4096 and 5120 columns in 98 and 125 us instead of 104
+// and 127 ([32760, .], 16 instead of 21 and 18 instead of 23 at 4095 rows), the memsets among it, but 3072
+// in 77 instead of 74.
 bool rows_form(int64_t rows, int64_t cols, bool swz, int* threads) {
   const int64_t units = swz ? sf_k_atoms(cols) * 4 : cols / kBlock;
   *threads = (int)((units + 31) / 32 * 32);

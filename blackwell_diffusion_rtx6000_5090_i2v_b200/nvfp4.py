@@ -188,7 +188,8 @@ class FP4Tensor:
         """The packed form of ``input.t()`` for a contiguous bf16 ``[rows, cols]`` matrix, without the
         transposed copy (additive; the operands of the gradient GEMMs).  ``[cols, K]`` with ``K`` =
         rows rounded up to 32, zeros appended; ``cols`` a multiple of 8.  ``amax``: as for
-        :meth:`from_bfloat16`.  Carries no linear scales."""
+        :meth:`from_bfloat16`.  Carries no linear scales.  For programs that keep such an operand; the
+        linear's own backward makes its operands inside one library call."""
         if input.dtype != torch.bfloat16:
             raise RuntimeError("[s4] [nvfp4] [tensor] Input must be BFloat16")
         if not input.is_cuda:

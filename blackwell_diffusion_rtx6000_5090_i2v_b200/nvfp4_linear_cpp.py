@@ -30,7 +30,8 @@ _weight_cache: dict = {}
 
 def quantized_weight(weight: torch.Tensor) -> FP4Tensor:
     """NVFP4 copy of a ``[N, K]`` bf16 weight, reused until the tensor is
-    modified in place, reallocated or freed."""
+    modified in place, reallocated or freed.  A write that its version count does not record
+    (through ``weight.data``, by a kernel given the pointer, by a graph replay) is not noticed."""
     try:
         version = weight._version
     except RuntimeError:

@@ -159,8 +159,8 @@ NVFP4_API int nvfp4_linear_backward_bf16(const void* dy_bf16, const void* x_bf16
                                const float* w_amax_dev, int64_t M, int64_t N, int64_t K, void* dx_bf16,
                                void* dw_bf16, void* workspace, int* status_dev, void* stream);
 
-/* Which N tiling nvfp4_gemm uses: 0 = chosen per shape (the default; today always uniform),
- * 1 = uniform 256-wide tiles, 2 = 448-column pairs of a 256-wide and a 192-wide tile (two
+/* Which N tiling nvfp4_gemm uses: 0 = chosen per shape (the default: 256-wide tiles, or 192-, 128-
+ * or 64-wide ones where a grid of at most two waves leaves SMs idle), 1 = uniform 256-wide tiles, 2 = 448-column pairs of a 256-wide and a 192-wide tile (two
  * disjoint accumulators in tensor memory: no hand-off between consecutive tiles, 8 % more
  * operand bytes per flop; measured 3-8 % slower than uniform on B200, kept selectable).
  * Process-wide; results do not depend on it: every output element is the same sum over K
