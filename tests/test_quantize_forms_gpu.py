@@ -99,3 +99,18 @@ def test_given_buffers_nothing_is_allocated(rows, cols):
     assert count() == before
     assert torch.equal(t.quantized_data(), want.quantized_data())
     assert torch.equal(t.scale_factors_swizzled(), want.scale_factors_swizzled())
+
+
+@pytest.mark.parametrize("rows,cols", [(33, 512), (700, 1024), (1000, 1280), (2000, 1536), (6000, 3072)])
+@pytest.mark.parametrize("linear", [True, False])
+def test_scale_layouts_that_are_not_wanted(oracle, rows, cols, linear):
+    from blackwell_diffusion_rtx6000_5090_i2v_b200 import nvfp4 as nv
+    x = student_t_bf16((rows, cols), 8)
+    packed, scales, amax = oracle.quantize(bits_of(x))
+    for kw in ({}, {"amax": torch.full((1,), amax, device="cuda")}):
+        t = nv.FP4Tensor.from_bfloat16(x.cuda(), linear_scales=linear, swizzled_scales=not linear, **kw)
+        assert np.array_equal(t.quantized_data().cpu().numpy(), packed.reshape(-1))
+        assert (t._scales is None, t._scales_swz is None) == (not linear, linear)
+        assert np.array_equal(t.scale_factors_swizzled().cpu().numpy(), oracle.swizzle_scales(scales, cols))
+        if linear:
+            assert np.array_equal(t.scale_factors().cpu().numpy(), scales.reshape(-1))
