@@ -33,6 +33,10 @@
 //
 // Sweep 1 walks the groups forwards and sweep 2 walks them backwards with an evict-first
 // hint: the tail of x that sweep 1 left in L2 (126 MB) is what sweep 2 reads first.
+#include <atomic>
+
+#include <cooperative_groups.h>
+
 #include "nvfp4_common.cuh"
 
 namespace nvfp4 {
@@ -493,6 +497,197 @@ norm_mod_kernel(const NormArgs p) {
   }
 }
 
+// Both sweeps in one launch, for tensors that the GPU's shared memory holds: every CTA has its rows
+// there from the first bulk copy on, puts h in their place, and packs h once the grid has met and the maximum
+// is known.  x is read once, h computed once, and a memset and a launch go.  The arithmetic is that of the
+// two sweeps, in their order.
+constexpr int kMaxGroups = 16;            // row groups of a CTA
+
+template <int kJ, bool kAffine, bool kMod>
+__global__ void __launch_bounds__(kMaxThreads)
+norm_mod_resident(const NormArgs p, int per_cta, unsigned* partial) {
+  constexpr int kR = RowsPerIter<kJ>::value;
+  constexpr int kV = 2 * kR;
+  extern __shared__ __align__(128) uint8_t rows_smem[];     // per_cta groups of kR rows
+  __shared__ __align__(16) float red[2][kV][kMaxWarps];
+  __shared__ unsigned red_max[kMaxWarps];
+  __shared__ float enc_tab[128];
+  __shared__ __align__(8) uint64_t full[kMaxGroups];
+  __shared__ int abort_flag;
+  const int T = blockDim.x;
+  const int warps = T >> 5;
+  const int units = p.cols >> 4;
+  const uint32_t row_bytes = (uint32_t)p.cols * 2u;
+  const int64_t row_first = (int64_t)blockIdx.x * per_cta * kR;
+  const int my_rows = (int)(p.rows - row_first < (int64_t)per_cta * kR ? p.rows - row_first : (int64_t)per_cta * kR);
+  const int my_groups = (my_rows + kR - 1) / kR;
+
+  if (threadIdx.x == 0) {
+    abort_flag = 0;
+    for (int s = 0; s < my_groups; ++s) mbar_init(smem_u32(&full[s]), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int s = 0; s < my_groups; ++s) {
+      const int n = my_rows - s * kR < kR ? my_rows - s * kR : kR;
+      const uint32_t bytes = (uint32_t)n * row_bytes, bar = smem_u32(&full[s]);
+      mbar_expect_tx(bar, bytes);
+      bulk_load(smem_u32(rows_smem) + (uint32_t)(s * kR) * row_bytes,
+                reinterpret_cast<const uint8_t*>(p.x) + (row_first + s * kR) * row_bytes, bytes, bar, 1);
+    }
+  }
+  for (int i = threadIdx.x; i < 2 * kV * kMaxWarps; i += T) (&red[0][0][0])[i] = 0.0f;
+
+  bool live[kJ];
+  float2 cw[kAffine ? kJ : 1][8], cb[kAffine ? kJ : 1][8];
+  float2 cs[kMod ? kJ : 1][8], ct[kMod ? kJ : 1][8];
+  int64_t swz_kb[kJ];
+  const bool has_w = kAffine && p.w, has_b = kAffine && p.b, has_s = kMod && p.scale, has_t = kMod && p.shift;
+#pragma unroll
+  for (int j = 0; j < kJ; ++j) {
+    const int u = threadIdx.x + j * T;
+    live[j] = u < units;
+    const int col = live[j] ? u * 16 : 0;
+    swz_kb[j] = (int64_t)(u >> 2) * kSfAtomBytes + (u & 3);
+    if (has_w) load16(p.w + col, cw[j]);
+    if (has_b) load16(p.b + col, cb[j]);
+    if (has_s) {
+      load16(p.scale + col, cs[j]);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) cs[j][e] = f2_add(make_float2(1.0f, 1.0f), cs[j][e]);
+    }
+    if (has_t) load16(p.shift + col, ct[j]);
+  }
+  // what only pads the swizzled layout: whole rows as words, and the K-blocks past the end of every row
+  if (p.sf_swz) {
+    const int64_t words = (int64_t)p.pad_rows * p.k_atoms;
+    for (int64_t i = (int64_t)blockIdx.x * T + threadIdx.x; i < words; i += (int64_t)gridDim.x * T) {
+      const int64_t row = p.rows + i / p.k_atoms, atom = i % p.k_atoms;
+      *reinterpret_cast<uint32_t*>(p.sf_swz + sf_swizzled_offset(row, atom * 4, p.k_atoms)) = 0u;
+    }
+    const int pad_kb = (int)p.k_atoms * 4 - units;
+    for (int i = threadIdx.x; i < my_rows * pad_kb; i += T)
+      p.sf_swz[sf_swizzled_offset(row_first + i / pad_kb, units + i % pad_kb, p.k_atoms)] = 0;
+  }
+  __syncthreads();
+
+  uint32_t amax_t = 0u;
+  const float cols_f = (float)p.cols;
+  for (int g = 0; g < my_groups; ++g) {
+    wait_group(smem_u32(&full[g]), 0u, &abort_flag, p.status);
+    uint8_t* group_ptr = rows_smem + (size_t)(g * kR) * row_bytes;
+    bool row_ok[kR];
+    uint32_t xp[kR][kJ][8];
+    float pivot[kR];
+#pragma unroll
+    for (int r = 0; r < kR; ++r) {
+      row_ok[r] = g * kR + r < my_rows;
+      const uint4* src = reinterpret_cast<const uint4*>(group_ptr + (size_t)r * row_bytes);
+      pivot[r] = (!p.rms && row_ok[r]) ? bf16lo_to_f32(*reinterpret_cast<const uint32_t*>(src)) : 0.0f;
+#pragma unroll
+      for (int j = 0; j < kJ; ++j) {
+        const bool on = live[j] && row_ok[r];
+        const int u = threadIdx.x + j * T;
+        const uint4 a = on ? src[2 * u] : make_uint4(0, 0, 0, 0);
+        const uint4 b = on ? src[2 * u + 1] : make_uint4(0, 0, 0, 0);
+        xp[r][j][0] = a.x; xp[r][j][1] = a.y; xp[r][j][2] = a.z; xp[r][j][3] = a.w;
+        xp[r][j][4] = b.x; xp[r][j][5] = b.y; xp[r][j][6] = b.z; xp[r][j][7] = b.w;
+      }
+    }
+    float acc[kV];
+#pragma unroll
+    for (int r = 0; r < kR; ++r) {
+      const float2 p2 = make_float2(pivot[r], pivot[r]);
+      float2 s1 = make_float2(0.0f, 0.0f), s2 = make_float2(0.0f, 0.0f);
+#pragma unroll
+      for (int j = 0; j < kJ; ++j) {
+        if (live[j] && row_ok[r]) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const float2 d = f2_sub(bf16x2_to_f2(xp[r][j][e]), p2);
+            s1 = f2_add(s1, d);
+            s2 = f2_fma(d, d, s2);
+          }
+        }
+      }
+      acc[2 * r] = s1.x + s1.y;
+      acc[2 * r + 1] = s2.x + s2.y;
+    }
+    cta_sum<kV>(acc, red[g & 1], warps);
+#pragma unroll
+    for (int r = 0; r < kR; ++r) {
+      const float m1 = acc[2 * r] / cols_f;
+      const float var = fmaxf(acc[2 * r + 1] / cols_f - m1 * m1, 0.0f);
+      const float mean = p.rms ? 0.0f : pivot[r] + m1;
+      const float rstd = rsqrtf((p.rms ? acc[2 * r + 1] / cols_f : var) + p.eps);
+      const float2 m2 = make_float2(mean, mean), r2 = make_float2(rstd, rstd);
+      uint4* dst = reinterpret_cast<uint4*>(group_ptr + (size_t)r * row_bytes);
+#pragma unroll
+      for (int j = 0; j < kJ; ++j) {
+        const int u = threadIdx.x + j * T;
+        uint32_t hp[8];
+        const uint32_t a2 = normalize16<kAffine, kMod>(
+            xp[r][j], m2, r2, cw[kAffine ? j : 0], cb[kAffine ? j : 0], cs[kMod ? j : 0], ct[kMod ? j : 0], has_w,
+            has_b, has_s, has_t, hp);
+        if (live[j] && row_ok[r]) {
+          amax_t = bf16x2_max_abs(amax_t, a2);
+          dst[2 * u] = make_uint4(hp[0], hp[1], hp[2], hp[3]);
+          dst[2 * u + 1] = make_uint4(hp[4], hp[5], hp[6], hp[7]);
+        }
+      }
+    }
+  }
+
+  // the maximum of the CTA, then of the grid
+  unsigned bits = __reduce_max_sync(0xffffffffu,
+                                    __float_as_uint(fmaxf(bf16lo_to_f32(amax_t), bf16hi_to_f32(amax_t))));
+  if ((threadIdx.x & 31) == 0) red_max[threadIdx.x >> 5] = bits;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < warps; ++w) bits = max(bits, red_max[w]);
+    partial[blockIdx.x] = bits;
+  }
+  cooperative_groups::this_grid().sync();
+  bits = 0u;
+  for (unsigned i = threadIdx.x; i < gridDim.x; i += T) bits = max(bits, load_u32(partial + i));
+  bits = __reduce_max_sync(0xffffffffu, bits);
+  if ((threadIdx.x & 31) == 0) red_max[threadIdx.x >> 5] = bits;
+  __syncthreads();
+  for (int w = 0; w < warps; ++w) bits = max(bits, red_max[w]);
+  const float s_enc = global_encode_scale(__uint_as_float(bits));
+  const float s_dec = __fdiv_rn(1.0f, s_enc);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *p.amax_out = bits;
+    if (p.gscale_out) *p.gscale_out = s_dec;
+  }
+  fill_encode_table(enc_tab, s_dec);
+  __syncthreads();
+
+#pragma unroll 2
+  for (int r = 0; r < my_rows; ++r) {
+    const int64_t row = row_first + r;
+    const uint4* src = reinterpret_cast<const uint4*>(rows_smem + (size_t)r * row_bytes);
+    const int64_t swz_row = (row >> 7) * (int64_t)p.k_atoms * kSfAtomBytes + (row & 31) * 16 + ((row >> 5) & 3) * 4;
+#pragma unroll
+    for (int j = 0; j < kJ; ++j) {
+      if (!live[j]) continue;
+      const int u = threadIdx.x + j * T;
+      const uint4 a = src[2 * u], b = src[2 * u + 1];     // this thread's own writes
+      const uint32_t h[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+      uint32_t a2 = 0u, sf;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) a2 = bf16x2_max_abs(a2, h[e]);
+      const uint2 out = pack_block(h, a2, s_enc, enc_tab, sf);
+      __stcs(reinterpret_cast<uint2*>(p.packed) + row * units + u, out);
+      if (p.sf_lin) p.sf_lin[row * units + u] = (uint8_t)sf;
+      if (p.sf_swz) p.sf_swz[swz_row + swz_kb[j]] = (uint8_t)sf;
+    }
+  }
+  if (abort_flag) {
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000LL) {
+    }
+  }
+}
+
 int check_args(const void* x, int64_t rows, int64_t cols) {
   if (rows < 0 || cols <= 0 || cols % kBlock != 0 || cols > kMaxJ * 16 * kMaxThreads ||
       rows >= ((int64_t)1 << 31))
@@ -505,14 +700,15 @@ int check_args(const void* x, int64_t rows, int64_t cols) {
 bool vec_ok(const float* p) { return aligned16(p); }
 
 // Blocks per thread (1 or 2) and threads per CTA (a multiple of 32) for a row of `units`
-// 16-element blocks.
-void shape_for(int units, int* j, int* threads) {
+// 16-element blocks and this many kinds of per-column vectors (affine, modulation).
+void shape_for(int units, int kinds, int* j, int* threads) {
   int J = 1;
   while (J < kMaxJ && units > J * kMaxThreads) J *= 2;
   // two blocks per thread whenever the row is long enough for two warps: the per-row
-  // bookkeeping is then shared by 32 elements instead of 16 (measured 17-20 % faster)
+  // bookkeeping is then shared by 32 elements instead of 16 (measured 17-20 % faster).  Not with all four
+  // vectors, which take 128 registers and leave none for the row (4 KB of spills in every group).
 #ifndef NVFP4_NORM_FORCE_J1
-  if (units % 2 == 0 && units / 2 >= 64) J = 2;
+  if (units % 2 == 0 && units / 2 >= 64 && kinds < 2) J = 2;
 #endif
   const int per = (units + J - 1) / J;
   *j = J;
@@ -549,11 +745,75 @@ int launch_variant(const NormArgs& a, int threads, cudaStream_t st) {
   return launch_dependent(kernel, dim3(grid), (unsigned)threads, smem, 1, st, a);
 }
 
+// Launches the one-launch form if the rows fit; *done says whether.
+template <int kJ, bool kAffine, bool kMod>
+int launch_resident(const NormArgs& a, int threads, unsigned* partial, cudaStream_t st, bool* done) {
+  auto kernel = norm_mod_resident<kJ, kAffine, kMod>;
+  constexpr int kR = RowsPerIter<kJ>::value;
+  constexpr int kSmemMax = 200 << 10, kSmemSm = 228 << 10, kSmemStatic = 2 << 10;   // reserve and statics of a CTA
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return NVFP4_ERR_BAD_ARG;
+  // CTAs per SM that the registers allow, by warps per CTA; asked for once
+  static std::atomic<int> known[64][kMaxWarps + 1];
+  int by_regs = known[dev][threads / 32].load(std::memory_order_acquire);
+  if (by_regs == 0) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&by_regs, kernel, threads, 0) != cudaSuccess || by_regs < 1)
+      return NVFP4_ERR_LAUNCH_FAILED;
+    known[dev][threads / 32].store(by_regs, std::memory_order_release);
+  }
+  const int64_t groups = (a.rows + kR - 1) / kR;
+  for (int per = 1; per <= kMaxGroups; ++per) {
+    const int64_t smem = (int64_t)per * kR * a.cols * 2;
+    if (smem > kSmemMax) break;
+    const int64_t by_smem = kSmemSm / (smem + kSmemStatic);
+    const int64_t at_a_time = sm_count() * (by_smem < by_regs ? by_smem : by_regs);
+    const int64_t ctas = (groups + per - 1) / per;
+    if (ctas > at_a_time || ctas > NVFP4_AMAX_PARTIALS) continue;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeCooperative;
+    attr.val.cooperative = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a, per, partial);
+    if (e == cudaSuccess) {
+      *done = true;
+      return NVFP4_OK;
+    }
+    cudaGetLastError();
+    if (e != cudaErrorCooperativeLaunchTooLarge) return NVFP4_ERR_LAUNCH_FAILED;
+    return NVFP4_OK;       // fewer SMs than the device has: the two sweeps run on any number
+  }
+  return NVFP4_OK;
+}
+
+int try_resident(const NormArgs& a, unsigned* partial, cudaStream_t st, bool* done) {
+  int J, threads;
+  const bool affine = a.w || a.b, mod = a.scale || a.shift;
+  shape_for(a.cols / 16, affine + mod, &J, &threads);
+#define NVFP4_NORM_CASE(JJ)                                                                       \
+  if (J == JJ) {                                                                                  \
+    if (affine && mod) return launch_resident<JJ, true, true>(a, threads, partial, st, done);     \
+    if (affine) return launch_resident<JJ, true, false>(a, threads, partial, st, done);           \
+    if (mod) return launch_resident<JJ, false, true>(a, threads, partial, st, done);              \
+    return launch_resident<JJ, false, false>(a, threads, partial, st, done);                      \
+  }
+  NVFP4_NORM_CASE(1)
+  NVFP4_NORM_CASE(2)
+#undef NVFP4_NORM_CASE
+  return NVFP4_ERR_BAD_ARG;
+}
+
 template <bool kQuantize>
 int launch(const NormArgs& a, cudaStream_t st) {
   int J, threads;
-  shape_for(a.cols / 16, &J, &threads);
   const bool affine = a.w || a.b, mod = a.scale || a.shift;
+  shape_for(a.cols / 16, affine + mod, &J, &threads);
 #define NVFP4_NORM_CASE(JJ)                                                           \
   if (J == JJ) {                                                                      \
     if (affine && mod) return launch_variant<kQuantize, JJ, true, true>(a, threads, st);   \
@@ -644,6 +904,42 @@ int nvfp4_norm_mod_quantize_bf16(const void* x_bf16, int64_t rows, int64_t cols,
   a.gscale_out = global_scale_dev;
   a.status = status_dev;
   return launch<true>(a, st);
+}
+
+int nvfp4_norm_mod_bf16(const void* x_bf16, int64_t rows, int64_t cols, const float* weight, const float* bias,
+                        const float* scale, const float* shift, int rms, float eps, float* row_stats,
+                        float* amax_dev, uint8_t* packed, uint8_t* scales_linear, uint8_t* scales_swizzled,
+                        float* global_scale_dev, float* partials, int* status_dev, void* stream) {
+  int rc = check_args(x_bf16, rows, cols);
+  if (rc != NVFP4_OK) return rc;
+  if (!amax_dev || (rows > 0 && !packed)) return NVFP4_ERR_BAD_ARG;
+  if ((reinterpret_cast<uintptr_t>(packed) & 7u) || !vec_ok(weight) || !vec_ok(bias) || !vec_ok(scale) ||
+      !vec_ok(shift))
+    return NVFP4_ERR_BAD_ALIGN;
+  rc = check_device_sm100();
+  if (rc != NVFP4_OK) return rc;
+  if (rows > 0 && partials && (reinterpret_cast<uintptr_t>(scales_swizzled) & 3u) == 0) {
+    NormArgs a{};
+    a.x = reinterpret_cast<const uint4*>(x_bf16);
+    a.rows = rows; a.cols = (int)cols;
+    a.w = weight; a.b = bias; a.scale = scale; a.shift = shift;
+    a.rms = rms; a.eps = eps;
+    a.amax_out = reinterpret_cast<unsigned*>(amax_dev);
+    a.packed = reinterpret_cast<uint32_t*>(packed);
+    a.sf_lin = scales_linear; a.sf_swz = scales_swizzled;
+    a.k_atoms = (uint32_t)sf_k_atoms(cols);
+    a.pad_rows = (int)(sf_row_tiles(rows) * 128 - rows);
+    a.gscale_out = global_scale_dev;
+    a.status = status_dev;
+    bool done = false;
+    rc = try_resident(a, reinterpret_cast<unsigned*>(partials), reinterpret_cast<cudaStream_t>(stream), &done);
+    if (rc != NVFP4_OK || done) return rc;
+  }
+  rc = nvfp4_norm_mod_amax_bf16(x_bf16, rows, cols, weight, bias, scale, shift, rms, eps, row_stats, amax_dev, nullptr,
+                                status_dev, stream);
+  if (rc != NVFP4_OK) return rc;
+  return nvfp4_norm_mod_quantize_bf16(x_bf16, rows, cols, weight, bias, scale, shift, row_stats, amax_dev, packed,
+                                      scales_linear, scales_swizzled, global_scale_dev, status_dev, stream);
 }
 
 }  // extern "C"

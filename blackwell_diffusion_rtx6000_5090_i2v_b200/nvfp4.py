@@ -259,7 +259,7 @@ class FP4Tensor:
                     raise RuntimeError("[s4] [nvfp4] [tensor] out buffers do not match the input")
                 self._amax, self._gscale, self._data = out.amax, out.gscale, out.data
                 self._scales = out.scales if linear_scales else None
-                self._scales_swz, stats = out.scales_swz, out.stats
+                self._scales_swz, stats, partials = out.scales_swz, out.stats.data_ptr(), out.partials.data_ptr()
             else:
                 self._amax = torch.empty(1, dtype=torch.float32, device=dev)
                 self._gscale = torch.empty(1, dtype=torch.float32, device=dev)
@@ -268,19 +268,28 @@ class FP4Tensor:
                                 if linear_scales else None)
                 self._scales_swz = torch.empty(N.swizzled_scale_bytes(rows, cols),
                                                dtype=torch.uint8, device=dev)
-                stats = torch.empty(rows, 2, dtype=torch.float32, device=dev)
+                work = torch.empty(rows * 2 + N.AMAX_PARTIALS, dtype=torch.float32, device=dev)
+                stats = work.data_ptr()
+                partials = stats + rows * 8
             normed = torch.empty_like(xc) if return_normed else None
             st = N.stream_ptr()
             status = N.ptr(N.status_word(dev))
             w_, b_, sc_, sh_ = (N.ptr(v) for v in vecs)
+            if amax_hook is None and normed is None:
+                N.check(N.lib.nvfp4_norm_mod_bf16(N.ptr(xc), rows, cols, w_, b_, sc_, sh_, 1 if rms else 0,
+                                                  float(eps), stats, N.ptr(self._amax), N.ptr(self._data),
+                                                  N.ptr(self._scales), N.ptr(self._scales_swz),
+                                                  N.ptr(self._gscale), partials, status, st),
+                        "[tensor] norm+quantize")
+                return self
             N.check(N.lib.nvfp4_norm_mod_amax_bf16(N.ptr(xc), rows, cols, w_, b_, sc_, sh_,
-                                                   1 if rms else 0, float(eps), N.ptr(stats),
+                                                   1 if rms else 0, float(eps), stats,
                                                    N.ptr(self._amax), N.ptr(normed), status, st),
                     "[tensor] norm+amax")
             if amax_hook is not None:
                 amax_hook(self._amax)
             N.check(N.lib.nvfp4_norm_mod_quantize_bf16(N.ptr(xc), rows, cols, w_, b_, sc_, sh_,
-                                                       N.ptr(stats), N.ptr(self._amax),
+                                                       stats, N.ptr(self._amax),
                                                        N.ptr(self._data), N.ptr(self._scales),
                                                        N.ptr(self._scales_swz),
                                                        N.ptr(self._gscale), status, st),

@@ -212,6 +212,16 @@ NVFP4_API int nvfp4_norm_mod_quantize_bf16(const void* x_bf16, int64_t rows, int
                                            uint8_t* scales_swizzled, float* global_scale_dev,
                                            int* status_dev, void* stream);
 
+/* Both sweeps in one call, with the same results: for tensors that the GPU's shared memory holds (some
+ * 13 million elements) one launch that reads x and computes the result once, else the two above.
+ * partials: NVFP4_AMAX_PARTIALS floats of scratch, nullable (then always the two); row_stats as above. */
+NVFP4_API int nvfp4_norm_mod_bf16(const void* x_bf16, int64_t rows, int64_t cols, const float* weight,
+                                  const float* bias, const float* scale, const float* shift, int rms,
+                                  float eps, float* row_stats, float* amax_dev, uint8_t* packed,
+                                  uint8_t* scales_linear, uint8_t* scales_swizzled,
+                                  float* global_scale_dev, float* partials, int* status_dev,
+                                  void* stream);
+
 /* q/k RMSNorm across heads + rotary embedding in one pass over the QKV linear's output: what
  * the reference block does with separate torch ops between to_qkv and attention
  * (fx/src/s4/models/wan22/wan_transformer.py:91-92,114-115 norm_q/norm_k; :61-75
