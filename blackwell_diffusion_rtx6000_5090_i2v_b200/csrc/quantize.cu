@@ -6,10 +6,15 @@
 // 64-bit packed stores.  Algorithmic bytes per element: 2 (bf16 in) + 0.5
 // (nibbles) + 0.0625 (scale) = 2.5625.
 //
-// Three ways to pack, by shape (quantize_impl, nvfp4_amax_quantize_bf16):
-//   small   amax and packing in one cluster of at most 8 CTAs that holds the tensor in registers
-//   rows    a thread owns one scale block of every row, four rows at a time: rows that one CTA spans
-//   flat    blocks numbered through the tensor: everything else
+// Four ways to pack, by shape (quantize_impl, nvfp4_amax_quantize_bf16):
+//   small     amax and packing in one cluster of at most 8 CTAs that holds the tensor in registers
+//   rows      a thread owns one scale block of every row, four rows at a time: rows that one CTA spans
+//   resident  amax and packing in one cooperative launch that holds the tensor in shared memory
+//   flat      blocks numbered through the tensor: everything else
+#include <atomic>
+
+#include <cooperative_groups.h>
+
 #include "nvfp4_common.cuh"
 
 namespace nvfp4 {
@@ -248,6 +253,9 @@ constexpr int kSmallThreads = 512;
 constexpr int kSmallCtas = 8;            // the portable cluster size
 constexpr int kSmallBlocks = 8;          // most blocks per thread
 constexpr int64_t kSmallMax = (int64_t)kSmallCtas * kSmallThreads * kSmallBlocks;
+// Above four blocks a thread the other forms are faster where they apply: [85, 3072] 4.7 us small, 4.8 rows;
+// [170, 3072] 6.8 small, 4.7 rows, 5.4 resident.
+constexpr int64_t kSmallBest = kSmallMax / 2;
 // Most bytes of swizzled scales, which the cluster zeroes: a few long rows are mostly pad, and a memset
 // has the whole GPU for it ([1, 65536], 1 MB: 9.7 us with memsets and two kernels, 5.0 here; [1, 262144],
 // 4 MB: 10.3 and 12.7; [1, 524288], 8 MB: 10.4 and 23).
@@ -335,6 +343,87 @@ quantize_small_kernel(const uint4* x, uint32_t n_blocks, uint32_t kb_per_row, in
     }
   }
   asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// Resident form: amax and packing of a tensor that the shared memory of the GPU holds.  Bound: HBM and the
+// meeting of the grid between the two.  Every thread copies its blocks there (asynchronously, all on their way
+// at once), takes their maximum, and packs them when the grid's is known: x is read once, in one launch.
+constexpr int kHeldThreads = 512;
+constexpr int kHeldBlocks = 6;           // most blocks per thread: two CTAs of 96 KB an SM
+
+__global__ void __launch_bounds__(kHeldThreads, 2)
+quantize_resident(const uint4* x, uint32_t n_blocks, uint32_t kb_per_row, int per, unsigned* partial, float* amax_out,
+                  uint2* packed, uint8_t* sf_lin, uint8_t* sf_swz, uint32_t swz_vecs, uint32_t k_atoms,
+                  float* gscale_out) {
+  extern __shared__ __align__(16) uint4 held[];       // [block of the thread][half][thread]
+  __shared__ unsigned warp_max[kHeldThreads / 32];
+  __shared__ float enc_tab[128];
+  const int t = threadIdx.x;
+  const uint32_t stride = gridDim.x * kHeldThreads, first = blockIdx.x * kHeldThreads + t;
+  for (int i = 0; i < per; ++i) {
+    const uint32_t b = first + i * stride;
+    if (b < n_blocks) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(held + (2 * i + h) * kHeldThreads + t);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(x + 2 * (size_t)b + h) : "memory");
+      }
+    }
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  // the scale bytes of real blocks go over these zeros once the grid has met
+  for (uint32_t i = first; i < swz_vecs; i += stride) reinterpret_cast<uint4*>(sf_swz)[i] = make_uint4(0, 0, 0, 0);
+  asm volatile("cp.async.wait_all;" ::: "memory");    // a thread reads what it copied, and nothing else
+  uint32_t m2 = 0u;
+  for (int i = 0; i < per; ++i) {
+    if (first + i * stride < n_blocks) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint4 v = held[(2 * i + h) * kHeldThreads + t];
+        m2 = bf16x2_max_abs(bf16x2_max_abs(bf16x2_max_abs(bf16x2_max_abs(m2, v.x), v.y), v.z), v.w);
+      }
+    }
+  }
+  unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(bf16lo_to_f32(m2), bf16hi_to_f32(m2))));
+  if ((t & 31) == 0) warp_max[t >> 5] = m;
+  __syncthreads();
+  if (t < 32) {
+    m = __reduce_max_sync(0xffffffffu, t < kHeldThreads / 32 ? warp_max[t] : 0u);
+    if (t == 0) partial[blockIdx.x] = m;
+  }
+  cooperative_groups::this_grid().sync();
+  m = 0u;
+  for (unsigned i = t; i < gridDim.x; i += kHeldThreads) m = max(m, load_u32(partial + i));
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((t & 31) == 0) warp_max[t >> 5] = m;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < kHeldThreads / 32; ++w) m = max(m, warp_max[w]);
+  const float amax_g = __uint_as_float(m);
+  const float s_enc = global_encode_scale(amax_g);
+  const float s_dec = __fdiv_rn(1.0f, s_enc);
+  if (first == 0) {
+    *amax_out = amax_g;
+    if (gscale_out) *gscale_out = s_dec;
+  }
+  fill_encode_table(enc_tab, s_dec);
+  __syncthreads();
+  for (int i = 0; i < per; ++i) {
+    const uint32_t b = first + i * stride;
+    if (b >= n_blocks) break;
+    const uint4 v0 = held[2 * i * kHeldThreads + t], v1 = held[(2 * i + 1) * kHeldThreads + t];
+    const uint32_t h[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+    uint32_t a2 = 0u, sf;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) a2 = bf16x2_max_abs(a2, h[e]);
+    const uint2 out = pack_block(h, a2, s_enc, enc_tab, sf);
+    __stcs(packed + b, out);
+    if (sf_lin) sf_lin[b] = (uint8_t)sf;
+    if (sf_swz) {
+      const uint32_t row = b / kb_per_row;
+      sf_swz[sf_swizzled_offset(row, b - row * kb_per_row, k_atoms)] = (uint8_t)sf;
+    }
+  }
 }
 
 // ---------------------------------------------------------- dequantize ----
@@ -540,6 +629,44 @@ unsigned amax_grid(int64_t n_vec) {
   return (unsigned)(want < 1 ? 1 : (want > most ? most : want));
 }
 
+// Launches the resident form if the tensor fits; *done says whether.
+int launch_resident(const void* x, int64_t rows, int64_t cols, float* amax, uint8_t* packed, uint8_t* sf_lin,
+                    uint8_t* sf_swz, float* gscale, float* partials, cudaStream_t st, bool* done) {
+  const int64_t n_blocks = rows * cols / kBlock, ctas_max = 2 * (int64_t)sm_count();
+  const int64_t per = (n_blocks + ctas_max * kHeldThreads - 1) / (ctas_max * kHeldThreads);
+  if (per > kHeldBlocks || ctas_max > NVFP4_AMAX_PARTIALS) return NVFP4_OK;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return NVFP4_ERR_BAD_ARG;
+  static std::atomic<bool> allowed[64];
+  if (!allowed[dev].load(std::memory_order_acquire)) {
+    if (cudaFuncSetAttribute(quantize_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kHeldBlocks * kHeldThreads * 32) != cudaSuccess)
+      return NVFP4_ERR_LAUNCH_FAILED;
+    allowed[dev].store(true, std::memory_order_release);
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((n_blocks + per * kHeldThreads - 1) / (per * kHeldThreads)));
+  cfg.blockDim = dim3(kHeldThreads);
+  cfg.dynamicSmemBytes = (size_t)per * kHeldThreads * 32;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeCooperative;
+  attr.val.cooperative = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(
+      &cfg, quantize_resident, reinterpret_cast<const uint4*>(x), (uint32_t)n_blocks, (uint32_t)(cols / kBlock), (int)per,
+      reinterpret_cast<unsigned*>(partials), amax, reinterpret_cast<uint2*>(packed), sf_lin, sf_swz,
+      (uint32_t)(sf_swz ? sf_swizzled_bytes(rows, cols) / 16 : 0), (uint32_t)sf_k_atoms(cols), gscale);
+  if (e == cudaSuccess) {
+    *done = true;
+    return NVFP4_OK;
+  }
+  cudaGetLastError();
+  // fewer SMs than the device has: the other forms run on any number
+  return e == cudaErrorCooperativeLaunchTooLarge ? NVFP4_OK : NVFP4_ERR_LAUNCH_FAILED;
+}
+
 template <int kB>
 int launch_small(const void* x, int64_t rows, int64_t cols, float* amax, uint8_t* packed, uint8_t* sf_lin,
                  uint8_t* sf_swz, float* gscale, int ctas, cudaStream_t st) {
@@ -598,8 +725,9 @@ int nvfp4_amax_quantize_bf16(const void* x, int64_t rows, int64_t cols, float* a
   if (!amax_dev) return NVFP4_ERR_BAD_ARG;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int64_t n_blocks = rows * cols / kBlock;
-  if (n_blocks > 0 && n_blocks <= kSmallMax && aligned16(scales_swizzled) &&
-      (!scales_swizzled || sf_swizzled_bytes(rows, cols) <= kSmallPad)) {
+  const bool small_fits = n_blocks > 0 && n_blocks <= kSmallMax && aligned16(scales_swizzled) &&
+                          (!scales_swizzled || sf_swizzled_bytes(rows, cols) <= kSmallPad);
+  auto small = [&]() {
     // as few blocks per thread as the cluster allows: latency is what counts here
     int ctas = 1;
     while (ctas < kSmallCtas && n_blocks > (int64_t)ctas * kSmallThreads) ctas *= 2;
@@ -608,7 +736,8 @@ int nvfp4_amax_quantize_bf16(const void* x, int64_t rows, int64_t cols, float* a
   launch_small<B>(x, rows, cols, amax_dev, packed, scales_linear, scales_swizzled, global_scale_dev, ctas, st)
     return per <= 1 ? NVFP4_SMALL(1) : per <= 2 ? NVFP4_SMALL(2) : per <= 4 ? NVFP4_SMALL(4) : NVFP4_SMALL(8);
 #undef NVFP4_SMALL
-  }
+  };
+  if (small_fits && n_blocks <= kSmallBest) return small();
   int threads;
   if (n_blocks > 0 && partials && rows_form(rows, cols, scales_swizzled != nullptr, &threads)) {
     const int64_t n_vec = n_blocks * 2;
@@ -632,6 +761,18 @@ int nvfp4_amax_quantize_bf16(const void* x, int64_t rows, int64_t cols, float* a
     a.word_swz = (reinterpret_cast<uintptr_t>(scales_swizzled) & 3u) == 0;
     return launch_rows(a, threads, st);
   }
+  // Widths that the rows form does not take: the resident form where the tensor fits.  Not ahead of the rows
+  // form, whose two kernels overlap what comes before and each other: flat with its memsets, rows, resident us
+  // [512, 4096] 9.3, -, 6.6; [1490, 4096] 14.5, -, 10.5; [2500, 5120] 19.9, -, 16.2; [900, 14336] 20.1, -, 16.4;
+  // [1024, 3072] -, 7.6, 8.6; [4096, 3072] -, 16.2, 16.2, and with the GEMM behind it 37.7 and 41.0.
+  if (n_blocks > 0 && partials && aligned16(scales_swizzled) &&
+      (!scales_swizzled || sf_swizzled_bytes(rows, cols) <= n_blocks * 4)) {
+    bool done = false;
+    rc = launch_resident(x, rows, cols, amax_dev, packed, scales_linear, scales_swizzled, global_scale_dev, partials, st,
+                         &done);
+    if (rc != NVFP4_OK || done) return rc;
+  }
+  if (small_fits) return small();
   rc = nvfp4_amax_bf16(x, rows * cols, amax_dev, stream);
   if (rc != NVFP4_OK) return rc;
   return quantize_impl(x, rows, cols, amax_dev, 0.0f, packed, scales_linear, scales_swizzled,
