@@ -69,6 +69,14 @@ for _name, (_res, _args) in SIGNATURES.items():
     _fn.restype = _res
     _fn.argtypes = _args
 
+_HOST_PATH = os.path.join(_HERE, "_host_calls.so")
+if not os.path.exists(_HOST_PATH):
+    raise ImportError(f"{_HOST_PATH} is missing: build it with "
+                      "`python -m blackwell_diffusion_rtx6000_5090_i2v_b200.build`")
+# Checks, allocations and the library call of the plain case in one native step; each returns None for
+# anything else, which the Python code around it then handles.
+from . import _host_calls as host  # noqa: E402
+
 OK = 0
 ACT_NONE, ACT_GELU_TANH = 0, 1
 AMAX_PARTIALS = 1184        # NVFP4_AMAX_PARTIALS of the header
@@ -124,6 +132,7 @@ def status_word(device: torch.device) -> torch.Tensor:
     if w is None:
         w = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", idx))
         _status_words[idx] = w
+        host.set_status(idx, w)
     return w
 
 

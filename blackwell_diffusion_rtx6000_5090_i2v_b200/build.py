@@ -15,6 +15,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libnvfp4_b200.so")
+HOST = os.path.join(HERE, "_host_calls.so")     # the Python layer's native calls into LIB
 
 NVCC_FLAGS = [
     "-std=c++17", "-O3", "-lineinfo",
@@ -49,9 +50,38 @@ def is_stale() -> bool:
     return any(os.path.getmtime(d) > t for d in deps if os.path.exists(d))
 
 
+def build_host(force: bool = False) -> str:
+    """The extension module that the Python layer calls the library through (needs torch's headers)."""
+    src = os.path.join(CSRC, "host_calls.cpp")
+    deps = [src, os.path.join(HERE, "..", "include", "nvfp4_b200.h")]
+    if not force and os.path.exists(HOST) and all(os.path.getmtime(d) <= os.path.getmtime(HOST) for d in deps):
+        return HOST
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension as ext
+    cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else os.environ.get("CXX", "g++")
+    include = [*ext.include_paths(), sysconfig.get_paths()["include"],
+               os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")]
+    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           "-DTORCH_EXTENSION_NAME=_host_calls", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           *[f for d in include for f in ("-isystem", d)], src, "-o", HOST,
+           "-L", HERE, "-l:libnvfp4_b200.so", "-Wl,-rpath,$ORIGIN",
+           *[f for d in ext.library_paths() for f in ("-L", d)],
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+    subprocess.run(cmd, check=True)
+    return HOST
+
+
 def build_library(force: bool = False, verbose: bool = False) -> str:
-    if not force and not is_stale():
-        return LIB
+    if force or is_stale():
+        _build_cuda(verbose)
+    build_host(force)
+    return LIB
+
+
+def _build_cuda(verbose: bool) -> None:
     nvcc = _nvcc()
     objs = []
     for src in sources():
@@ -64,7 +94,6 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
         objs.append(obj)
     cmd = [nvcc, *_host_cxx(), "-shared", "-o", LIB, *objs, "-cudart", "static"]
     subprocess.run(cmd, check=True)
-    return LIB
 
 
 if __name__ == "__main__":

@@ -322,6 +322,11 @@ def attention_native(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
     """The package's own attention kernel (head dimension 128): ``[Lq, H, D]`` x ``[Lk, H, D]`` ->
     ``[Lq, H, D]`` bf16, non-causal, scale 1/sqrt(D); q, k, v may be strided views (last
     dimension contiguous).  ``amax``: a zeroed one-element fp32 tensor that receives max|o|."""
+    if q.is_cuda:
+        N.status_word(q.device)
+    o = N.host.attention(q, k, v, amax, out)
+    if o is not None:
+        return o
     Lq, H, D = q.shape
     Lk = k.shape[0]
     for t in (q, k, v):

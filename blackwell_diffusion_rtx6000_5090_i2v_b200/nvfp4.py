@@ -84,6 +84,15 @@ class PackedBuffers:
             self.partials = torch.empty(N.AMAX_PARTIALS, dtype=torch.float32, device=self.device)  # quantizer
         self.device = self.data.device       # with its index, as tensors report it
 
+    @property
+    def tensors(self):
+        return [self.data, self.scales, self.scales_swz, self.amax, self.gscale, self.stats, self.partials]
+
+    def holds(self, x: torch.Tensor, linear_scales: bool) -> bool:
+        cols = x.shape[-1] if x.dim() else 0
+        return cols > 0 and self.matches(x.numel() // cols, cols, x.device) and \
+            not (linear_scales and self.scales is None)
+
     def matches(self, rows: int, cols: int, device) -> bool:
         return (rows, cols) == (self.rows, self.cols) and torch.device(device) == self.device
 
@@ -128,6 +137,12 @@ class FP4Tensor:
         self._device = input.device
         n = input.numel()
         self._numel = n
+        if out is None and amax is None and amax_hook is None:
+            made = N.host.quantize(input, linear_scales, swizzled_scales)
+            if made is not None:
+                (self._rows, self._cols, self._data, self._scales, self._scales_swz, self._amax,
+                 self._gscale) = made
+                return self
         with N.device_guard(input.device):
             x = input.contiguous()
             last = x.shape[-1] if x.dim() >= 1 and n > 0 else 0
@@ -233,6 +248,17 @@ class FP4Tensor:
             raise RuntimeError("[s4] [nvfp4] [tensor] Input must be BFloat16")
         if not x.is_cuda:
             raise RuntimeError("[s4] [nvfp4] [tensor] Input must be on CUDA device")
+        if not return_normed and amax_hook is None and (out is None or out.holds(x, linear_scales)):
+            N.status_word(x.device)
+            made = N.host.norm_quantize(x, weight, bias, scale, shift, rms, eps, linear_scales,
+                                        None if out is None else out.tensors)
+            if made is not None:
+                self = object.__new__(FP4Tensor)
+                self._shape, self._mode, self._device = list(x.shape), QuantizationMode.block_1d, x.device
+                self._numel = x.numel()
+                (self._rows, self._cols, self._data, self._scales, self._scales_swz, self._amax,
+                 self._gscale) = made
+                return self
         cols = x.shape[-1]
         if cols % FP4_BLOCK_SIZE != 0 or cols > 16384:
             raise RuntimeError("[s4] [nvfp4] [tensor] fused norm needs cols % 16 == 0, cols <= 16384")
@@ -343,6 +369,10 @@ class FP4Tensor:
     # ------------------------------------------------------------ access --
     def to_bfloat16(self) -> torch.Tensor:
         """Dequantize (fx/src/s4/nvfp4/tensor.h:53-72)."""
+        if self._numel == self._rows * self._cols and self._scales is not None:
+            flat = N.host.dequantize(self._data, self._scales, self._amax, self._rows, self._cols, self._shape)
+            if flat is not None:
+                return flat
         with N.device_guard(self._device):
             flat = torch.empty(self._rows * self._cols, dtype=torch.bfloat16, device=self._device)
             scales = self.scale_factors_full()
@@ -425,6 +455,11 @@ def _gemm_packed(a: FP4Tensor, b: FP4Tensor, alpha: float, beta: float,
         raise RuntimeError("[s4] [nvfp4] [gemm] Operands must be on the same device")
     if K % 32 != 0 or Nn % 8 != 0:
         raise RuntimeError("[s4] [nvfp4] [gemm] K must be a multiple of 32 and N of 8")
+    N.status_word(dev)
+    done = N.host.gemm(a._data, b._data, a.scale_factors_swizzled(), b.scale_factors_swizzled(), a._gscale,
+                       b._gscale, M, Nn, K, alpha, beta, c, bias, gate, bool(gelu), out, out_amax)
+    if done is not None:
+        return done if out is None else out
     if out is None:
         out = torch.empty((M, Nn), dtype=torch.bfloat16, device=dev)
     elif out.shape != (M, Nn) or out.dtype != torch.bfloat16 or not out.is_contiguous():

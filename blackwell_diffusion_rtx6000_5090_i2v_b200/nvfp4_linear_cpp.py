@@ -50,6 +50,19 @@ def quantized_weight(weight: torch.Tensor) -> FP4Tensor:
     return q
 
 
+def _packed_before(weight: torch.Tensor) -> Optional[FP4Tensor]:
+    """What :func:`quantized_weight` would return without packing anything, or None."""
+    hit = _weight_cache.get(id(weight))
+    if hit is None:
+        return None
+    ref, version, ptr, q = hit
+    try:
+        same = ref() is weight and version == weight._version and ptr == weight.data_ptr()
+    except RuntimeError:
+        return None
+    return q if same and q._scales_swz is not None else None
+
+
 def _transposable(t: torch.Tensor) -> bool:
     # what the transposing quantizer reads in place; the rest goes through a transposed copy
     return t.is_contiguous() and t.numel() > 0 and t.size(1) % 8 == 0 and t.data_ptr() % 16 == 0
@@ -122,6 +135,12 @@ def linear(input: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
     """``residual + gate * act(input @ weight.T + bias)`` over flattened batch
     dims: quantize the activation, one tcgen05 GEMM with everything else fused
     into its epilogue."""
+    if out is None:
+        q = _packed_before(weight)
+        if q is not None:
+            y = N.host.linear(input, weight, q._data, q._scales_swz, q._gscale, bias, gate, residual, bool(gelu))
+            if y is not None:
+                return y
     if input.dim() < 2:
         raise RuntimeError(f"{_PFX} Input must be at least 2D, got {input.dim()}D")
     if weight.dim() != 2:
