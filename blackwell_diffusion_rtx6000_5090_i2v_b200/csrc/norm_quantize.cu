@@ -745,51 +745,71 @@ int launch_variant(const NormArgs& a, int threads, cudaStream_t st) {
   return launch_dependent(kernel, dim3(grid), (unsigned)threads, smem, 1, st, a);
 }
 
+// Row groups per CTA of the one-launch form: the least with which all CTAs are on the GPU at a time, or 0.  How many
+// an SM holds is the runtime's answer for the dynamic size at hand: a sum of shared-memory constants that was 256
+// bytes short gave [3800, 4096] a launch that is refused, which an eager call survives by way of the two sweeps and a
+// stream capture does not.  The last answer is kept per thread, so that only a change of shape asks.
+template <typename Kernel>
+int groups_per_cta(Kernel kernel, int dev, int threads, int64_t groups, int64_t group_bytes) {
+  constexpr int kSmemMax = 200 << 10, kSmemSm = 228 << 10;
+  struct Last {
+    Kernel kernel;             // all variants have the one type
+    int dev, threads, per;
+    int64_t groups, group_bytes;
+  };
+  static thread_local Last last{};
+  if (last.kernel == kernel && last.dev == dev && last.threads == threads && last.groups == groups && last.group_bytes == group_bytes)
+    return last.per;
+  int found = 0;
+  for (int per = 1; per <= kMaxGroups && per * group_bytes <= kSmemMax && !found; ++per) {
+    const int64_t ctas = (groups + per - 1) / per, bytes = per * group_bytes;
+    // more than the rows alone leave room for: not worth the question
+    if (ctas > NVFP4_AMAX_PARTIALS || ctas > sm_count() * (kSmemSm / bytes)) continue;
+    int an_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&an_sm, kernel, threads, (size_t)bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    if (ctas <= (int64_t)sm_count() * an_sm) found = per;
+  }
+  last = {kernel, dev, threads, found, groups, group_bytes};
+  return found;
+}
+
 // Launches the one-launch form if the rows fit; *done says whether.
 template <int kJ, bool kAffine, bool kMod>
 int launch_resident(const NormArgs& a, int threads, unsigned* partial, cudaStream_t st, bool* done) {
   auto kernel = norm_mod_resident<kJ, kAffine, kMod>;
   constexpr int kR = RowsPerIter<kJ>::value;
-  constexpr int kSmemMax = 200 << 10, kSmemSm = 228 << 10, kSmemStatic = 2 << 10;   // reserve and statics of a CTA
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return NVFP4_ERR_BAD_ARG;
-  // CTAs per SM that the registers allow, by warps per CTA; asked for once
-  static std::atomic<int> known[64][kMaxWarps + 1];
-  int by_regs = known[dev][threads / 32].load(std::memory_order_acquire);
-  if (by_regs == 0) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&by_regs, kernel, threads, 0) != cudaSuccess || by_regs < 1)
+  static std::atomic<bool> allowed[64];
+  if (!allowed[dev].load(std::memory_order_acquire)) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 << 10) != cudaSuccess)
       return NVFP4_ERR_LAUNCH_FAILED;
-    known[dev][threads / 32].store(by_regs, std::memory_order_release);
+    allowed[dev].store(true, std::memory_order_release);
   }
-  const int64_t groups = (a.rows + kR - 1) / kR;
-  for (int per = 1; per <= kMaxGroups; ++per) {
-    const int64_t smem = (int64_t)per * kR * a.cols * 2;
-    if (smem > kSmemMax) break;
-    const int64_t by_smem = kSmemSm / (smem + kSmemStatic);
-    const int64_t at_a_time = sm_count() * (by_smem < by_regs ? by_smem : by_regs);
-    const int64_t ctas = (groups + per - 1) / per;
-    if (ctas > at_a_time || ctas > NVFP4_AMAX_PARTIALS) continue;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeCooperative;
-    attr.val.cooperative = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a, per, partial);
-    if (e == cudaSuccess) {
-      *done = true;
-      return NVFP4_OK;
-    }
-    cudaGetLastError();
-    if (e != cudaErrorCooperativeLaunchTooLarge) return NVFP4_ERR_LAUNCH_FAILED;
-    return NVFP4_OK;       // fewer SMs than the device has: the two sweeps run on any number
+  const int64_t groups = (a.rows + kR - 1) / kR, group_bytes = (int64_t)kR * a.cols * 2;
+  const int per = groups_per_cta(kernel, dev, threads, groups, group_bytes);
+  if (per == 0) return NVFP4_OK;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((groups + per - 1) / per));
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = (size_t)(per * group_bytes);
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeCooperative;
+  attr.val.cooperative = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a, per, partial);
+  if (e == cudaSuccess) {
+    *done = true;
+    return NVFP4_OK;
   }
-  return NVFP4_OK;
+  cudaGetLastError();
+  // fewer SMs than the device has: the two sweeps run on any number
+  return e == cudaErrorCooperativeLaunchTooLarge ? NVFP4_OK : NVFP4_ERR_LAUNCH_FAILED;
 }
 
 int try_resident(const NormArgs& a, unsigned* partial, cudaStream_t st, bool* done) {

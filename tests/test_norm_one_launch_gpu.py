@@ -7,12 +7,13 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def _run(one, x, vecs, rms, linear=True, swizzled=True, shift_swz=0, partials=True):
+def _run(one, x, vecs, rms, linear=True, swizzled=True, shift_swz=0, partials=True, stats=None, check=True):
     from blackwell_diffusion_rtx6000_5090_i2v_b200 import _native as N
     rows, cols = x.shape
     dev = x.device
     f32 = dict(dtype=torch.float32, device=dev)
-    stats, slots = torch.empty(rows, 2, **f32), torch.full((2,), float("nan"), **f32)
+    stats = torch.empty(rows, 2, **f32) if stats is None else stats
+    slots = torch.full((2,), float("nan"), **f32)
     part = torch.full((N.AMAX_PARTIALS,), float("nan"), **f32)
     data = torch.full((rows * cols // 2 + 16,), 0xA5, dtype=torch.uint8, device=dev)
     lin = torch.full((rows * cols // 16 + 16,), 0xA5, dtype=torch.uint8, device=dev) if linear else None
@@ -32,7 +33,8 @@ def _run(one, x, vecs, rms, linear=True, swizzled=True, shift_swz=0, partials=Tr
         rc = rc or N.lib.nvfp4_norm_mod_quantize_bf16(x.data_ptr(), rows, cols, w, b, sc, sh, stats.data_ptr(), amax,
                                                       data.data_ptr(), N.ptr(lin), p_swz, gs, status, st)
     assert rc == 0
-    N.check_status()
+    if check:
+        N.check_status()
     return [t for t in (data, lin, swz, slots) if t is not None]
 
 
@@ -96,3 +98,38 @@ def test_two_streams_and_a_graph():
         graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(t._data, want[0]._data) and torch.equal(t._gscale, want[0]._gscale)
+
+
+def _one_launch(rows, cols, kind, graph=False):
+    """Whether the call took the one-launch form, which leaves the row statistics alone; the same bytes either way."""
+    x, vecs = _inputs(rows, cols, kind, rows)
+    want = _run(False, x, vecs, 0)
+    stats = torch.full((rows, 2), float("nan"), device="cuda")
+    if graph:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            got = _run(True, x, vecs, 0, stats=stats, check=False)
+        g.replay()
+    else:
+        got = _run(True, x, vecs, 0, stats=stats)
+    torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    untouched = torch.isnan(stats)
+    assert bool(untouched.all()) or not bool(untouched.any())
+    return bool(untouched.all())
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("rows,cols,kind,one", [
+    # two CTAs an SM by their rows alone, one with their own shared memory and the reserve added
+    (3552, 4096, 2, True), (3553, 4096, 2, False), (4144, 4096, 2, False),
+    (7992, 2048, 1, True), (7993, 2048, 1, False), (8288, 2048, 2, False),
+    (4441, 3584, 2, False), (4736, 3584, 2, False),
+    (1776, 7168, 2, True), (1777, 7168, 2, True), (2072, 7168, 2, True), (2073, 7168, 2, False),    # seven groups a CTA
+    (593, 14336, 0, True), (888, 14336, 0, True), (889, 14336, 0, False),
+    (4737, 3072, 0, True), (5328, 3072, 0, True), (5329, 3072, 0, False),                    # three CTAs an SM, not six
+    (1, 16, 0, True), (20001, 128, 1, True), (27280, 3072, 2, False),
+])
+def test_where_the_rows_fit(rows, cols, kind, one, graph):
+    assert _one_launch(rows, cols, kind, graph) == one
