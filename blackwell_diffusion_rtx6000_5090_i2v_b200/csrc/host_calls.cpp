@@ -180,6 +180,8 @@ Maybe attention(const Tensor& q, const Tensor& k, const Tensor& v, const Maybe& 
         t->device() != q.device())
       return {};
   if (k.size(0) != v.size(0)) return {};
+  if (amax && (!plain(*amax) || amax->scalar_type() != at::kFloat || amax->numel() < 1 || amax->device() != q.device()))
+    return {};
   Tensor o = empty({q.size(0), H, D}, at::kBFloat16, q);
   check(nvfp4_attention_bf16(q.data_ptr(), q.stride(0), q.stride(1), k.data_ptr(), k.stride(0), k.stride(1),
                              v.data_ptr(), v.stride(0), v.stride(1), q.size(0), k.size(0), (int)H, (int)D,

@@ -332,13 +332,24 @@ def attention_native(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
     for t in (q, k, v):
         if t.dtype != torch.bfloat16 or t.stride(2) != 1 or t.shape[1:] != (H, D):
             raise ValueError("attention_native wants bf16 [L, H, D] tensors with a contiguous last dimension")
-    if out is None:
-        out = torch.empty(Lq, H, D, dtype=torch.bfloat16, device=q.device)
-    N.check(N.lib.nvfp4_attention_bf16(
-        q.data_ptr(), q.stride(0), q.stride(1), k.data_ptr(), k.stride(0), k.stride(1),
-        v.data_ptr(), v.stride(0), v.stride(1), Lq, Lk, H, D, 1.0 / D ** 0.5, out.data_ptr(),
-        out.stride(0), out.stride(1), None if amax is None else amax.data_ptr(),
-        N.ptr(N.status_word(q.device)), N.stream_ptr()), "attention")
+    # the kernel is given addresses: whatever it reads or writes through them is looked at here
+    if v.shape[0] != Lk:
+        raise ValueError(f"attention_native: {Lk} keys and {v.shape[0]} values")
+    if not q.is_cuda or any(t is not None and t.device != q.device for t in (k, v, amax, out)):
+        raise ValueError("attention_native wants its tensors on one CUDA device")
+    if out is not None and (out.dtype != torch.bfloat16 or out.dim() != 3 or out.stride(2) != 1
+                            or any(have < need for have, need in zip(out.shape, (Lq, H, D)))):
+        raise ValueError("attention_native: out must be bf16 [Lq, H, D] with a contiguous last dimension")
+    if amax is not None and (amax.dtype != torch.float32 or amax.numel() < 1):
+        raise ValueError("attention_native: amax must be a one-element float32 tensor")
+    with N.device_guard(q.device):
+        if out is None:
+            out = torch.empty(Lq, H, D, dtype=torch.bfloat16, device=q.device)
+        N.check(N.lib.nvfp4_attention_bf16(
+            q.data_ptr(), q.stride(0), q.stride(1), k.data_ptr(), k.stride(0), k.stride(1),
+            v.data_ptr(), v.stride(0), v.stride(1), Lq, Lk, H, D, 1.0 / D ** 0.5, out.data_ptr(),
+            out.stride(0), out.stride(1), None if amax is None else amax.data_ptr(),
+            N.ptr(N.status_word(q.device)), N.stream_ptr()), "attention")
     return out
 
 

@@ -131,8 +131,12 @@ def test_gemm_and_attention():
                dict(C=y), dict(out_amax=torch.zeros(1, device="cuda"))):
         assert _same(*_both(lambda: nv.fp4_gemm(a, b, **kw)))
     q, k, v = _bf(130, 2, 384).split(128, dim=-1)
-    for args in ((q, k, v), (q, k.contiguous(), v), (q.float(), k, v), (q[:, :, ::2], k, v), (q[:, :1], k, v)):
+    for args in ((q, k, v), (q, k.contiguous(), v), (q.float(), k, v), (q[:, :, ::2], k, v), (q[:, :1], k, v),
+                 (q, k, v[:-1]), (q, k[:-1], v), (q, k.cpu(), v), (q.cpu(), k.cpu(), v.cpu())):
         assert _same(*_both(lambda: dit.attention_native(*args)))
+    for slot in (torch.zeros(1, device="cuda"), torch.zeros(9, device="cuda")[3:4], torch.zeros(1), y,
+                 torch.zeros(0, device="cuda"), torch.zeros(1, device="cuda", dtype=torch.float64)):
+        assert _same(*_both(lambda: (dit.attention_native(q, k, v, amax=slot.zero_()), slot.clone())))
 
 
 def test_dispatch_modes_and_function_transforms_are_left_alone():
