@@ -415,6 +415,12 @@ norm_mod_kernel(const NormArgs p) {
           reinterpret_cast<float2*>(p.stats)[base + r] = make_float2(mean[r], rstd[r]);
       }
     } else {
+      // The blocks were asked for above, but nothing has used them yet: where other kernels keep the SM's load units
+      // busy, some are still to be read when the refill, which does not queue behind them, lands.  (In sweep 1 the
+      // sums have used them.)  The fence holds every thread's reads ahead of the copy that thread 0 starts
+      // (without it one call in twenty was wrong beside a quantizer on another stream; 95.3 -> 96.2 us for both sweeps
+      // of [27280, 3072]).
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncthreads();
       refill();
 #pragma unroll
