@@ -5,13 +5,21 @@
 // Every function returns None for what is not the plain case (other types, devices, layouts or alignments,
 // tensor subclasses, an active dispatch mode, an empty tensor): the Python code that called it then does what it
 // always did, errors included.  Nothing is kept between calls but the address of each device's status word.
+//
+// The calls let go of the interpreter lock, as the ctypes calls and torch's own allocations do: a launch waits where the
+// stream's queue is full and an allocation may reach the driver, and neither needs the interpreter.  Their errors are
+// torch's (an allocation that does not fit raises torch.OutOfMemoryError).
 #include <ATen/TensorSubclassLikeUtils.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
 
+#include <atomic>
+#include <optional>
 #include <string>
+#include <tuple>
+#include <vector>
 
 #include "../../include/nvfp4_b200.h"
 
@@ -20,7 +28,7 @@ namespace {
 using at::Tensor;
 using Maybe = std::optional<Tensor>;
 
-int* g_status[64];           // per device; set once, before the first call there (under the GIL)
+std::atomic<int*> g_status[64];           // per device; set once, before the first call there
 
 void check(int rc, const char* what) {
   if (rc != NVFP4_OK)
@@ -41,7 +49,9 @@ bool fits(const Maybe& t, at::ScalarType type, int64_t numel, const Tensor& like
 }
 void* ptr(const Maybe& t) { return t ? t->data_ptr() : nullptr; }
 Maybe nonempty(const Maybe& t) { return t && t->numel() > 0 ? t : Maybe(); }
-int* status_of(const Tensor& t) { return t.get_device() < 64 ? g_status[t.get_device()] : nullptr; }
+int* status_of(const Tensor& t) {
+  return t.get_device() < 64 ? g_status[t.get_device()].load(std::memory_order_acquire) : nullptr;
+}
 void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
 Tensor empty(at::IntArrayRef size, at::ScalarType type, const Tensor& like) {
   return at::empty(size, at::TensorOptions().dtype(type).device(like.device()));
@@ -51,7 +61,7 @@ uint8_t* u8(const Tensor& t) { return static_cast<uint8_t*>(t.data_ptr()); }
 uint8_t* u8(const Maybe& t) { return t ? u8(*t) : nullptr; }
 
 void set_status(int64_t device, const Tensor& word) {
-  if (device >= 0 && device < 64) g_status[device] = static_cast<int*>(word.data_ptr());
+  if (device >= 0 && device < 64) g_status[device].store(static_cast<int*>(word.data_ptr()), std::memory_order_release);
 }
 
 // y = residual + gate * act(x @ w.T + bias) with the packed weight of `weight`
@@ -79,11 +89,14 @@ Maybe linear(const Tensor& x, const Tensor& weight, const Tensor& w_data, const 
   return y;
 }
 
-// (rows, cols, data, scales, swizzled scales, amax, tensor scale) of a bf16 tensor of whole blocks
-py::object quantize(const Tensor& x, bool linear_scales, bool swizzled_scales) {
+// rows, cols, data, scales, swizzled scales, amax, tensor scale
+using Packed = std::tuple<int64_t, int64_t, Tensor, Maybe, Maybe, Tensor, Tensor>;
+
+// Of a bf16 tensor of whole blocks.
+std::optional<Packed> quantize(const Tensor& x, bool linear_scales, bool swizzled_scales) {
   if (!plain(x) || modes() || x.scalar_type() != at::kBFloat16 || x.dim() < 1 || x.numel() == 0 ||
       x.size(-1) % 16 != 0 || !x.is_contiguous())
-    return py::none();
+    return {};
   const c10::cuda::CUDAGuard guard(x.device());
   const int64_t cols = x.size(-1), rows = x.numel() / cols;
   Tensor amax = empty({1}, at::kFloat, x), gscale = empty({1}, at::kFloat, x);
@@ -95,21 +108,21 @@ py::object quantize(const Tensor& x, bool linear_scales, bool swizzled_scales) {
   check(nvfp4_amax_quantize_bf16(x.data_ptr(), rows, cols, f32(amax), u8(data), u8(scales), u8(swz), f32(gscale),
                                  f32(partials), stream_of(x)),
         "[tensor] amax+quantize");
-  return py::make_tuple(rows, cols, data, scales, swz, amax, gscale);
+  return Packed(rows, cols, data, scales, swz, amax, gscale);
 }
 
 // The same of norm(x) * weight + bias, modulated; into the given buffers (data, scales, swizzled scales, amax,
 // tensor scale, row statistics, partial maxima) or new ones.
-py::object norm_quantize(const Tensor& x, const Maybe& weight, const Maybe& bias, const Maybe& scale,
+std::optional<Packed> norm_quantize(const Tensor& x, const Maybe& weight, const Maybe& bias, const Maybe& scale,
                          const Maybe& shift, bool rms, double eps, bool linear_scales,
                          const std::optional<std::vector<Maybe>>& out) {
   if (!plain(x) || modes() || x.scalar_type() != at::kBFloat16 || x.dim() < 1 || x.numel() == 0 ||
       !x.is_contiguous() || !status_of(x))
-    return py::none();
+    return {};
   const int64_t cols = x.size(-1), rows = x.numel() / cols;
-  if (cols % 16 != 0 || cols > 16384) return py::none();
+  if (cols % 16 != 0 || cols > 16384) return {};
   for (const Maybe* v : {&weight, &bias, &scale, &shift})
-    if (!fits(*v, at::kFloat, cols, x)) return py::none();
+    if (!fits(*v, at::kFloat, cols, x)) return {};
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor data, amax, gscale, work;
   Maybe scales, swz;
@@ -135,7 +148,7 @@ py::object norm_quantize(const Tensor& x, const Maybe& weight, const Maybe& bias
                             stats, f32(amax), u8(data), u8(scales), u8(swz), f32(gscale), partials, status_of(x),
                             stream_of(x)),
         "[tensor] norm+quantize");
-  return py::make_tuple(rows, cols, data, scales, swz, amax, gscale);
+  return Packed(rows, cols, data, scales, swz, amax, gscale);
 }
 
 Maybe dequantize(const Tensor& data, const Tensor& scales, const Tensor& amax, int64_t rows, int64_t cols,
@@ -195,10 +208,10 @@ Maybe attention(const Tensor& q, const Tensor& k, const Tensor& v, const Maybe& 
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("set_status", &set_status);
-  m.def("linear", &linear);
-  m.def("quantize", &quantize);
-  m.def("norm_quantize", &norm_quantize);
-  m.def("dequantize", &dequantize);
-  m.def("gemm", &gemm);
-  m.def("attention", &attention);
+  m.def("linear", torch::wrap_pybind_function_no_gil(linear));
+  m.def("quantize", torch::wrap_pybind_function_no_gil(quantize));
+  m.def("norm_quantize", torch::wrap_pybind_function_no_gil(norm_quantize));
+  m.def("dequantize", torch::wrap_pybind_function_no_gil(dequantize));
+  m.def("gemm", torch::wrap_pybind_function_no_gil(gemm));
+  m.def("attention", torch::wrap_pybind_function_no_gil(attention));
 }
