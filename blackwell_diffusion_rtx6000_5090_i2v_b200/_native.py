@@ -9,6 +9,7 @@ import contextlib
 import ctypes as C
 import functools
 import os
+import threading
 
 import torch
 
@@ -123,6 +124,7 @@ def ptr(t: torch.Tensor | None):
 
 
 _status_words: dict[int, torch.Tensor] = {}
+_status_lock = threading.Lock()
 
 
 def status_word(device: torch.device) -> torch.Tensor:
@@ -130,9 +132,12 @@ def status_word(device: torch.device) -> torch.Tensor:
     idx = device.index if device.index is not None else torch.cuda.current_device()
     w = _status_words.get(idx)
     if w is None:
-        w = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", idx))
-        _status_words[idx] = w
-        host.set_status(idx, w)
+        with _status_lock:      # one word a device: its address is kept by the native calls
+            w = _status_words.get(idx)
+            if w is None:
+                w = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", idx))
+                host.set_status(idx, w)
+                _status_words[idx] = w
     return w
 
 
