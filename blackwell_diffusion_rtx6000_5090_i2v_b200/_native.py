@@ -1,4 +1,5 @@
-"""ctypes binding of libnvfp4_b200.so -- the only route to the CUDA kernels.
+"""Binding of libnvfp4_b200.so -- the only route to the CUDA kernels -- by ctypes, and by an
+extension module for the frequent calls.
 
 There is no CPU or PyTorch fallback: if the library is missing the import of
 this module raises, and every failed call raises ``RuntimeError``.
@@ -10,8 +11,11 @@ import ctypes as C
 import functools
 import os
 import threading
+import warnings
 
 import torch
+
+from . import build
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 _LIB_PATH = os.path.join(_HERE, "libnvfp4_b200.so")
@@ -70,13 +74,32 @@ for _name, (_res, _args) in SIGNATURES.items():
     _fn.restype = _res
     _fn.argtypes = _args
 
-_HOST_PATH = os.path.join(_HERE, "_host_calls.so")
-if not os.path.exists(_HOST_PATH):
-    raise ImportError(f"{_HOST_PATH} is missing: build it with "
-                      "`python -m blackwell_diffusion_rtx6000_5090_i2v_b200.build`")
-# Checks, allocations and the library call of the plain case in one native step; each returns None for
-# anything else, which the Python code around it then handles.
-from . import _host_calls as host  # noqa: E402
+
+class _Declines:
+    """In place of the extension module: every call is left to the Python code behind it."""
+    built_for = None
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
+def _load_host():
+    """The extension of csrc/host_calls.cpp: checks, allocations and the library call of the plain case in one native
+    step; each of its calls returns None for anything else, which the Python code around it then handles.  It
+    is bound to one torch and one Python: without one that fits, everything takes the Python code."""
+    try:
+        from . import _host_calls as module
+        if module.built_for == build.host_built_for():
+            return module
+        reason = f"it is built for {module.built_for}"
+    except (ImportError, AttributeError) as e:
+        reason = str(e)
+    warnings.warn(f"the native calls are not in use, so that calls take the host longer ({reason}): build them with "
+                  "`python -m blackwell_diffusion_rtx6000_5090_i2v_b200.build`", RuntimeWarning, stacklevel=2)
+    return _Declines()
+
+
+host = _load_host()
 
 OK = 0
 ACT_NONE, ACT_GELU_TANH = 0, 1

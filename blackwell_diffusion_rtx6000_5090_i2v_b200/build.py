@@ -50,12 +50,25 @@ def is_stale() -> bool:
     return any(os.path.getmtime(d) > t for d in deps if os.path.exists(d))
 
 
+def host_built_for() -> str:
+    """What the extension module is bound to; it carries this text."""
+    import torch
+    return f"torch {torch.__version__}, Python {sys.version_info[0]}.{sys.version_info[1]}"
+
+
+def host_is_stale() -> bool:
+    deps = [os.path.join(CSRC, "host_calls.cpp"), os.path.join(HERE, "..", "include", "nvfp4_b200.h")]
+    if not os.path.exists(HOST) or any(os.path.getmtime(d) > os.path.getmtime(HOST) for d in deps if os.path.exists(d)):
+        return True
+    with open(HOST, "rb") as f:
+        return host_built_for().encode() not in f.read()
+
+
 def build_host(force: bool = False) -> str:
     """The extension module that the Python layer calls the library through (needs torch's headers)."""
-    src = os.path.join(CSRC, "host_calls.cpp")
-    deps = [src, os.path.join(HERE, "..", "include", "nvfp4_b200.h")]
-    if not force and os.path.exists(HOST) and all(os.path.getmtime(d) <= os.path.getmtime(HOST) for d in deps):
+    if not force and not host_is_stale():
         return HOST
+    src = os.path.join(CSRC, "host_calls.cpp")
     import sysconfig
 
     import torch
@@ -65,6 +78,7 @@ def build_host(force: bool = False) -> str:
                os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")]
     cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
            "-DTORCH_EXTENSION_NAME=_host_calls", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           f'-DNVFP4_BUILT_FOR="{host_built_for()}"',
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
            *[f for d in include for f in ("-isystem", d)], src, "-o", HOST,
            "-L", HERE, "-l:libnvfp4_b200.so", "-Wl,-rpath,$ORIGIN",

@@ -207,6 +207,7 @@ Maybe attention(const Tensor& q, const Tensor& k, const Tensor& v, const Maybe& 
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.attr("built_for") = NVFP4_BUILT_FOR;
   m.def("set_status", &set_status);
   m.def("linear", torch::wrap_pybind_function_no_gil(linear));
   m.def("quantize", torch::wrap_pybind_function_no_gil(quantize));
