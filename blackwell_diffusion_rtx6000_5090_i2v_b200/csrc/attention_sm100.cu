@@ -51,6 +51,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <cfloat>
 #include <cstdint>
 
 #include "nvfp4_common.cuh"
@@ -550,14 +551,15 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     if (group == 1) asm volatile("bar.arrive %0, %1;" ::"r"(other_bar), "n"(128) : "memory");
     int j0 = 0;                                // running number of the block's first tile
     for (int i = 0; i < blocks; ++i, j0 += n) {
-      float m_ref = 0.f;                       // the row's reference
+      float m_ref = -FLT_MAX;                  // the row's reference: no key yet, or none but keys with -inf
       float m_sum = 0.f;                       // ... and that of the sums below
       float2 sum0 = make_float2(0.f, 0.f), sum1 = make_float2(0.f, 0.f);   // this group's part of the row sum
       // The reference after a tile whose row maximum is m: the first tile's, raised where a later one exceeds it
-      // by more than 2^8.  Both threads of a row apply this to the same maxima.
-      auto follow = [&](float m, bool begins) {
+      // by more than 2^8.  Both threads of a row apply this to the same maxima.  It is a number where every key so far
+      // has -inf, so that these get no weight and any other raises it.
+      auto follow = [&](float m) {
         const float m_new = m * c;
-        if (begins || m_new - m_ref > kRescaleStep) m_ref = m_new;
+        if (m_new - m_ref > kRescaleStep) m_ref = m_new;
       };
       for (int j = j0 + ((j0 & 1) ^ group); j < j0 + n; j += 2) {
         const uint32_t parity = (uint32_t)(j >> 1) & 1u;
@@ -589,9 +591,9 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         asm volatile("bar.sync %0, %1;" ::"r"(my_bar), "n"(128) : "memory");
         const float before = fmaxf(*max_slot(j - 1, 0), *max_slot(j - 1, 1));     // the other group's
         mx = fmaxf(mx, *max_slot(j, half ^ 1));
-        if (j > j0) follow(before, j - 1 == j0);
+        if (j > j0) follow(before);
         const float m_old = m_ref;
-        follow(mx, j == j0);
+        follow(mx);
         if (__any_sync(0xffffffffu, m_ref != m_sum)) {
           if (__any_sync(0xffffffffu, j > j0 && m_ref != m_old)) {
             // O is at rest once the product of the tile before has been added.  (The one before that first: a
@@ -671,7 +673,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       if (kSplit) {
         // the partial result goes where the operands were: no product reads them any more
         if (group == 0 && half == 0)
-          *reinterpret_cast<float2*>(smem_gen + kPartBytes + r * 8) = make_float2(l > 0.f ? m_ref : -INFINITY, l);
+          *reinterpret_cast<float2*>(smem_gen + kPartBytes + r * 8) = make_float2(m_ref > -FLT_MAX ? m_ref : -INFINITY, l);
 #pragma unroll
         for (int q = 0; q < 8; ++q)
           *reinterpret_cast<uint4*>(smem_gen + part_offset(r, col / 4 + q)) =
@@ -680,7 +682,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(lead_o_empty);
-        const float inv = 1.f / l;
+        const float inv = m_ref > -FLT_MAX ? 1.f / l : NAN;      // (no key has any weight)
 #pragma unroll
         for (int e = 0; e < 16; ++e)
           o[e] = f2_to_bf16x2(make_float2(__uint_as_float(o[2 * e]) * inv, __uint_as_float(o[2 * e + 1]) * inv));
