@@ -277,11 +277,12 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 // scarcer resource here: 16 results per clock per SM against 128 FMA lanes).  x = i + f with
 // f in [-0.5, 0.5] by magic-number rounding, a cubic for 2^f (relative error 7.5e-5, a fiftieth
 // of a bf16 rounding step), and i added into the exponent field.  x is clamped at -126, where
-// the result (1e-38) is already nothing next to the row's largest term.
+// the result (1e-38) is already nothing next to the row's largest term.  A NaN stays one through the clamp, and
+// its result, the sum of two NaN patterns, is the largest float: infinity as a bf16, and NaN in the row's output.
 __device__ __forceinline__ float2 exp2_fma(float2 x) {
   const float kMagic = 12582912.f;   // 1.5 * 2^23: the sum's low mantissa bits hold round(x)
-  x.x = fmaxf(x.x, -126.f);
-  x.y = fmaxf(x.y, -126.f);
+  asm("max.NaN.f32 %0, %0, 0fC2FC0000;" : "+f"(x.x));     // -126
+  asm("max.NaN.f32 %0, %0, 0fC2FC0000;" : "+f"(x.y));
   const float2 magic = make_float2(kMagic, kMagic);
   const float2 r = f2_add(x, magic);
   const float2 f = f2_sub(x, f2_sub(r, magic));

@@ -66,3 +66,17 @@ def test_rows_of_infinite_scores_keep_to_themselves(Lq, Lk, H):
     q[::3, :, 0] = -1.0                                 # +inf there: NaN in these rows alone
     o = _check(q, k, v)
     assert bool(torch.isnan(o[::3]).all())
+
+
+@pytest.mark.parametrize("Lq,Lk,H", [(130, 128, 1), (130, 300, 2), (1000, 1000, 5)])
+def test_a_key_with_nan_reaches_every_row(Lq, Lk, H):
+    """Whichever way its exponential takes: most element pairs through the special-function unit, some through a
+    polynomial."""
+    from blackwell_diffusion_rtx6000_5090_i2v_b200 import dit, nvfp4
+    q, k, v = _inputs(Lq, Lk, H)
+    for key in [*range(128), Lk - 1]:
+        bad = k.clone()
+        bad[key, :, 5] = float("nan")
+        o = dit.attention_native(q, bad, v)
+        assert bool(torch.isnan(o).all()), key
+    nvfp4.check_status()
