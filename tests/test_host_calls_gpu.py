@@ -90,7 +90,7 @@ def test_linear_sees_a_changed_weight_and_strides():
 def test_quantize_and_back(make, kw):
     from blackwell_diffusion_rtx6000_5090_i2v_b200.nvfp4 import FP4Tensor
     x = make()
-    assert _same(*_both(lambda: _packed(FP4Tensor.from_bfloat16(x, **kw))[1 if kw.get("swizzled_scales") else 0:2]))
+    assert _same(*_both(lambda: _packed(FP4Tensor.from_bfloat16(x, **kw))[:3]))
     first = 5 if x.numel() == 0 else 3             # an empty tensor's slots are not written
     assert _same(*_both(lambda: _packed(FP4Tensor.from_bfloat16(x, **kw))[first:]))
     assert _same(*_both(lambda: FP4Tensor.from_bfloat16(x, **kw).to_bfloat16()))
@@ -112,7 +112,7 @@ def test_norm(rows, cols, vecs, given):
         out = PackedBuffers(rows, cols, "cuda") if given else None
         t = FP4Tensor.from_norm_mod(x, out=out, **v)
         slots = [t._gscale, t._amax] if rows else []      # an empty tensor's scale is not written
-        return [t._data, *slots, t._rows, t._cols, t._shape, t.scale_factors_swizzled()[:0]]
+        return [t._data, *slots, t._rows, t._cols, t._shape, t._scales, t._scales_swz]
     if cols % 16 or (given and rows == 0):
         with pytest.raises(Exception):
             call()

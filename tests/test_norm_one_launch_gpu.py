@@ -133,3 +133,23 @@ def _one_launch(rows, cols, kind, graph=False):
 ])
 def test_where_the_rows_fit(rows, cols, kind, one, graph):
     assert _one_launch(rows, cols, kind, graph) == one
+
+
+@pytest.mark.parametrize("rows,cols", [(300, 3072), (64, 10240), (1900, 272)])
+@pytest.mark.parametrize("kind", [0, 2])
+@pytest.mark.parametrize("rms", [0, 1])
+@pytest.mark.parametrize("what", ["inf", "-inf", "nan", "nan row", "largest", "all nan"])
+def test_special_values(rows, cols, kind, rms, what):
+    x, vecs = _inputs(rows, cols, kind, rows)
+    if what == "nan row":
+        x[rows // 2] = float("nan")
+    elif what == "all nan":
+        x[:] = float("nan")
+    elif what == "largest":
+        x[3] = torch.finfo(torch.bfloat16).max
+        x[4, ::2] = torch.finfo(torch.bfloat16).min
+    else:
+        x[rows // 3, cols // 2] = float(what)
+        x[rows - 1, 0] = float(what)                  # the row's first element, which the sums are taken around
+    for a, b in zip(_run(True, x, vecs, rms), _run(False, x, vecs, rms)):
+        assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
