@@ -938,7 +938,7 @@ int nvfp4_norm_mod_bf16(const void* x_bf16, int64_t rows, int64_t cols, const fl
                         float* global_scale_dev, float* partials, int* status_dev, void* stream) {
   int rc = check_args(x_bf16, rows, cols);
   if (rc != NVFP4_OK) return rc;
-  if (!amax_dev || (rows > 0 && !packed)) return NVFP4_ERR_BAD_ARG;
+  if (!row_stats || !amax_dev || (rows > 0 && !packed)) return NVFP4_ERR_BAD_ARG;     // whichever form it takes
   if ((reinterpret_cast<uintptr_t>(packed) & 7u) || !vec_ok(weight) || !vec_ok(bias) || !vec_ok(scale) ||
       !vec_ok(shift))
     return NVFP4_ERR_BAD_ALIGN;

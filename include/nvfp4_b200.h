@@ -80,9 +80,11 @@ NVFP4_API int nvfp4_quantize_bf16(const void* x_bf16, int64_t rows, int64_t cols
                         float* global_scale_dev, void* stream);
 
 /* nvfp4_amax_bf16 and nvfp4_quantize_bf16 in one call, with the same results: amax_dev receives
- * max|x|.  Tensors of up to 524288 elements take one kernel.  partials (nullable): device scratch of
- * NVFP4_AMAX_PARTIALS floats, used by this call alone, that spares larger tensors the memset of
- * the amax slot. */
+ * max|x|.  One kernel for tensors of up to 262144 elements (524288 where no other form applies) and, given
+ * partials, of up to some 14.5 million where rows are longer than 3072 elements (and at some shorter ones); the latter is a
+ * cooperative launch: what that means beside other streams stands with nvfp4_norm_mod_bf16 below.  partials
+ * (nullable): device scratch of NVFP4_AMAX_PARTIALS floats, used by this call alone; without it the maximum takes a
+ * memset and a pass of its own. */
 #define NVFP4_AMAX_PARTIALS 1184
 NVFP4_API int nvfp4_amax_quantize_bf16(const void* x_bf16, int64_t rows, int64_t cols, float* amax_dev,
                              uint8_t* packed, uint8_t* scales_linear, uint8_t* scales_swizzled,
@@ -213,8 +215,12 @@ NVFP4_API int nvfp4_norm_mod_quantize_bf16(const void* x_bf16, int64_t rows, int
                                            int* status_dev, void* stream);
 
 /* Both sweeps in one call, with the same results: for tensors that the GPU's shared memory holds (some
- * 13 million elements) one launch that reads x and computes the result once, else the two above.
- * partials: NVFP4_AMAX_PARTIALS floats of scratch, nullable (then always the two); row_stats as above. */
+ * 13 million elements) one launch that reads x and computes the result once, else the two above.  partials:
+ * NVFP4_AMAX_PARTIALS floats of scratch, nullable (then always the two).  row_stats: scratch of 2 * rows floats, never
+ * null; what it holds afterwards is unspecified (the one launch leaves it alone).
+ * The one launch is a cooperative one: its CTAs are on the GPU all at a time and meet.  Beside a long kernel on another
+ * stream those that have found room wait, in the SMs that they hold, until the others have as well, and it
+ * does not start before the call ahead of it in its stream has ended; where that hurts, the two sweeps overlap both. */
 NVFP4_API int nvfp4_norm_mod_bf16(const void* x_bf16, int64_t rows, int64_t cols, const float* weight,
                                   const float* bias, const float* scale, const float* shift, int rms,
                                   float eps, float* row_stats, float* amax_dev, uint8_t* packed,
