@@ -644,10 +644,23 @@ int launch_resident(const void* x, int64_t rows, int64_t cols, float* amax, uint
       return NVFP4_ERR_LAUNCH_FAILED;
     allowed[dev].store(true, std::memory_order_release);
   }
+  const size_t smem = (size_t)per * kHeldThreads * 32;
+  const int64_t ctas = (n_blocks + per * kHeldThreads - 1) / (per * kHeldThreads);
+  // CTAs that an SM holds, plus one; asked for once (a launch that is refused would invalidate a stream capture)
+  static std::atomic<int> known[64][kHeldBlocks + 1];
+  int an_sm = known[dev][per].load(std::memory_order_acquire);
+  if (an_sm == 0) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&an_sm, quantize_resident, kHeldThreads, smem) != cudaSuccess) {
+      cudaGetLastError();
+      return NVFP4_OK;
+    }
+    known[dev][per].store(++an_sm, std::memory_order_release);
+  }
+  if (ctas > (int64_t)sm_count() * (an_sm - 1)) return NVFP4_OK;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((n_blocks + per * kHeldThreads - 1) / (per * kHeldThreads)));
+  cfg.gridDim = dim3((unsigned)ctas);
   cfg.blockDim = dim3(kHeldThreads);
-  cfg.dynamicSmemBytes = (size_t)per * kHeldThreads * 32;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeCooperative;
