@@ -511,7 +511,7 @@ constexpr int kMaxGroups = 16;            // row groups of a CTA
 
 template <int kJ, bool kAffine, bool kMod>
 __global__ void __launch_bounds__(kMaxThreads)
-norm_mod_resident(const NormArgs p, int per_cta, unsigned* partial) {
+norm_mod_resident_kernel(const NormArgs p, int per_cta, unsigned* partial) {
   constexpr int kR = RowsPerIter<kJ>::value;
   constexpr int kV = 2 * kR;
   extern __shared__ __align__(128) uint8_t rows_smem[];     // per_cta groups of kR rows
@@ -785,7 +785,7 @@ int groups_per_cta(Kernel kernel, int dev, int threads, int64_t groups, int64_t 
 // Launches the one-launch form if the rows fit; *done says whether.
 template <int kJ, bool kAffine, bool kMod>
 int launch_resident(const NormArgs& a, int threads, unsigned* partial, cudaStream_t st, bool* done) {
-  auto kernel = norm_mod_resident<kJ, kAffine, kMod>;
+  auto kernel = norm_mod_resident_kernel<kJ, kAffine, kMod>;
   constexpr int kR = RowsPerIter<kJ>::value;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return NVFP4_ERR_BAD_ARG;

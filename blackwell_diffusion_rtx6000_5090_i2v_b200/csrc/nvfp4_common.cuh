@@ -227,9 +227,10 @@ __device__ __forceinline__ void load_block_once(const uint4* src, bool wide, uin
 }
 
 // Launch with programmatic stream serialization: the launch latency and the prologue of `kernel`
-// overlap the tail of its predecessor, which costs a few microseconds a launch where kernels are short:
-// no kernel says before its end that the next may start.  The kernel calls grid_dependency_wait() and loads
-// as above.  `cluster`: CTAs per cluster along x.  Amax + pack of [27280, 3072] 67.7 -> 64.0 us, norm +
+// overlap the tail of its predecessor, which costs a few microseconds a launch where kernels are short.
+// No kernel that this may follow says before its end that the next may start.  (One does, attention's, to the
+// launch of its own that shares the blocks left over, which waits for it at its end and so stands for it to
+// whatever comes after.)  The kernel calls grid_dependency_wait() and loads as above.  `cluster`: CTAs per cluster along x.  Amax + pack of [27280, 3072] 67.7 -> 64.0 us, norm +
 // quantize 98.0 -> 94.5 us, each called back to back; a GEMM or RoPE of that size within the spread of its
 // runs.
 template <typename... Params, typename... Args>

@@ -352,9 +352,9 @@ constexpr int kHeldThreads = 512;
 constexpr int kHeldBlocks = 6;           // most blocks per thread: two CTAs of 96 KB an SM
 
 __global__ void __launch_bounds__(kHeldThreads, 2)
-quantize_resident(const uint4* x, uint32_t n_blocks, uint32_t kb_per_row, int per, unsigned* partial, float* amax_out,
-                  uint2* packed, uint8_t* sf_lin, uint8_t* sf_swz, uint32_t swz_vecs, uint32_t k_atoms,
-                  float* gscale_out) {
+quantize_resident_kernel(const uint4* x, uint32_t n_blocks, uint32_t kb_per_row, int per, unsigned* partial,
+                         float* amax_out, uint2* packed, uint8_t* sf_lin, uint8_t* sf_swz, uint32_t swz_vecs,
+                         uint32_t k_atoms, float* gscale_out) {
   extern __shared__ __align__(16) uint4 held[];       // [block of the thread][half][thread]
   __shared__ unsigned warp_max[kHeldThreads / 32];
   __shared__ float enc_tab[128];
@@ -639,7 +639,7 @@ int launch_resident(const void* x, int64_t rows, int64_t cols, float* amax, uint
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return NVFP4_ERR_BAD_ARG;
   static std::atomic<bool> allowed[64];
   if (!allowed[dev].load(std::memory_order_acquire)) {
-    if (cudaFuncSetAttribute(quantize_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(quantize_resident_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              kHeldBlocks * kHeldThreads * 32) != cudaSuccess)
       return NVFP4_ERR_LAUNCH_FAILED;
     allowed[dev].store(true, std::memory_order_release);
@@ -650,7 +650,7 @@ int launch_resident(const void* x, int64_t rows, int64_t cols, float* amax, uint
   static std::atomic<int> known[64][kHeldBlocks + 1];
   int an_sm = known[dev][per].load(std::memory_order_acquire);
   if (an_sm == 0) {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&an_sm, quantize_resident, kHeldThreads, smem) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&an_sm, quantize_resident_kernel, kHeldThreads, smem) != cudaSuccess) {
       cudaGetLastError();
       return NVFP4_OK;
     }
@@ -668,7 +668,7 @@ int launch_resident(const void* x, int64_t rows, int64_t cols, float* amax, uint
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   const cudaError_t e = cudaLaunchKernelEx(
-      &cfg, quantize_resident, reinterpret_cast<const uint4*>(x), (uint32_t)n_blocks, (uint32_t)(cols / kBlock), (int)per,
+      &cfg, quantize_resident_kernel, reinterpret_cast<const uint4*>(x), (uint32_t)n_blocks, (uint32_t)(cols / kBlock), (int)per,
       reinterpret_cast<unsigned*>(partials), amax, reinterpret_cast<uint2*>(packed), sf_lin, sf_swz,
       (uint32_t)(sf_swz ? sf_swizzled_bytes(rows, cols) / 16 : 0), (uint32_t)sf_k_atoms(cols), gscale);
   if (e == cudaSuccess) {
