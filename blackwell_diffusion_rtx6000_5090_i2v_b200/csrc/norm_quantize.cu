@@ -415,20 +415,29 @@ norm_mod_kernel(const NormArgs p) {
           reinterpret_cast<float2*>(p.stats)[base + r] = make_float2(mean[r], rstd[r]);
       }
     } else {
+      auto take_stats = [&]() {
+#pragma unroll
+        for (int r = 0; r < kR; ++r) {
+          mean[r] = mean_n[r];
+          rstd[r] = rstd_n[r];
+        }
+        if (g + gridDim.x < groups) fetch_stats(g + gridDim.x);
+      };
       // The blocks were asked for above, but nothing has used them yet: where other kernels keep the SM's load units
       // busy, some are still to be read when the refill, which does not queue behind them, lands.  (In sweep 1 the
-      // sums have used them.)  The fence holds every thread's reads ahead of the copy that thread 0 starts
-      // (without it one call in twenty was wrong beside a quantizer on another stream; 95.3 -> 96.2 us for both sweeps
-      // of [27280, 3072]).
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncthreads();
-      refill();
-#pragma unroll
-      for (int r = 0; r < kR; ++r) {
-        mean[r] = mean_n[r];
-        rstd[r] = rstd_n[r];
+      // sums have used them.)  The fence holds every thread's reads ahead of the copy that thread 0 starts: without it
+      // one call in twenty was wrong beside a quantizer on another stream.  Where there is nothing to refill, no thread
+      // waits for the others.  With no vectors, or with all, the row statistics go ahead of it, so that their load is on
+      // its way meanwhile.  Sweep pairs, us, without the fence, with it, as it is: [27280, 3072] no vectors 82.9, 83.8,
+      // 82.5, modulation 96.2, 96.6, 96.5, all four 145.1, 150.7, 147.6; [32760, 5120] modulation 186.0, 186.8, 186.6.
+      constexpr bool kStatsFirst = kAffine == kMod;
+      if (kStatsFirst) take_stats();
+      if (g + (int64_t)kStages * gridDim.x < groups) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
+        refill();
       }
-      if (g + gridDim.x < groups) fetch_stats(g + gridDim.x);
+      if (!kStatsFirst) take_stats();
     }
 
 #pragma unroll
