@@ -22,8 +22,9 @@
 // arrivals across the pair of release.cluster scope (a fence of about 1000 cycles each), 2000 with waits whose
 // lanes polled two barriers (up to a thousand cycles of delay), 1750 with the two groups' exponentials at the
 // same time; 1450 with a thread per row (half the warps, the same latencies per tile), 1330 as it is.
-// [32760, 5, 128] 2610 -> 2170 us, [3121, 12, 128] 96 -> 65, [27280 x 512 keys, 24] 284 -> 211, [512 x 512, 24]
-// 14.2 -> 10.7; beside the library kernel, in the same order, 2110, 74, 149, 10.1.
+// Against the one CTA, us: [32760, 5, 128] back to back 2537 -> 2329; replayed from a graph [3121, 12] 94 -> 64,
+// [27280 x 512 keys, 24] 257 -> 214 to 226, [512 x 512, 24] 14.4 -> 10.8; [1, 1] 5.8 -> 7.4, where the pair's hand-offs are
+// latency alone.  The library kernel, in the same order, 2110, 74, 149, 10.1.
 //
 // Blocks that would leave pairs idle in a last wave are computed by several pairs each, which share the
 // block's keys and join their results through distributed shared memory (kParts > 1, and launch()).
@@ -522,10 +523,10 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     }
   } else {
     // ------------------------------------------------------- softmax ----
-    // Two groups of four warps take the tiles by turns, a thread one row of its group's tile.  The two
-    // threads of a row follow the same maxima: their warps meet at named barriers, where a warp waits at
-    // every tile of its own and arrives, without waiting, when it is through with the tile before one of
-    // the other's.  A warp whose wait has run out goes through the rest of the walk without waiting, so
+    // Two groups of eight warps take the tiles by turns; two threads of a group have a row of its tile, 64 keys
+    // each.  The four threads of a row follow the same maxima: their warps meet at named barriers, where a
+    // warp waits at every tile of its own and arrives, without waiting, when it is through with the tile before one
+    // of the other's.  A warp whose wait has run out goes through the rest of the walk without waiting, so
     // that no other is left at a barrier.
     const int group = warp >> 3;
     const int half = (warp >> 2) & 1;          // which 64 keys of the tile

@@ -111,8 +111,8 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 // (Of CTA scope: what the barriers hand over is tensor memory and what TMA wrote, not other threads' stores;
-// with cluster scope a wait drops the SM's cached lines, bias and gate among them: 27280 x 3072 x 3072 with
-// gate and residual 169 -> 156 us.)
+// with cluster scope a wait drops the SM's cached lines, bias and gate among them, for a share of the gain that
+// mbar_arrive_cluster() states.)
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -147,8 +147,9 @@ __device__ __forceinline__ void cluster_sync_all() {
 // shared accumulator columns.  But of the default scope: no memory that other CTAs read is published here,
 // only this thread's reading of tensor memory, and a release of cluster scope is a fence that waits for every
 // store of the thread, about 1000 cycles ahead of each tile's hand-off (468 against 176 cycles one way with
-// nothing else running).  27280 x 14336 x 3072 with GELU 662 -> 597 us, 27280 x 9216 x 3072 414 -> 356, 4095 x
-// 5120 x 5120 with gate and residual 60.2 -> 55.5.
+// nothing else running).  Both scopes together, us in bursts (sustained): 27280 x 14336 x 3072 with GELU 559 -> 526 (651 ->
+// 604), 27280 x 9216 x 3072 322 -> 305 (375 -> 357), 27280 x 3072 x 3072 with gate and residual 156 -> 138 (179 -> 164), 4095 x
+// 5120 x 5120 with gate and residual 55.9 -> 52.9 (61.1 -> 58.7).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }

@@ -2,6 +2,7 @@
 
     python -m blackwell_diffusion_rtx6000_5090_i2v_b200.profile_case gemm --m 8192 --n 9216 --k 3072
     python -m blackwell_diffusion_rtx6000_5090_i2v_b200.profile_case quantize --m 27280 --k 3072
+    python -m blackwell_diffusion_rtx6000_5090_i2v_b200.profile_case amax_quantize --m 2500 --k 5120
     python -m blackwell_diffusion_rtx6000_5090_i2v_b200.profile_case norm --m 27280 --k 3072
     python -m blackwell_diffusion_rtx6000_5090_i2v_b200.profile_case rope --m 27280 --k 3072
     python -m blackwell_diffusion_rtx6000_5090_i2v_b200.profile_case return --m 32760 --k 5120
@@ -36,7 +37,7 @@ def _time(fn, warmup, iters):
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("kernel", choices=["gemm", "quantize", "amax", "norm", "rope", "return", "attention"])
+    ap.add_argument("kernel", choices=["gemm", "quantize", "amax", "amax_quantize", "norm", "rope", "return", "attention"])
     ap.add_argument("--tiling", choices=["auto", "uniform", "alternating"], default="auto")
     ap.add_argument("--m", type=int, default=8192)
     ap.add_argument("--n", type=int, default=9216)
@@ -128,6 +129,9 @@ def main():
         n = a.m * a.k
         print(f"norm+mod+quantize [{a.m}, {a.k}]: {ms:.4f} ms, algorithmic {2.5625 * n / ms / 1e6:.1f} "
               f"GB/s, moved {4.5625 * n / ms / 1e6:.1f} GB/s")
+    elif a.kernel == "amax_quantize":
+        ms = _time(lambda: FP4Tensor.from_bfloat16(x, linear_scales=False), a.warmup, a.iters)
+        print(f"amax+quantize [{a.m}, {a.k}]: {ms:.4f} ms, algorithmic {2.5625 * a.m * a.k / ms / 1e6:.1f} GB/s")
     else:
         q = FP4Tensor.from_bfloat16(x, linear_scales=False)
         if a.kernel == "quantize":
