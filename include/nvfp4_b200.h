@@ -220,7 +220,8 @@ NVFP4_API int nvfp4_norm_mod_quantize_bf16(const void* x_bf16, int64_t rows, int
  * null; what it holds afterwards is unspecified (the one launch leaves it alone).
  * The one launch is a cooperative one: its CTAs are on the GPU all at a time and meet.  Beside a long kernel on another
  * stream those that have found room wait, in the SMs that they hold, until the others have as well, and it
- * does not start before the call ahead of it in its stream has ended; where that hurts, the two sweeps overlap both. */
+ * does not start before the call ahead of it in its stream has ended; where that hurts, the two sweeps overlap both.
+ * A kernel that waits for other ranks belongs on the same stream, not beside it. */
 NVFP4_API int nvfp4_norm_mod_bf16(const void* x_bf16, int64_t rows, int64_t cols, const float* weight,
                                   const float* bias, const float* scale, const float* shift, int rms,
                                   float eps, float* row_stats, float* amax_dev, uint8_t* packed,
