@@ -50,6 +50,7 @@ SIGNATURES = {
     "nvfp4_linear_bf16": (_i, [_p, _i64, _i64, _p, _p, _p, _i64, _p, _p, _p, _i, _p, _p, _p, _p]),
     "nvfp4_linear_backward_workspace_bytes": (_i64, [_i64, _i64, _i64]),
     "nvfp4_linear_backward_bf16": (_i, [_p, _p, _p, _p, _i64, _i64, _i64, _p, _p, _p, _p, _p]),
+    "nvfp4_linear_backward_bias_bf16": (_i, [_p, _p, _p, _p, _i64, _i64, _i64, _p, _p, _p, _p, _p, _p]),
     "nvfp4_gemm_set_tiling": (_i, [_i]),
     "nvfp4_gemm_stacked": (_i, [_p, _p, _p, _p, _p, _p, _i64, _i64, _i64, _i64, _p, _p, _p, _p]),
     "nvfp4_norm_mod_amax_bf16": (_i, [_p, _i64, _i64, _p, _p, _p, _p, _i, _f, _p, _p, _p, _p, _p]),

@@ -264,4 +264,37 @@ int check_device_sm100();                 // NVFP4_OK or NVFP4_ERR_UNSUPPORTED_A
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 int sm_count();                           // SMs of the current device (cached per device)
 
+// One tensor of launch_amax_partials(): n a multiple of 8, 16-byte aligned.  `first`, `count` are filled in.
+struct AmaxJob {
+  const void* x;
+  int64_t n;
+  int first, count;
+};
+int launch_amax_partials(AmaxJob (&jobs)[3], int n_jobs, float* partials, unsigned* zero, int n_zero, void* stream);
+
+// One bf16 matrix of quantize_jobs() (x null: none), read once: its NVFP4 form, that of its transpose and its column
+// sums, each where the pointers are given.
+constexpr int kQuantizeJobs = 3;
+struct QuantizeJob {
+  const void* x;                 // [rows, cols], cols a multiple of 8
+  uint32_t rows, cols;
+  const float* amax;             // its maximum, where n_partial is 0
+  int first_partial, n_partial;  // else which of the partial maxima are its own
+  uint2* t_packed;               // transpose: [cols, rows padded to 32]
+  uint8_t* t_scales;
+  float* t_gscale;
+  uint32_t t_units, t_k_atoms;   // scale blocks per row, K atoms
+  uint2* packed;                 // itself: cols a multiple of 16
+  uint8_t* scales;
+  float* gscale;
+  uint32_t units, k_atoms;
+  __nv_bfloat16* col_sum;        // [cols]
+  float* col_partial;            // scratch: [row tiles][column tiles * 64]
+  unsigned* col_count;           // scratch: [column tiles], zeroed
+  uint32_t col_tiles, row_tiles; // filled in
+};
+int64_t quantize_job_col_tiles(int64_t cols);
+int64_t quantize_job_row_tiles(int64_t rows);
+int quantize_jobs(const QuantizeJob (&jobs)[kQuantizeJobs], const float* partials, void* stream);
+
 }  // namespace nvfp4

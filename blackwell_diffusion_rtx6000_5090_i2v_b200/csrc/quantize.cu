@@ -28,17 +28,43 @@ constexpr int kBlocksPerThread = 2;  // two 16-element scale blocks (64 B of inp
 
 // kPartial: every CTA leaves its own maximum in out[blockIdx.x] for the packing kernel to combine,
 // so that no slot has to be zeroed first, and launched by launch_dependent(); else one atomic per CTA
-// on the zeroed slot.
-template <bool kPartial>
-__global__ void __launch_bounds__(kThreads) amax_bf16_kernel(const uint4* x, int64_t n_vec,
+// on the zeroed slot.  kTensors: how many tensors share the launch (AmaxJob), each with its own CTAs.
+template <int kTensors>
+struct AmaxArgs {
+  const uint4* x[kTensors];
+  int64_t n_vec[kTensors];
+  unsigned first[kTensors + 1];   // CTAs of tensor i: first[i] up to first[i + 1]
+  unsigned* zero;                 // kPartial, nullable: words that the next kernel wants zeroed
+  int n_zero;
+};
+
+template <bool kPartial, int kTensors>
+__global__ void __launch_bounds__(kThreads) amax_bf16_kernel(const AmaxArgs<kTensors> p,
                                                              const __nv_bfloat16* tail, int n_tail,
                                                              unsigned* out) {
   __nv_bfloat162 m2[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) m2[j] = __nv_bfloat162(__float2bfloat16(0.f), __float2bfloat16(0.f));
-  if (kPartial) grid_dependency_wait();
-  const int64_t stride = (int64_t)gridDim.x * kThreads;
-  int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  const uint4* x = p.x[0];
+  int64_t n_vec = p.n_vec[0];
+  unsigned first = p.first[0], end = p.first[1];
+#pragma unroll
+  for (int k = 1; k < kTensors; ++k) {
+    if (blockIdx.x >= p.first[k]) {
+      x = p.x[k];
+      n_vec = p.n_vec[k];
+      first = p.first[k];
+      end = p.first[k + 1];
+    }
+  }
+  const unsigned cta = blockIdx.x - first, ctas = end - first;
+  if (kPartial) {
+    grid_dependency_wait();
+    if (blockIdx.x == 0)
+      for (int i = threadIdx.x; i < p.n_zero; i += kThreads) p.zero[i] = 0u;
+  }
+  const int64_t stride = (int64_t)ctas * kThreads;
+  int64_t i = (int64_t)cta * kThreads + threadIdx.x;
   // four independent 16-byte loads in flight per thread
   for (; i + 3 * stride < n_vec; i += 4 * stride) {
     uint4 v[4];
@@ -46,16 +72,16 @@ __global__ void __launch_bounds__(kThreads) amax_bf16_kernel(const uint4* x, int
     for (int j = 0; j < 4; ++j) v[j] = load_u32x4(x + i + j * stride);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v[j]);
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v[j]);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) m2[k] = __hmax2(m2[k], __habs2(p[k]));
+      for (int k = 0; k < 4; ++k) m2[k] = __hmax2(m2[k], __habs2(h[k]));
     }
   }
   for (; i < n_vec; i += stride) {
     uint4 v = load_u32x4(x + i);
-    const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v);
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) m2[k] = __hmax2(m2[k], __habs2(p[k]));
+    for (int k = 0; k < 4; ++k) m2[k] = __hmax2(m2[k], __habs2(h[k]));
   }
   __nv_bfloat162 m = __hmax2(__hmax2(m2[0], m2[1]), __hmax2(m2[2], m2[3]));
   float a = fmaxf(__bfloat162float(m.x), __bfloat162float(m.y));
@@ -692,6 +718,34 @@ int launch_small(const void* x, int64_t rows, int64_t cols, float* amax, uint8_t
 
 }  // namespace
 
+// The maxima of up to three tensors in one launch, each tensor's CTAs in proportion to its size: `job.first` and
+// `job.count` say which of the partial maxima are a tensor's.
+int launch_amax_partials(AmaxJob (&jobs)[3], int n_jobs, float* partials, unsigned* zero, int n_zero, void* stream) {
+  int64_t want = 0;
+  for (int i = 0; i < n_jobs; ++i) want += amax_grid(jobs[i].n / 8);
+  AmaxArgs<3> a{};
+  unsigned next = 0;
+  for (int i = 0; i < 3; ++i) {
+    a.first[i] = next;
+    if (i >= n_jobs) continue;
+    const int64_t n_vec = jobs[i].n / 8;
+    int64_t ctas = amax_grid(n_vec);
+    // rounded down, and three single CTAs at most on top of that: no more than there is room for
+    if (want > NVFP4_AMAX_PARTIALS) ctas = ctas * (NVFP4_AMAX_PARTIALS - 3) / want + 1;
+    a.x[i] = static_cast<const uint4*>(jobs[i].x);
+    a.n_vec[i] = n_vec;
+    jobs[i].first = (int)next;
+    jobs[i].count = (int)ctas;
+    next += (unsigned)ctas;
+  }
+  a.first[3] = next;
+  a.zero = zero;
+  a.n_zero = n_zero;
+  return launch_dependent(amax_bf16_kernel<true, 3>, dim3(next), kThreads, 0, 1,
+                          reinterpret_cast<cudaStream_t>(stream), a, (const __nv_bfloat16*)nullptr, 0,
+                          reinterpret_cast<unsigned*>(partials));
+}
+
 }  // namespace nvfp4
 
 using namespace nvfp4;
@@ -710,10 +764,10 @@ int nvfp4_amax_bf16(const void* x, int64_t n, float* amax_dev, void* stream) {
   if (!aligned16(x)) return NVFP4_ERR_BAD_ALIGN;
   const int64_t n_vec = n / 8;
   const int n_tail = (int)(n - n_vec * 8);
-  amax_bf16_kernel<false><<<amax_grid(n_vec), kThreads, 0, st>>>(
-      reinterpret_cast<const uint4*>(x), n_vec,
-      reinterpret_cast<const __nv_bfloat16*>(x) + n_vec * 8, n_tail,
-      reinterpret_cast<unsigned*>(amax_dev));
+  const unsigned grid = amax_grid(n_vec);
+  const AmaxArgs<1> a{{reinterpret_cast<const uint4*>(x)}, {n_vec}, {0u, grid}, nullptr, 0};
+  amax_bf16_kernel<false, 1><<<grid, kThreads, 0, st>>>(
+      a, reinterpret_cast<const __nv_bfloat16*>(x) + n_vec * 8, n_tail, reinterpret_cast<unsigned*>(amax_dev));
   return launch_status();
 }
 
@@ -755,8 +809,9 @@ int nvfp4_amax_quantize_bf16(const void* x, int64_t rows, int64_t cols, float* a
   if (n_blocks > 0 && partials && rows_form(rows, cols, scales_swizzled != nullptr, &threads)) {
     const int64_t n_vec = n_blocks * 2;
     const unsigned grid = amax_grid(n_vec);
-    rc = launch_dependent(amax_bf16_kernel<true>, dim3(grid), kThreads, 0, 1, st, reinterpret_cast<const uint4*>(x),
-                          n_vec, (const __nv_bfloat16*)nullptr, 0, reinterpret_cast<unsigned*>(partials));
+    const AmaxArgs<1> first{{reinterpret_cast<const uint4*>(x)}, {n_vec}, {0u, grid}, nullptr, 0};
+    rc = launch_dependent(amax_bf16_kernel<true, 1>, dim3(grid), kThreads, 0, 1, st, first,
+                          (const __nv_bfloat16*)nullptr, 0, reinterpret_cast<unsigned*>(partials));
     if (rc != NVFP4_OK) return rc;
     PackArgs a{};
     a.x = reinterpret_cast<const uint4*>(x);

@@ -271,11 +271,13 @@ def backward(grad_output: torch.Tensor, input: torch.Tensor, weight: torch.Tenso
         with N.device_guard(dev):
             ws = torch.empty(N.lib.nvfp4_linear_backward_workspace_bytes(m, out_features, k),
                              dtype=torch.uint8, device=dev)
+            if needs_bias_grad:
+                grad_bias = torch.empty(out_features, dtype=torch.bfloat16, device=dev)
             # the maximum of the weight is taken here, not from the forward's packed copy: a write
             # through weight.data would leave that one behind
-            N.check(N.lib.nvfp4_linear_backward_bf16(
+            N.check(N.lib.nvfp4_linear_backward_bias_bf16(
                 go.data_ptr(), x2.data_ptr() if one_dw else None, weight.data_ptr() if one_dx else None,
-                None, m, out_features, k, N.ptr(grad_input), N.ptr(grad_weight), ws.data_ptr(),
+                None, m, out_features, k, N.ptr(grad_input), N.ptr(grad_weight), N.ptr(grad_bias), ws.data_ptr(),
                 N.status_word(dev).data_ptr(), N.stream_ptr()), "[linear] backward")
         if one_dx:
             grad_input = grad_input.reshape(input.shape)
@@ -283,7 +285,7 @@ def backward(grad_output: torch.Tensor, input: torch.Tensor, weight: torch.Tenso
         grad_input = gemm(go, weight.t().contiguous(), 1.0, 0.0).reshape(input.shape)
     if needs_weight_grad and not one_dw:
         grad_weight = gemm(go.t().contiguous(), x2.t().contiguous(), 1.0, 0.0)
-    if needs_bias_grad:
+    if needs_bias_grad and grad_bias is None:
         grad_bias = go.sum(0)
     return [grad_input, grad_weight, grad_bias]
 

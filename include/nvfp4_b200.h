@@ -160,6 +160,10 @@ NVFP4_API int64_t nvfp4_linear_backward_workspace_bytes(int64_t M, int64_t N, in
 NVFP4_API int nvfp4_linear_backward_bf16(const void* dy_bf16, const void* x_bf16, const void* w_bf16,
                                const float* w_amax_dev, int64_t M, int64_t N, int64_t K, void* dx_bf16,
                                void* dw_bf16, void* workspace, int* status_dev, void* stream);
+/* The same, and the bias gradient db[N] = column sums of dy (fp32 sums, bf16 result; nullable). */
+NVFP4_API int nvfp4_linear_backward_bias_bf16(const void* dy_bf16, const void* x_bf16, const void* w_bf16,
+                               const float* w_amax_dev, int64_t M, int64_t N, int64_t K, void* dx_bf16,
+                               void* dw_bf16, void* db_bf16, void* workspace, int* status_dev, void* stream);
 
 /* Which N tiling nvfp4_gemm uses: 0 = chosen per shape (the default: 256-wide tiles, or 192-, 128-
  * or 64-wide ones where a grid of at most two waves leaves SMs idle), 1 = uniform 256-wide tiles, 2 = 448-column pairs of a 256-wide and a 192-wide tile (two
