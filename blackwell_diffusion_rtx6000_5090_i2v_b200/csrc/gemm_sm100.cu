@@ -49,6 +49,8 @@
 // that tensor memory is released and the CTA exits.
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "nvfp4_common.cuh"
 
 namespace nvfp4 {
@@ -423,7 +425,11 @@ struct TileWalk {
   }
 };
 
-template <bool kAlt>
+// What an epilogue does beyond scaling, as known when the kernel is compiled (kEpiAny: as its parameters say).  With the
+// checks in the kernel every 8-column piece was several branches and the pieces could not be interleaved.
+enum { kEpiBias = 1, kEpiGelu = 2, kEpiGate = 4, kEpiResidual = 8, kEpiAmax = 16, kEpiAny = -1 };
+
+template <bool kAlt, int kEpi>
 __global__ void __launch_bounds__(kThreads, 1)
 nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
                   const __grid_constant__ CUtensorMap map_b,
@@ -644,6 +650,11 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
     // that the lane-per-row writes spread over the banks) and leaves with one TMA store, which
     // also clips at M and N.
     const int q = warp & 3;  // tensor-memory lane quarter this warp may read
+    const bool with_bias = kEpi < 0 ? p.bias != nullptr : (kEpi & kEpiBias) != 0;
+    const bool with_gelu = kEpi < 0 ? p.act == NVFP4_ACT_GELU_TANH : (kEpi & kEpiGelu) != 0;
+    const bool with_gate = kEpi < 0 ? p.gate != nullptr : (kEpi & kEpiGate) != 0;
+    const bool with_c = kEpi < 0 ? p.c != nullptr : (kEpi & kEpiResidual) != 0;
+    const bool with_amax = kEpi < 0 ? p.d_amax != nullptr : (kEpi & kEpiAmax) != 0;
     const float scale_a = p.alpha * (p.ga ? load_f32(p.ga) : 1.0f);
     const float scale_ab = scale_a * ((p.gb && p.gb_group == 0) ? load_f32(p.gb) : 1.0f);
     const uint32_t lead_acc_empty0 = mapa_u32(acc_empty_bar(0), 0);
@@ -703,7 +714,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         // the layout the result will leave in, while tensor memory is being read: as per-lane
         // row-strided 16-byte loads it put sixteen exposed global-memory latencies per tile on
         // this warp and made a K = 3072 GEMM with a residual epilogue-bound (half speed).
-        if (p.c) {
+        if (with_c) {
           // the previous store must have finished reading the slab
           asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
           __syncwarp();
@@ -731,7 +742,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         }
         // per-column operands of the whole group first, so that their loads overlap
         uint4 bb[8];
-        if (p.bias) {
+        if (with_bias) {
 #pragma unroll
           for (int g = 0; g < 8; ++g)
             bb[g] = col0 + g * 8 < p.N
@@ -741,7 +752,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         // stacked weights: the tensor scale of the weight this group's columns belong to
         const float scale = (p.gb_group > 0 && col0 < p.N)
                                 ? scale_a * load_f32(p.gb + col0 / p.gb_group) : scale_ab;
-        if (!p.c) {
+        if (!with_c) {
           // the previous store must have finished reading the slab
           asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
           __syncwarp();
@@ -759,7 +770,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         for (int g = 0; g < 8; ++g) {
           float2 v[4];
           const bool in_n = col0 + g * 8 < p.N;
-          if (p.bias) {
+          if (with_bias) {
             const uint32_t bw[4] = {bb[g].x, bb[g].y, bb[g].z, bb[g].w};
 #pragma unroll
             for (int e = 0; e < 4; ++e)
@@ -772,11 +783,11 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
               v[e] = f2_mul(make_float2(__uint_as_float(x[g * 8 + 2 * e]),
                                         __uint_as_float(x[g * 8 + 2 * e + 1])), scale2);
           }
-          if (p.act == NVFP4_ACT_GELU_TANH) {
+          if (with_gelu) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) v[e] = gelu_tanh2(v[e]);
           }
-          if (p.gate && in_n) {
+          if (with_gate && in_n) {
             const float4 g0 = load_f32x4(p.gate + col0 + g * 8);
             const float4 g1 = load_f32x4(p.gate + col0 + g * 8 + 4);
             v[0] = f2_mul(v[0], make_float2(g0.x, g0.y));
@@ -784,14 +795,14 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
             v[2] = f2_mul(v[2], make_float2(g1.x, g1.y));
             v[3] = f2_mul(v[3], make_float2(g1.z, g1.w));
           }
-          if (p.c) {   // rows past M and columns past N were zero-filled by the load
+          if (with_c) {   // rows past M and columns past N were zero-filled by the load
             const uint4 cc = *reinterpret_cast<const uint4*>(slab + lane * 128 + ((g ^ (lane & 7)) << 4));
             const uint32_t cw[4] = {cc.x, cc.y, cc.z, cc.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) v[e] = f2_fma(beta2, bf16x2_to_f2(cw[e]), v[e]);
           }
           uint32_t o[4];
-          const bool counted = p.d_amax && row < p.M && in_n;
+          const bool counted = with_amax && row < p.M && in_n;
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             o[e] = f2_to_bf16x2(v[e]);
@@ -811,7 +822,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
     }
     // the CTA's shared memory must outlive the stores that read it
     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-    if (p.d_amax) {
+    if (with_amax) {
       // non-negative floats order like their bit patterns: one atomic per warp per launch
       const float a = fmaxf(bf16lo_to_f32(amax2), bf16hi_to_f32(amax2));
       const unsigned bits = __reduce_max_sync(0xffffffffu, __float_as_uint(a));
@@ -950,7 +961,7 @@ int tile_width(int64_t m_tiles, int64_t M, int64_t N, int64_t K) {
   return best;
 }
 
-template <bool kAlt>
+template <bool kAlt, int kEpi>
 int launch_gemm(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_b_narrow,
                 const CUtensorMap& map_sfa, const CUtensorMap& map_sfb, const CUtensorMap& map_d,
                 const CUtensorMap& map_c, const gemm::Params& p, int64_t tiles, cudaStream_t stream) {
@@ -958,7 +969,7 @@ int launch_gemm(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtens
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    if (cudaFuncSetAttribute(gemm::nvfp4_gemm_kernel<kAlt>,
+    if (cudaFuncSetAttribute(gemm::nvfp4_gemm_kernel<kAlt, kEpi>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                              gemm::kSmemBytes) != cudaSuccess)
       return NVFP4_ERR_LAUNCH_FAILED;
@@ -967,7 +978,7 @@ int launch_gemm(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtens
   // one CTA pair (cluster of two) per pair of SMs, each pair walking its tiles
   const int max_pairs = sm_count() / 2;
   const unsigned pairs = (unsigned)(tiles < max_pairs ? tiles : max_pairs);
-  return launch_dependent(gemm::nvfp4_gemm_kernel<kAlt>, dim3(2 * pairs, 1, 1), gemm::kThreads, gemm::kSmemBytes, 2,
+  return launch_dependent(gemm::nvfp4_gemm_kernel<kAlt, kEpi>, dim3(2 * pairs, 1, 1), gemm::kThreads, gemm::kSmemBytes, 2,
                           stream, map_a, map_b, map_b_narrow, map_sfa, map_sfb, map_d, map_c, p);
 }
 
@@ -1058,10 +1069,26 @@ int gemm_impl(const uint8_t* a_packed, const uint8_t* b_packed, const uint8_t* a
   if (d_amax_dev && cudaMemsetAsync(d_amax_dev, 0, sizeof(float), st) != cudaSuccess)
     return NVFP4_ERR_LAUNCH_FAILED;
   const int64_t tiles = (int64_t)p.m_tiles * (p.n_a > p.n_b ? p.n_a : p.n_b);
-  return alt || narrow ? launch_gemm<true>(map_a, map_b, map_b_narrow, map_sfa, map_sfb, map_d, map_c, p,
-                                           tiles, st)
-                       : launch_gemm<false>(map_a, map_b, map_b_narrow, map_sfa, map_sfb, map_d, map_c, p,
-                                            tiles, st);
+  auto launch = [&](auto kernel_epi) {
+    constexpr int kEpi = decltype(kernel_epi)::value;
+    return alt || narrow
+               ? launch_gemm<true, kEpi>(map_a, map_b, map_b_narrow, map_sfa, map_sfb, map_d, map_c, p, tiles, st)
+               : launch_gemm<false, kEpi>(map_a, map_b, map_b_narrow, map_sfa, map_sfb, map_d, map_c, p, tiles, st);
+  };
+#define NVFP4_EPI(E) \
+  case (E): return launch(std::integral_constant<int, (E)>())
+  using namespace gemm;
+  switch ((bias_bf16 ? kEpiBias : 0) | (act == NVFP4_ACT_GELU_TANH ? kEpiGelu : 0) | (gate_f32 ? kEpiGate : 0) |
+          (c_bf16 ? kEpiResidual : 0) | (d_amax_dev ? kEpiAmax : 0)) {
+    NVFP4_EPI(0);
+    NVFP4_EPI(kEpiBias);
+    NVFP4_EPI(kEpiBias | kEpiGelu);
+    NVFP4_EPI(kEpiBias | kEpiGelu | kEpiAmax);
+    NVFP4_EPI(kEpiBias | kEpiResidual);
+    NVFP4_EPI(kEpiBias | kEpiGate | kEpiResidual);
+    default: return launch(std::integral_constant<int, kEpiAny>());
+  }
+#undef NVFP4_EPI
 }
 
 }  // namespace
