@@ -373,14 +373,17 @@ struct Tile {
 // Alternating tiling: wide and narrow tiles form two lists numbered like the uniform tiles
 // (tile_coords over the list's columns); pair q takes items q, q + Q, ... of each list, wide
 // on its even turns and narrow on its odd ones, and finishes whichever list is left over.
-template <bool kAlt>
+// kNarrowOne: tiles of at most 128 columns, which lie in one scale atom.
+enum { kUniform, kAlternating, kNarrow, kNarrowOne };
+
+template <int kTiling>
 struct TileWalk {
   int m_tiles, N, stride, n_a, n_b, i_a, i_b, t, tile_w;
   __device__ TileWalk(const Params& p, int pair, int num_pairs)
       : m_tiles(p.m_tiles), N(p.N), stride(num_pairs), n_a(p.n_a), n_b(p.n_b), i_a(pair),
         i_b(pair), t(0), tile_w(p.tile_w) {}
   __device__ __forceinline__ bool next(Tile& o) {
-    if (!kAlt) {
+    if (kTiling == kUniform) {
       if (i_a >= m_tiles * n_a) return false;
       int nt;
       tile_coords(i_a, m_tiles, n_a, o.mt, nt);
@@ -391,7 +394,7 @@ struct TileWalk {
       ++t;
       return true;
     }
-    if (tile_w > 0) {
+    if (kTiling >= kNarrow) {
       if (i_a >= m_tiles * n_a) return false;
       int nt;
       tile_coords(i_a, m_tiles, n_a, o.mt, nt);
@@ -426,10 +429,14 @@ struct TileWalk {
 };
 
 // What an epilogue does beyond scaling, as known when the kernel is compiled (kEpiAny: as its parameters say).  With the
-// checks in the kernel every 8-column piece was several branches and the pieces could not be interleaved.
+// checks in the kernel every 8-column piece was several branches and the pieces could not be interleaved.  The epilogue
+// bounds a GEMM of short K; us before and after, plain: 4096 x 3072 x 3072 21.2 -> 19.9, 27280 x 14336 x 3072 with GELU 524
+// -> 491, with gate and residual 4095 x 5120 x 5120 51.0 -> 46.5, 27280 x 3072 x 3072 138 -> 121, 1760 x 3072 x 3072 19.4 ->
+// 14.9, 27280 x 3072 x 14336 427 -> 425.  (More than the parameters' 128 bytes take the compiler to other code for the
+// general one, 4 % slower.)
 enum { kEpiBias = 1, kEpiGelu = 2, kEpiGate = 4, kEpiResidual = 8, kEpiAmax = 16, kEpiAny = -1 };
 
-template <bool kAlt, int kEpi>
+template <int kTiling, int kEpi>
 __global__ void __launch_bounds__(kThreads, 1)
 nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
                   const __grid_constant__ CUtensorMap map_b,
@@ -438,6 +445,8 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
                   const __grid_constant__ CUtensorMap map_sfb,
                   const __grid_constant__ CUtensorMap map_d,
                   const __grid_constant__ CUtensorMap map_c, const Params p) {
+  constexpr bool kAlt = kTiling != kUniform;     // two accumulators of their own columns
+  constexpr bool kOneAtom = kTiling == kNarrowOne;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -509,7 +518,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
     int s = 0;
     uint32_t ph = 0;
     bool ok = true;
-    TileWalk<kAlt> walk(p, pair, num_pairs);
+    TileWalk<kTiling> walk(p, pair, num_pairs);
     Tile tl;
     while (ok && walk.next(tl)) {
       // first scale atom of this CTA's A rows / of the two 128-row atoms that cover the tile's
@@ -517,12 +526,12 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       const int sfa_atom = (2 * tl.mt + (int)rank) * p.k_atoms;
       const int sfb_atom0 = (tl.n0 >> 7) * p.k_atoms;
       const int sfb_atom1 = sfb_atom0 + p.k_atoms;
-      // this CTA's half of the tile's B rows; narrower tiles use a box of half their width
-      const bool narrow = kAlt && (tl.buf == 1 || p.tile_w > 0);
+      // this CTA's half of the tile's B rows; narrower tiles use a box of half their width (the narrow tilings'
+      // only map: one picked at run time costs the warp 40 cycles a stage)
+      const bool narrow = kTiling == kAlternating && tl.buf == 1;
       const int b_row = tl.n0 + (int)rank * (tl.w >> 1);
-      const CUtensorMap* mb = narrow ? &map_b_narrow : &map_b;
-      const int narrow_bytes = p.tile_w > 0 ? p.tile_w / 2 * (BK / 2) : kBBytesNarrow;
-      const uint32_t stage_tx = 2u * (uint32_t)(kStageBytes - (narrow ? kBBytes - narrow_bytes : 0));
+      const int b_bytes = kTiling >= kNarrow ? p.tile_w / 2 * (BK / 2) : narrow ? kBBytesNarrow : kBBytes;
+      const uint32_t stage_tx = 2u * (uint32_t)(kStageBytes - (kBBytes - b_bytes) - (kOneAtom ? kSfbBytes / 2 : 0));
       for (int kt = 0; kt < p.k_tiles; ++kt) {
         ok = mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, p.status, 0x100 + s);
         ok = __all_sync(0xffffffffu, ok);
@@ -534,13 +543,15 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         const uint32_t lead_full = mapa_u32(full_bar(s), 0);
         mbar_expect_tx(full_bar(s), stage_tx, rank == 0 ? on : 0u);
         tma_load_2d(&map_a, lead_full, st, kt * (BK / 2), (2 * tl.mt + (int)rank) * BM, keep, on);
-        tma_load_2d(mb, lead_full, st + kABytes, kt * (BK / 2), b_row, keep, on);
+        tma_load_2d(kTiling == kAlternating && narrow ? &map_b_narrow : &map_b, lead_full, st + kABytes, kt * (BK / 2),
+                    b_row, keep, on);
         tma_load_2d(&map_sfa, lead_full, st + kABytes + kBBytes, 0, sfa_atom + kt * (BK / 64), keep,
                     on);
         tma_load_2d(&map_sfb, lead_full, st + kABytes + kBBytes + kSfaBytes, 0,
                     sfb_atom0 + kt * (BK / 64), keep, on);
-        tma_load_2d(&map_sfb, lead_full, st + kABytes + kBBytes + kSfaBytes + kSfbBytes / 2, 0,
-                    sfb_atom1 + kt * (BK / 64), keep, on);
+        if (!kOneAtom)
+          tma_load_2d(&map_sfb, lead_full, st + kABytes + kBBytes + kSfaBytes + kSfbBytes / 2, 0,
+                      sfb_atom1 + kt * (BK / 64), keep, on);
         if (++s == kStages) {
           s = 0;
           ph ^= 1u;
@@ -566,7 +577,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       int uses0 = 0, uses1 = 0;                         // tiles each accumulator has held
       const uint32_t sfa_t = tmem_base + kSfCol;        // SFA of K-block j at +4j
       const uint32_t sfb_t = tmem_base + kSfCol + 16;   // SFB of K-block j at +8j (two atoms)
-      TileWalk<kAlt> walk(p, pair, num_pairs);
+      TileWalk<kTiling> walk(p, pair, num_pairs);
       Tile tl;
       while (ok && walk.next(tl)) {
         const int t = walk.t - 1;                       // ordinal of this tile
@@ -586,7 +597,8 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
           for (int j = 0; j < BK / 64; ++j) {
             tc_cp_sf_pair(sfa_t + 4 * j, desc_sf(sfa_s + j * kSfAtomBytes), on);
             tc_cp_sf_pair(sfb_t + 8 * j, desc_sf(sfb_s + j * kSfAtomBytes), on);
-            tc_cp_sf_pair(sfb_t + 8 * j + 4, desc_sf(sfb_s + kSfbBytes / 2 + j * kSfAtomBytes), on);
+            if (!kOneAtom)
+              tc_cp_sf_pair(sfb_t + 8 * j + 4, desc_sf(sfb_s + kSfbBytes / 2 + j * kSfAtomBytes), on);
           }
           if (kt == 0) {
             // Only the MMAs need the accumulator; the scale copies above went ahead of these
@@ -667,21 +679,13 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
     bool ok = true;
     uint32_t c_phase = 0;                // parity of this warp's residual-tile barrier
     int uses0 = 0, uses1 = 0;
-    TileWalk<kAlt> walk(p, pair, num_pairs);
+    TileWalk<kTiling> walk(p, pair, num_pairs);
     Tile tl;
     while (ok && walk.next(tl)) {
       const int buf = tl.buf;
       const uint32_t lead_acc_empty = buf ? lead_acc_empty1 : lead_acc_empty0;
-      ok = mbar_wait(acc_full_bar(buf), (uint32_t)(buf ? uses1 : uses0) & 1u, abort_flag, p.status,
-                     0x400 + buf);
-      if (buf) ++uses1; else ++uses0;
-      // the whole warp must agree before the .sync.aligned loads below
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      tc_fence_after();
       const int row0 = (2 * tl.mt + (int)rank) * BM + q * 32;
       const int row = row0 + lane;
-      const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + acc_col(buf);
       constexpr int kGroups = BN / 64;   // uniform tiling: the first group processed is the one
                                          // both accumulators share
       static_assert(256 - kAccCol1 == 64, "the shared columns must be exactly one group");
@@ -691,6 +695,30 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       if (kAlt) g_first = warp >= 6 ? per_half : 0;
       const int end = g_first + per_half < n_groups ? g_first + per_half : n_groups;
       const int last_gi = g_first >= n_groups ? -1 : end - 1;
+      // tensor-memory column group: the uniform tiling walks them so that the shared group
+      // comes first
+      auto column_group = [&](int gi) { return kAlt ? gi : (buf ? gi : (gi + kGroups - 1) % kGroups); };
+      uint4 bb[8];
+      auto load_bias = [&](int col0) {
+#pragma unroll
+        for (int g = 0; g < 8; ++g)
+          bb[g] = col0 + g * 8 < p.N
+                      ? load_u32x4(p.bias + col0 + g * 8)
+                      : make_uint4(0, 0, 0, 0);
+      };
+      // Wide tiles: asked for ahead of the sums, and for the second group when the first has left.  (27280 x 14336 x 3072
+      // with GELU 498 -> 496 us, 4096 x 3072 x 3072 20.1 -> 19.6.  In the other tilings, and for the residual's tile,
+      // that is slower: 512 x 3072 x 4096 10.7 -> 11.3, 4095 x 5120 x 5120 with gate and residual 47.7 -> 50.4.)
+      constexpr bool kEarlyBias = !kAlt && kEpi >= 0 && !(kEpi & kEpiResidual);
+      if (kEarlyBias && with_bias) load_bias(tl.n0 + column_group(g_first) * 64);
+      ok = mbar_wait(acc_full_bar(buf), (uint32_t)(buf ? uses1 : uses0) & 1u, abort_flag, p.status,
+                     0x400 + buf);
+      if (buf) ++uses1; else ++uses0;
+      // the whole warp must agree before the .sync.aligned loads below
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + acc_col(buf);
       if (kAlt && last_gi < 0) {
         // nothing of this tile is ours; the accumulator's barrier still counts every warp
         __syncwarp();
@@ -702,12 +730,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
       for (int gj = 0; gj < 2; ++gj) {
         const int gi = g_first + gj;
         if (kAlt && gi > last_gi) break;
-        // tensor-memory column group: the uniform tiling walks them so that the shared group
-        // comes first
-        const int cg = kAlt ? gi : (buf ? gi : (gi + kGroups - 1) % kGroups);
-        const int col0 = tl.n0 + cg * 64;
-        // tensor-memory loads first (they are asynchronous until the wait below): for the
-        // shared group they sit on the path to the next tile's first MMA
+        const int cg = column_group(gi), col0 = tl.n0 + cg * 64;
         tc_ld_32x32(acc + cg * 64, *reinterpret_cast<uint32_t(*)[32]>(&x[0]));
         tc_ld_32x32(acc + cg * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&x[32]));
         // The residual tile (32 rows x 64 columns of C) comes into the slab by one TMA load, in
@@ -741,14 +764,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
           if (lane == 0) mbar_arrive_cluster(mapa_u32(acc_rest_bar(buf), 0));
         }
         // per-column operands of the whole group first, so that their loads overlap
-        uint4 bb[8];
-        if (with_bias) {
-#pragma unroll
-          for (int g = 0; g < 8; ++g)
-            bb[g] = col0 + g * 8 < p.N
-                        ? load_u32x4(p.bias + col0 + g * 8)
-                        : make_uint4(0, 0, 0, 0);
-        }
+        if (!kEarlyBias && with_bias) load_bias(col0);
         // stacked weights: the tensor scale of the weight this group's columns belong to
         const float scale = (p.gb_group > 0 && col0 < p.N)
                                 ? scale_a * load_f32(p.gb + col0 / p.gb_group) : scale_ab;
@@ -766,6 +782,14 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         // epilogue warps have about as many issue slots per tile as the main loop has cycles.
         const float2 scale2 = make_float2(scale, scale);
         const float2 beta2 = make_float2(p.beta, p.beta);
+        // (All of the residual's row ahead of the loop: the compiler cannot tell a piece's place from that of the result
+        // stored before it, and would read them one after the other.)
+        uint4 cc[8];
+        if (with_c) {
+#pragma unroll
+          for (int g = 0; g < 8; ++g)
+            cc[g] = *reinterpret_cast<const uint4*>(slab + lane * 128 + ((g ^ (lane & 7)) << 4));
+        }
 #pragma unroll
         for (int g = 0; g < 8; ++g) {
           float2 v[4];
@@ -787,17 +811,16 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
 #pragma unroll
             for (int e = 0; e < 4; ++e) v[e] = gelu_tanh2(v[e]);
           }
-          if (with_gate && in_n) {
-            const float4 g0 = load_f32x4(p.gate + col0 + g * 8);
-            const float4 g1 = load_f32x4(p.gate + col0 + g * 8 + 4);
+          if (with_gate) {      // (past N: any, nothing of it is stored)
+            const float* gate = p.gate + (in_n ? col0 + g * 8 : 0);
+            const float4 g0 = load_f32x4(gate), g1 = load_f32x4(gate + 4);
             v[0] = f2_mul(v[0], make_float2(g0.x, g0.y));
             v[1] = f2_mul(v[1], make_float2(g0.z, g0.w));
             v[2] = f2_mul(v[2], make_float2(g1.x, g1.y));
             v[3] = f2_mul(v[3], make_float2(g1.z, g1.w));
           }
           if (with_c) {   // rows past M and columns past N were zero-filled by the load
-            const uint4 cc = *reinterpret_cast<const uint4*>(slab + lane * 128 + ((g ^ (lane & 7)) << 4));
-            const uint32_t cw[4] = {cc.x, cc.y, cc.z, cc.w};
+            const uint32_t cw[4] = {cc[g].x, cc[g].y, cc[g].z, cc[g].w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) v[e] = f2_fma(beta2, bf16x2_to_f2(cw[e]), v[e]);
           }
@@ -818,6 +841,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
         tma_store_2d(&map_d, smem_u32(slab), col0, row0, stream_out,
                      (row0 < p.M && col0 < p.N) ? on : 0u);
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        if (kEarlyBias && with_bias && gj == 0) load_bias(tl.n0 + column_group(gi + 1) * 64);
       }
     }
     // the CTA's shared memory must outlive the stores that read it
@@ -961,7 +985,7 @@ int tile_width(int64_t m_tiles, int64_t M, int64_t N, int64_t K) {
   return best;
 }
 
-template <bool kAlt, int kEpi>
+template <int kTiling, int kEpi>
 int launch_gemm(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_b_narrow,
                 const CUtensorMap& map_sfa, const CUtensorMap& map_sfb, const CUtensorMap& map_d,
                 const CUtensorMap& map_c, const gemm::Params& p, int64_t tiles, cudaStream_t stream) {
@@ -969,7 +993,7 @@ int launch_gemm(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtens
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    if (cudaFuncSetAttribute(gemm::nvfp4_gemm_kernel<kAlt, kEpi>,
+    if (cudaFuncSetAttribute(gemm::nvfp4_gemm_kernel<kTiling, kEpi>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                              gemm::kSmemBytes) != cudaSuccess)
       return NVFP4_ERR_LAUNCH_FAILED;
@@ -978,7 +1002,7 @@ int launch_gemm(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtens
   // one CTA pair (cluster of two) per pair of SMs, each pair walking its tiles
   const int max_pairs = sm_count() / 2;
   const unsigned pairs = (unsigned)(tiles < max_pairs ? tiles : max_pairs);
-  return launch_dependent(gemm::nvfp4_gemm_kernel<kAlt, kEpi>, dim3(2 * pairs, 1, 1), gemm::kThreads, gemm::kSmemBytes, 2,
+  return launch_dependent(gemm::nvfp4_gemm_kernel<kTiling, kEpi>, dim3(2 * pairs, 1, 1), gemm::kThreads, gemm::kSmemBytes, 2,
                           stream, map_a, map_b, map_b_narrow, map_sfa, map_sfb, map_d, map_c, p);
 }
 
@@ -1008,17 +1032,16 @@ int gemm_impl(const uint8_t* a_packed, const uint8_t* b_packed, const uint8_t* a
   const int64_t m_tiles = (M + 2 * gemm::BM - 1) / (2 * gemm::BM);     // 256-row pair tiles
   const int width = g_tiling_mode == 0 ? tile_width(m_tiles, M, N, K) : gemm::BN;
   const bool narrow = width < gemm::BN, alt = g_tiling_mode == 2;
-  const int narrow_w = narrow ? width : gemm::kAltNarrow;
 
   CUtensorMap map_a, map_b, map_b_narrow, map_sfa, map_sfb, map_d, map_c;
   if (!gemm::make_map(&map_a, a_packed, M, K / 2, gemm::BM) ||
-      !gemm::make_map(&map_b, b_packed, N, K / 2, gemm::BN / 2) ||
-      ((narrow || alt) && !gemm::make_map(&map_b_narrow, b_packed, N, K / 2, narrow_w / 2)) ||
+      !gemm::make_map(&map_b, b_packed, N, K / 2, width / 2) ||
+      (alt && !gemm::make_map(&map_b_narrow, b_packed, N, K / 2, gemm::kAltNarrow / 2)) ||
       !gemm::make_sf_map(&map_sfa, a_scales_swizzled, sf_row_tiles(M) * sf_k_atoms(K)) ||
       !gemm::make_sf_map(&map_sfb, b_scales_swizzled, sf_row_tiles(N) * sf_k_atoms(K)) ||
       !gemm::make_d_map(&map_d, d_bf16, M, N))
     return NVFP4_ERR_LAUNCH_FAILED;
-  if (!narrow && !alt) map_b_narrow = map_b;   // never dereferenced
+  if (!alt) map_b_narrow = map_b;   // never dereferenced
   // beta == 0 means C is not read at all (BLAS convention): a NaN in it cannot reach D
   if (beta == 0.0f) c_bf16 = nullptr;
   if (c_bf16) {
@@ -1071,9 +1094,10 @@ int gemm_impl(const uint8_t* a_packed, const uint8_t* b_packed, const uint8_t* a
   const int64_t tiles = (int64_t)p.m_tiles * (p.n_a > p.n_b ? p.n_a : p.n_b);
   auto launch = [&](auto kernel_epi) {
     constexpr int kEpi = decltype(kernel_epi)::value;
-    return alt || narrow
-               ? launch_gemm<true, kEpi>(map_a, map_b, map_b_narrow, map_sfa, map_sfb, map_d, map_c, p, tiles, st)
-               : launch_gemm<false, kEpi>(map_a, map_b, map_b_narrow, map_sfa, map_sfb, map_d, map_c, p, tiles, st);
+    auto* fn = !narrow ? launch_gemm<gemm::kUniform, kEpi>
+                       : width <= 128 ? launch_gemm<gemm::kNarrowOne, kEpi> : launch_gemm<gemm::kNarrow, kEpi>;
+    if (alt) fn = launch_gemm<gemm::kAlternating, gemm::kEpiAny>;
+    return fn(map_a, map_b, map_b_narrow, map_sfa, map_sfb, map_d, map_c, p, tiles, st);
   };
 #define NVFP4_EPI(E) \
   case (E): return launch(std::integral_constant<int, (E)>())
