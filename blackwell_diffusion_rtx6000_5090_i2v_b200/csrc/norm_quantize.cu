@@ -28,12 +28,17 @@
 // warp stage folds the 2 kR values instead of reducing them one by one; the divisions of
 // the quantizer are gone (x/6 by an exact three-operation form, the encode scale from a
 // 128-entry table per tensor); scale offsets split into a per-row and a per-thread part.
+// What is known of a call is a template parameter (kWhole), the widening of x is part of its subtraction, |h| and its
+// maximum are one instruction, and the means' divisions are three operations.  Both sweeps, us, before and after:
+// [27280, 3072] modulation 96.4 -> 82.1, affine 96.4 -> 81.9, all four vectors 147 -> 123, [32760, 5120] modulation 186 -> 157,
+// [12000, 6384] 152 -> 122; 31 M -> 25 M instructions a sweep.
 // Sweep 1 leaves mean and rstd per row in a small stats buffer so that sweep 2, which needs
 // no reduction at all, repeats exactly the same arithmetic.
 //
 // Sweep 1 walks the groups forwards and sweep 2 walks them backwards with an evict-first
 // hint: the tail of x that sweep 1 left in L2 (126 MB) is what sweep 2 reads first.
 #include <atomic>
+#include <type_traits>
 
 #include <cooperative_groups.h>
 
@@ -151,6 +156,17 @@ __device__ __forceinline__ void wait_group(uint32_t bar, uint32_t parity, volati
   }
 }
 
+// x / n, bit-identical to the IEEE quotient, with `inv` the rounded reciprocal of n: a product and one residual
+// correction (P. Markstein, IBM J. Res. Dev. 34, 1990).  Where the residual is not exact or not a number, the division.
+template <bool kFast>
+__device__ __forceinline__ float div_by(float x, float n, float inv) {
+  if (!kFast) return __fdiv_rn(x, n);
+  const float q0 = __fmul_rn(x, inv);
+  const float q = __fmaf_rn(__fmaf_rn(-n, q0, x), inv, q0);
+  const float a = fabsf(x);
+  return (a >= 1e-25f && a <= 1e37f) ? q : __fdiv_rn(x, n);
+}
+
 // One fold step of the multi-value warp sum: a lane hands kHalf of its 2*kHalf values to the
 // partner across `mask` and keeps the sums of the other kHalf.
 template <int kHalf>
@@ -206,17 +222,24 @@ __device__ __forceinline__ void cta_sum(float (&v)[kV], float (*red)[kMaxWarps],
   }
 }
 
-// h for one 16-element block as 8 packed bf16 pairs, and the running bf16x2 max of |h|.
+// Both lanes of a bf16 pair minus m, in fp32 (exact widening, one rounding): no instruction for the widening.
+__device__ __forceinline__ float2 bf16x2_sub(uint32_t w, float m) {
+  float2 d;
+  asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %2;\n\tsub.rn.f32.bf16 %0, lo, %3;\n\tsub.rn.f32.bf16 %1, hi, %3;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "r"(w), "f"(m));
+  return d;
+}
+
+// h for one 16-element block as 8 packed bf16 pairs, and the running bf16x2 max of |h| and a2, whose signs mean nothing.
 template <bool kAffine, bool kMod>
-__device__ __forceinline__ uint32_t normalize16(const uint32_t (&xp)[8], float2 m2, float2 r2,
+__device__ __forceinline__ uint32_t normalize16(uint32_t a2, const uint32_t (&xp)[8], float2 m2, float2 r2,
                                                 const float2 (&cw)[8], const float2 (&cb)[8],
                                                 const float2 (&cs)[8], const float2 (&ct)[8],
                                                 bool has_w, bool has_b, bool has_s, bool has_t,
                                                 uint32_t (&hp)[8]) {
-  uint32_t a2 = 0u;
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
-    float2 y = f2_mul(f2_sub(bf16x2_to_f2(xp[e]), m2), r2);
+    float2 y = f2_mul(bf16x2_sub(xp[e], m2.x), r2);
     if (kAffine) {
       if (has_w) y = f2_mul(y, cw[e]);
       if (has_b) y = f2_add(y, cb[e]);
@@ -227,12 +250,14 @@ __device__ __forceinline__ uint32_t normalize16(const uint32_t (&xp)[8], float2 
     }
     // the quantizer's input is the bf16 tensor the unfused model would have produced
     hp[e] = f2_to_bf16x2(y);
-    a2 = bf16x2_max_abs(a2, hp[e]);
+    asm("max.xorsign.abs.bf16x2 %0, %0, %1;" : "+r"(a2) : "r"(hp[e]));     // one instruction, where abs and max are two
   }
   return a2;
 }
 
-template <bool kQuantize, int kJ, bool kAffine, bool kMod>
+// kWhole: both vectors of every kind are given and every thread has blocks (T * kJ * 16 == cols), so that nothing of that
+// is asked for each pair of elements or block.
+template <bool kQuantize, int kJ, bool kAffine, bool kMod, bool kWhole>
 __global__ void __launch_bounds__(kMaxThreads)
 norm_mod_kernel(const NormArgs p) {
   constexpr int kR = RowsPerIter<kJ>::value;
@@ -302,16 +327,16 @@ norm_mod_kernel(const NormArgs p) {
 #pragma unroll
   for (int j = 0; j < kJ; ++j) {
     const int u = threadIdx.x + j * T;
-    live[j] = u < units;
+    live[j] = kWhole || u < units;
     const int col = live[j] ? u * 16 : 0;
     swz_kb[j] = (int64_t)(u >> 2) * kSfAtomBytes + (u & 3);
     if (kAffine) {
-      has_w = p.w != nullptr; has_b = p.b != nullptr;
+      has_w = kWhole || p.w != nullptr; has_b = kWhole || p.b != nullptr;
       if (has_w) load16(p.w + col, cw[j]);
       if (has_b) load16(p.b + col, cb[j]);
     }
     if (kMod) {
-      has_s = p.scale != nullptr; has_t = p.shift != nullptr;
+      has_s = kWhole || p.scale != nullptr; has_t = kWhole || p.shift != nullptr;
       if (has_s) {
         load16(p.scale + col, cs[j]);
 #pragma unroll
@@ -322,7 +347,7 @@ norm_mod_kernel(const NormArgs p) {
   }
 
   uint32_t amax_t = 0u;                 // bf16x2 running max of |h| (sweep 1)
-  const float cols_f = (float)p.cols;
+  const float cols_f = (float)p.cols, cols_inv = __fdiv_rn(1.0f, cols_f);
 
   // sweep 2 asks for a group's row statistics one group ahead: the load would otherwise sit
   // at the head of every group's dependency chain
@@ -361,16 +386,15 @@ norm_mod_kernel(const NormArgs p) {
     float pivot[kR];                    // first element of the row
 #pragma unroll
     for (int r = 0; r < kR; ++r) {
-      row_ok[r] = base + r < p.rows;
+      row_ok[r] = r == 0 || base + r < p.rows;
       const uint4* src = reinterpret_cast<const uint4*>(slot_ptr + (size_t)r * row_bytes);
       pivot[r] = (!kQuantize && !p.rms && row_ok[r])
                      ? bf16lo_to_f32(*reinterpret_cast<const uint32_t*>(src)) : 0.0f;
 #pragma unroll
       for (int j = 0; j < kJ; ++j) {
-        const bool on = live[j] && row_ok[r];
-        const int u = threadIdx.x + j * T;
-        const uint4 a = on ? src[2 * u] : make_uint4(0, 0, 0, 0);
-        const uint4 b = on ? src[2 * u + 1] : make_uint4(0, 0, 0, 0);
+        // (a thread without a block reads another's, a row past the end what the slot held: neither is used)
+        const int u = live[j] ? threadIdx.x + j * T : 0;
+        const uint4 a = src[2 * u], b = src[2 * u + 1];
         xp[r][j][0] = a.x; xp[r][j][1] = a.y; xp[r][j][2] = a.z; xp[r][j][3] = a.w;
         xp[r][j][4] = b.x; xp[r][j][5] = b.y; xp[r][j][6] = b.z; xp[r][j][7] = b.w;
       }
@@ -394,7 +418,7 @@ norm_mod_kernel(const NormArgs p) {
           if (live[j] && row_ok[r]) {
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-              const float2 d = f2_sub(bf16x2_to_f2(xp[r][j][e]), p2);
+              const float2 d = bf16x2_sub(xp[r][j][e], p2.x);
               s1 = f2_add(s1, d);
               s2 = f2_fma(d, d, s2);
             }
@@ -407,10 +431,10 @@ norm_mod_kernel(const NormArgs p) {
       refill();
 #pragma unroll
       for (int r = 0; r < kR; ++r) {
-        const float m1 = acc[2 * r] / cols_f;
-        const float var = fmaxf(acc[2 * r + 1] / cols_f - m1 * m1, 0.0f);
+        const float m1 = div_by<kWhole>(acc[2 * r], cols_f, cols_inv), m2 = div_by<kWhole>(acc[2 * r + 1], cols_f, cols_inv);
+        const float var = fmaxf(m2 - m1 * m1, 0.0f);
         mean[r] = p.rms ? 0.0f : pivot[r] + m1;
-        rstd[r] = rsqrtf((p.rms ? acc[2 * r + 1] / cols_f : var) + p.eps);
+        rstd[r] = rsqrtf((p.rms ? m2 : var) + p.eps);
         if (threadIdx.x == 0 && row_ok[r])
           reinterpret_cast<float2*>(p.stats)[base + r] = make_float2(mean[r], rstd[r]);
       }
@@ -454,11 +478,11 @@ norm_mod_kernel(const NormArgs p) {
         const bool on = live[j] && row_ok[r];
         uint32_t hp[8];
         const uint32_t a2 = normalize16<kAffine, kMod>(
-            xp[r][j], m2, r2, cw[kAffine ? j : 0], cb[kAffine ? j : 0], cs[kMod ? j : 0],
+            kQuantize ? 0u : amax_t, xp[r][j], m2, r2, cw[kAffine ? j : 0], cb[kAffine ? j : 0], cs[kMod ? j : 0],
             ct[kMod ? j : 0], has_w, has_b, has_s, has_t, hp);
         if (!kQuantize) {
           if (on) {
-            amax_t = bf16x2_max_abs(amax_t, a2);
+            amax_t = a2;
             if (p.h_out) {
               uint4* dst = p.h_out + (row * units + u) * 2;
               dst[0] = make_uint4(hp[0], hp[1], hp[2], hp[3]);
@@ -466,7 +490,7 @@ norm_mod_kernel(const NormArgs p) {
             }
           }
         } else if (on) {
-          const float amax_b = fmaxf(bf16lo_to_f32(a2), bf16hi_to_f32(a2));
+          const float amax_b = fmaxf(fabsf(bf16lo_to_f32(a2)), fabsf(bf16hi_to_f32(a2)));
           float d = __fmul_rn(div_by_6(amax_b), s_enc);
           d = fminf(d, FLT_MAX);
           const uint8_t sf = (uint8_t)__nv_cvt_float_to_fp8(d, __NV_SATFINITE, __NV_E4M3);
@@ -491,7 +515,7 @@ norm_mod_kernel(const NormArgs p) {
   }
 
   if (!kQuantize) {
-    const float amax_f = fmaxf(bf16lo_to_f32(amax_t), bf16hi_to_f32(amax_t));
+    const float amax_f = fmaxf(fabsf(bf16lo_to_f32(amax_t)), fabsf(bf16hi_to_f32(amax_t)));
     const unsigned bits = __reduce_max_sync(0xffffffffu, __float_as_uint(amax_f));
     __syncthreads();
     if ((threadIdx.x & 31) == 0) red_max[threadIdx.x >> 5] = __uint_as_float(bits);
@@ -518,7 +542,7 @@ norm_mod_kernel(const NormArgs p) {
 // two sweeps, in their order.
 constexpr int kMaxGroups = 16;            // row groups of a CTA
 
-template <int kJ, bool kAffine, bool kMod>
+template <int kJ, bool kAffine, bool kMod, bool kWhole>
 __global__ void __launch_bounds__(kMaxThreads)
 norm_mod_resident_kernel(const NormArgs p, int per_cta, unsigned* partial) {
   constexpr int kR = RowsPerIter<kJ>::value;
@@ -555,11 +579,12 @@ norm_mod_resident_kernel(const NormArgs p, int per_cta, unsigned* partial) {
   float2 cw[kAffine ? kJ : 1][8], cb[kAffine ? kJ : 1][8];
   float2 cs[kMod ? kJ : 1][8], ct[kMod ? kJ : 1][8];
   int64_t swz_kb[kJ];
-  const bool has_w = kAffine && p.w, has_b = kAffine && p.b, has_s = kMod && p.scale, has_t = kMod && p.shift;
+  const bool has_w = kAffine && (kWhole || p.w), has_b = kAffine && (kWhole || p.b), has_s = kMod && (kWhole || p.scale),
+             has_t = kMod && (kWhole || p.shift);
 #pragma unroll
   for (int j = 0; j < kJ; ++j) {
     const int u = threadIdx.x + j * T;
-    live[j] = u < units;
+    live[j] = kWhole || u < units;
     const int col = live[j] ? u * 16 : 0;
     swz_kb[j] = (int64_t)(u >> 2) * kSfAtomBytes + (u & 3);
     if (has_w) load16(p.w + col, cw[j]);
@@ -585,7 +610,7 @@ norm_mod_resident_kernel(const NormArgs p, int per_cta, unsigned* partial) {
   __syncthreads();
 
   uint32_t amax_t = 0u;
-  const float cols_f = (float)p.cols;
+  const float cols_f = (float)p.cols, cols_inv = __fdiv_rn(1.0f, cols_f);
   for (int g = 0; g < my_groups; ++g) {
     wait_group(smem_u32(&full[g]), 0u, &abort_flag, p.status);
     uint8_t* group_ptr = rows_smem + (size_t)(g * kR) * row_bytes;
@@ -594,15 +619,14 @@ norm_mod_resident_kernel(const NormArgs p, int per_cta, unsigned* partial) {
     float pivot[kR];
 #pragma unroll
     for (int r = 0; r < kR; ++r) {
-      row_ok[r] = g * kR + r < my_rows;
+      row_ok[r] = r == 0 || g * kR + r < my_rows;
       const uint4* src = reinterpret_cast<const uint4*>(group_ptr + (size_t)r * row_bytes);
       pivot[r] = (!p.rms && row_ok[r]) ? bf16lo_to_f32(*reinterpret_cast<const uint32_t*>(src)) : 0.0f;
 #pragma unroll
       for (int j = 0; j < kJ; ++j) {
-        const bool on = live[j] && row_ok[r];
-        const int u = threadIdx.x + j * T;
-        const uint4 a = on ? src[2 * u] : make_uint4(0, 0, 0, 0);
-        const uint4 b = on ? src[2 * u + 1] : make_uint4(0, 0, 0, 0);
+        // (a thread without a block reads another's, a row past the end what the slot held: neither is used)
+        const int u = live[j] ? threadIdx.x + j * T : 0;
+        const uint4 a = src[2 * u], b = src[2 * u + 1];
         xp[r][j][0] = a.x; xp[r][j][1] = a.y; xp[r][j][2] = a.z; xp[r][j][3] = a.w;
         xp[r][j][4] = b.x; xp[r][j][5] = b.y; xp[r][j][6] = b.z; xp[r][j][7] = b.w;
       }
@@ -617,7 +641,7 @@ norm_mod_resident_kernel(const NormArgs p, int per_cta, unsigned* partial) {
         if (live[j] && row_ok[r]) {
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
-            const float2 d = f2_sub(bf16x2_to_f2(xp[r][j][e]), p2);
+            const float2 d = bf16x2_sub(xp[r][j][e], p2.x);
             s1 = f2_add(s1, d);
             s2 = f2_fma(d, d, s2);
           }
@@ -629,10 +653,10 @@ norm_mod_resident_kernel(const NormArgs p, int per_cta, unsigned* partial) {
     cta_sum<kV>(acc, red[g & 1], warps);
 #pragma unroll
     for (int r = 0; r < kR; ++r) {
-      const float m1 = acc[2 * r] / cols_f;
-      const float var = fmaxf(acc[2 * r + 1] / cols_f - m1 * m1, 0.0f);
+      const float m1 = div_by<kWhole>(acc[2 * r], cols_f, cols_inv), sq = div_by<kWhole>(acc[2 * r + 1], cols_f, cols_inv);
+      const float var = fmaxf(sq - m1 * m1, 0.0f);
       const float mean = p.rms ? 0.0f : pivot[r] + m1;
-      const float rstd = rsqrtf((p.rms ? acc[2 * r + 1] / cols_f : var) + p.eps);
+      const float rstd = rsqrtf((p.rms ? sq : var) + p.eps);
       const float2 m2 = make_float2(mean, mean), r2 = make_float2(rstd, rstd);
       uint4* dst = reinterpret_cast<uint4*>(group_ptr + (size_t)r * row_bytes);
 #pragma unroll
@@ -640,10 +664,10 @@ norm_mod_resident_kernel(const NormArgs p, int per_cta, unsigned* partial) {
         const int u = threadIdx.x + j * T;
         uint32_t hp[8];
         const uint32_t a2 = normalize16<kAffine, kMod>(
-            xp[r][j], m2, r2, cw[kAffine ? j : 0], cb[kAffine ? j : 0], cs[kMod ? j : 0], ct[kMod ? j : 0], has_w,
+            amax_t, xp[r][j], m2, r2, cw[kAffine ? j : 0], cb[kAffine ? j : 0], cs[kMod ? j : 0], ct[kMod ? j : 0], has_w,
             has_b, has_s, has_t, hp);
         if (live[j] && row_ok[r]) {
-          amax_t = bf16x2_max_abs(amax_t, a2);
+          amax_t = a2;
           dst[2 * u] = make_uint4(hp[0], hp[1], hp[2], hp[3]);
           dst[2 * u + 1] = make_uint4(hp[4], hp[5], hp[6], hp[7]);
         }
@@ -653,7 +677,7 @@ norm_mod_resident_kernel(const NormArgs p, int per_cta, unsigned* partial) {
 
   // the maximum of the CTA, then of the grid
   unsigned bits = __reduce_max_sync(0xffffffffu,
-                                    __float_as_uint(fmaxf(bf16lo_to_f32(amax_t), bf16hi_to_f32(amax_t))));
+                                    __float_as_uint(fmaxf(fabsf(bf16lo_to_f32(amax_t)), fabsf(bf16hi_to_f32(amax_t)))));
   if ((threadIdx.x & 31) == 0) red_max[threadIdx.x >> 5] = bits;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -730,9 +754,9 @@ void shape_for(int units, int kinds, int* j, int* threads) {
   *threads = ((per + 31) / 32) * 32;
 }
 
-template <bool kQuantize, int kJ, bool kAffine, bool kMod>
+template <bool kQuantize, int kJ, bool kAffine, bool kMod, bool kWhole>
 int launch_variant(const NormArgs& a, int threads, cudaStream_t st) {
-  auto kernel = norm_mod_kernel<kQuantize, kJ, kAffine, kMod>;
+  auto kernel = norm_mod_kernel<kQuantize, kJ, kAffine, kMod, kWhole>;
   constexpr int kR = RowsPerIter<kJ>::value;
   const size_t smem = (size_t)kStages * kR * a.cols * 2;
   // (dynamic shared memory limit, CTAs per SM) of the last geometry this variant saw on each
@@ -792,9 +816,9 @@ int groups_per_cta(Kernel kernel, int dev, int threads, int64_t groups, int64_t 
 }
 
 // Launches the one-launch form if the rows fit; *done says whether.
-template <int kJ, bool kAffine, bool kMod>
+template <int kJ, bool kAffine, bool kMod, bool kWhole>
 int launch_resident(const NormArgs& a, int threads, unsigned* partial, cudaStream_t st, bool* done) {
-  auto kernel = norm_mod_resident_kernel<kJ, kAffine, kMod>;
+  auto kernel = norm_mod_resident_kernel<kJ, kAffine, kMod, kWhole>;
   constexpr int kR = RowsPerIter<kJ>::value;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return NVFP4_ERR_BAD_ARG;
@@ -827,39 +851,36 @@ int launch_resident(const NormArgs& a, int threads, unsigned* partial, cudaStrea
   return e == cudaErrorCooperativeLaunchTooLarge ? NVFP4_OK : NVFP4_ERR_LAUNCH_FAILED;
 }
 
-int try_resident(const NormArgs& a, unsigned* partial, cudaStream_t st, bool* done) {
-  int J, threads;
+// Calls f with the variant of the kernels for these arguments: blocks per thread, affine, modulation, kWhole.
+template <typename F>
+int with_variant(const NormArgs& a, int* threads, F&& f) {
+  int J;
   const bool affine = a.w || a.b, mod = a.scale || a.shift;
-  shape_for(a.cols / 16, affine + mod, &J, &threads);
-#define NVFP4_NORM_CASE(JJ)                                                                       \
-  if (J == JJ) {                                                                                  \
-    if (affine && mod) return launch_resident<JJ, true, true>(a, threads, partial, st, done);     \
-    if (affine) return launch_resident<JJ, true, false>(a, threads, partial, st, done);           \
-    if (mod) return launch_resident<JJ, false, true>(a, threads, partial, st, done);              \
-    return launch_resident<JJ, false, false>(a, threads, partial, st, done);                      \
-  }
-  NVFP4_NORM_CASE(1)
-  NVFP4_NORM_CASE(2)
-#undef NVFP4_NORM_CASE
-  return NVFP4_ERR_BAD_ARG;
+  shape_for(a.cols / 16, affine + mod, &J, threads);
+  const bool whole = (!affine || (a.w && a.b)) && (!mod || (a.scale && a.shift)) && *threads * J * 16 == a.cols;
+  auto go = [&](auto j, auto with_affine, auto with_mod) {
+    return whole ? f(j, with_affine, with_mod, std::true_type()) : f(j, with_affine, with_mod, std::false_type());
+  };
+  auto kinds = [&](auto j) {
+    if (affine) return mod ? go(j, std::true_type(), std::true_type()) : go(j, std::true_type(), std::false_type());
+    return mod ? go(j, std::false_type(), std::true_type()) : go(j, std::false_type(), std::false_type());
+  };
+  return J == 1 ? kinds(std::integral_constant<int, 1>()) : kinds(std::integral_constant<int, 2>());
+}
+
+int try_resident(const NormArgs& a, unsigned* partial, cudaStream_t st, bool* done) {
+  int threads;
+  return with_variant(a, &threads, [&](auto j, auto affine, auto mod, auto whole) {
+    return launch_resident<j(), affine(), mod(), whole()>(a, threads, partial, st, done);
+  });
 }
 
 template <bool kQuantize>
 int launch(const NormArgs& a, cudaStream_t st) {
-  int J, threads;
-  const bool affine = a.w || a.b, mod = a.scale || a.shift;
-  shape_for(a.cols / 16, affine + mod, &J, &threads);
-#define NVFP4_NORM_CASE(JJ)                                                           \
-  if (J == JJ) {                                                                      \
-    if (affine && mod) return launch_variant<kQuantize, JJ, true, true>(a, threads, st);   \
-    if (affine) return launch_variant<kQuantize, JJ, true, false>(a, threads, st);    \
-    if (mod) return launch_variant<kQuantize, JJ, false, true>(a, threads, st);       \
-    return launch_variant<kQuantize, JJ, false, false>(a, threads, st);               \
-  }
-  NVFP4_NORM_CASE(1)
-  NVFP4_NORM_CASE(2)
-#undef NVFP4_NORM_CASE
-  return NVFP4_ERR_BAD_ARG;
+  int threads;
+  return with_variant(a, &threads, [&](auto j, auto affine, auto mod, auto whole) {
+    return launch_variant<kQuantize, j(), affine(), mod(), whole()>(a, threads, st);
+  });
 }
 
 }  // namespace
