@@ -11,6 +11,7 @@
 //   rows      a thread owns one scale block of every row, four rows at a time: rows that one CTA spans
 //   resident  amax and packing in one cooperative launch that holds the tensor in shared memory
 //   flat      blocks numbered through the tensor: everything else
+#include <algorithm>
 #include <atomic>
 
 #include <cooperative_groups.h>
@@ -26,28 +27,67 @@ constexpr int kBlocksPerThread = 2;  // two 16-element scale blocks (64 B of inp
 
 // ---------------------------------------------------------------- amax ----
 
-// kPartial: every CTA leaves its own maximum in out[blockIdx.x] for the packing kernel to combine,
-// so that no slot has to be zeroed first, and launched by launch_dependent(); else one atomic per CTA
-// on the zeroed slot.  kTensors: how many tensors share the launch (AmaxJob), each with its own CTAs.
+// Two forms.  For a slot: one atomic per CTA on the zeroed slot, any length.  In front of a packing kernel
+// (kTensors > 0): every CTA leaves its own maximum in out[blockIdx.x] for that kernel to combine, so that no slot
+// has to be zeroed first, launched by launch_dependent(); kTensors tensors share the launch, each with its own CTAs.
+//
+// Bound: HBM.  The second form has four 32-byte loads a thread on their way and four CTAs an SM.  kKeep: of a tensor
+// that L2 does not hold it is asked to keep the last kKeptBytes, which the packing kernel reads first (and lets go).
+// amax + pack, us, with 16-byte loads and eight CTAs an SM, without and with the hint: [27280, 3072] 62.4, 61.5, 60.1;
+// 15000 rows 35.8, 34.8, 35.2; 4096 rows 12.1, 11.9, 11.7, but 35.1 instead of 34.6 with the GEMM behind it, whose operands
+// and output want the room.
+constexpr int64_t kKeptBytes = 60 << 20;
+constexpr int64_t kKeepFrom = 126 << 20;      // the size of L2
+
 template <int kTensors>
 struct AmaxArgs {
   const uint4* x[kTensors];
-  int64_t n_vec[kTensors];
+  int64_t n_vec[kTensors];        // 16-byte pieces
   unsigned first[kTensors + 1];   // CTAs of tensor i: first[i] up to first[i + 1]
-  unsigned* zero;                 // kPartial, nullable: words that the next kernel wants zeroed
+  unsigned wide;                  // bit i: tensor i starts on a 32-byte boundary
+  unsigned* zero;                 // nullable: words that the next kernel wants zeroed
   int n_zero;
 };
 
-template <bool kPartial, int kTensors>
-__global__ void __launch_bounds__(kThreads) amax_bf16_kernel(const AmaxArgs<kTensors> p,
-                                                             const __nv_bfloat16* tail, int n_tail,
-                                                             unsigned* out) {
-  __nv_bfloat162 m2[4];
+__device__ __forceinline__ uint32_t max_abs_u4(uint32_t m, const uint4& v) {
+  return bf16x2_max_abs(bf16x2_max_abs(bf16x2_max_abs(bf16x2_max_abs(m, v.x), v.y), v.z), v.w);
+}
+// The CTA's maximum, on thread 0.  Non-negative floats order like their bit patterns.
+__device__ __forceinline__ unsigned cta_max(float a) {
+  __shared__ unsigned warp_max[kThreads / 32];
+  unsigned bits = __reduce_max_sync(0xffffffffu, __float_as_uint(a));
+  if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = bits;
+  __syncthreads();
+  if (threadIdx.x < 32) bits = __reduce_max_sync(0xffffffffu, threadIdx.x < kThreads / 32 ? warp_max[threadIdx.x] : 0u);
+  return bits;
+}
+
+__global__ void __launch_bounds__(kThreads) amax_slot_kernel(const uint4* x, int64_t n_vec, const __nv_bfloat16* tail,
+                                                             int n_tail, unsigned* out) {
+  uint32_t m[4] = {0u, 0u, 0u, 0u};
+  const int64_t stride = (int64_t)gridDim.x * kThreads;
+  int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  // four independent 16-byte loads in flight per thread
+  for (; i + 3 * stride < n_vec; i += 4 * stride) {
+    uint4 v[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) m2[j] = __nv_bfloat162(__float2bfloat16(0.f), __float2bfloat16(0.f));
+    for (int j = 0; j < 4; ++j) v[j] = load_u32x4(x + i + j * stride);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) m[j] = max_abs_u4(m[j], v[j]);
+  }
+  for (; i < n_vec; i += stride) m[0] = max_abs_u4(m[0], load_u32x4(x + i));
+  const uint32_t h = bf16x2_max_abs(bf16x2_max_abs(bf16x2_max_abs(m[0], m[1]), m[2]), m[3]);
+  float a = fmaxf(bf16lo_to_f32(h), bf16hi_to_f32(h));
+  if (blockIdx.x == 0 && threadIdx.x < n_tail) a = fmaxf(a, fabsf(__bfloat162float(tail[threadIdx.x])));
+  const unsigned b = cta_max(a);
+  if (threadIdx.x == 0 && b != 0u) atomicMax(out, b);
+}
+
+template <int kTensors, bool kKeep>
+__global__ void __launch_bounds__(kThreads) amax_bf16_kernel(const AmaxArgs<kTensors> p, unsigned* out) {
   const uint4* x = p.x[0];
   int64_t n_vec = p.n_vec[0];
-  unsigned first = p.first[0], end = p.first[1];
+  unsigned first = p.first[0], end = p.first[1], wide = p.wide & 1u;
 #pragma unroll
   for (int k = 1; k < kTensors; ++k) {
     if (blockIdx.x >= p.first[k]) {
@@ -55,51 +95,50 @@ __global__ void __launch_bounds__(kThreads) amax_bf16_kernel(const AmaxArgs<kTen
       n_vec = p.n_vec[k];
       first = p.first[k];
       end = p.first[k + 1];
+      wide = p.wide >> k & 1u;
     }
   }
-  const unsigned cta = blockIdx.x - first, ctas = end - first;
-  if (kPartial) {
-    grid_dependency_wait();
-    if (blockIdx.x == 0)
-      for (int i = threadIdx.x; i < p.n_zero; i += kThreads) p.zero[i] = 0u;
-  }
-  const int64_t stride = (int64_t)ctas * kThreads;
-  int64_t i = (int64_t)cta * kThreads + threadIdx.x;
-  // four independent 16-byte loads in flight per thread
-  for (; i + 3 * stride < n_vec; i += 4 * stride) {
-    uint4 v[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = load_u32x4(x + i + j * stride);
+  uint64_t keep, drop;
+  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(keep));
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(drop));
+  grid_dependency_wait();
+  if (blockIdx.x == 0)
+    for (int i = threadIdx.x; i < p.n_zero; i += kThreads) p.zero[i] = 0u;
+  const int64_t n = n_vec / 2, stride = (int64_t)(end - first) * kThreads, kept = n - kKeptBytes / 32;
+  uint32_t m[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+  for (int64_t i = (int64_t)(blockIdx.x - first) * kThreads + threadIdx.x; i < n; i += 4 * stride) {
+    uint32_t v[4][8];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v[j]);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) m2[k] = __hmax2(m2[k], __habs2(h[k]));
+      const int64_t at = i + j * stride;
+      const uint4* src = x + 2 * (at < n ? at : i);      // past the end: the first piece again
+      if (!wide) {
+        const uint4 a = load_u32x4(src), b = load_u32x4(src + 1);
+        v[j][0] = a.x; v[j][1] = a.y; v[j][2] = a.z; v[j][3] = a.w;
+        v[j][4] = b.x; v[j][5] = b.y; v[j][6] = b.z; v[j][7] = b.w;
+      } else if (kKeep) {
+        const uint64_t policy = at >= kept ? keep : drop;
+        asm volatile("ld.global.L1::no_allocate.L2::cache_hint.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8], %9;"
+                     : "=r"(v[j][0]), "=r"(v[j][1]), "=r"(v[j][2]), "=r"(v[j][3]), "=r"(v[j][4]), "=r"(v[j][5]),
+                       "=r"(v[j][6]), "=r"(v[j][7])
+                     : "l"(src), "l"(policy));
+      } else {
+        asm volatile("ld.global.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(v[j][0]), "=r"(v[j][1]), "=r"(v[j][2]), "=r"(v[j][3]), "=r"(v[j][4]), "=r"(v[j][5]),
+                       "=r"(v[j][6]), "=r"(v[j][7])
+                     : "l"(src));
+      }
     }
-  }
-  for (; i < n_vec; i += stride) {
-    uint4 v = load_u32x4(x + i);
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) m2[k] = __hmax2(m2[k], __habs2(h[k]));
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int k = 0; k < 8; ++k) m[k] = bf16x2_max_abs(m[k], v[j][k]);
   }
-  __nv_bfloat162 m = __hmax2(__hmax2(m2[0], m2[1]), __hmax2(m2[2], m2[3]));
-  float a = fmaxf(__bfloat162float(m.x), __bfloat162float(m.y));
-  if (blockIdx.x == 0 && threadIdx.x < n_tail)
-    a = fmaxf(a, fabsf(__bfloat162float(tail[threadIdx.x])));
-  // non-negative floats order like their bit patterns
-  unsigned bits = __reduce_max_sync(0xffffffffu, __float_as_uint(a));
-  __shared__ unsigned warp_max[kThreads / 32];
-  if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = bits;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    unsigned b = threadIdx.x < kThreads / 32 ? warp_max[threadIdx.x] : 0u;
-    b = __reduce_max_sync(0xffffffffu, b);
-    if (threadIdx.x == 0) {
-      if (kPartial) out[blockIdx.x] = b;
-      else if (b != 0u) atomicMax(out, b);
-    }
-  }
+  if ((n_vec & 1) && blockIdx.x == first && threadIdx.x == 0) m[0] = max_abs_u4(m[0], load_u32x4(x + n_vec - 1));
+#pragma unroll
+  for (int k = 1; k < 8; ++k) m[0] = bf16x2_max_abs(m[0], m[k]);
+  const unsigned b = cta_max(fmaxf(bf16lo_to_f32(m[0]), bf16hi_to_f32(m[0])));
+  if (threadIdx.x == 0) out[blockIdx.x] = b;
 }
 
 // ------------------------------------------------------------ quantize ----
@@ -655,6 +694,12 @@ unsigned amax_grid(int64_t n_vec) {
   return (unsigned)(want < 1 ? 1 : (want > most ? most : want));
 }
 
+// CTAs of amax_bf16_kernel: a thread of theirs has 32 bytes of a small tensor, and four fit an SM.
+int64_t wanted_ctas(int64_t n_vec) { return std::max<int64_t>((n_vec / 2 + kThreads - 1) / kThreads, 1); }
+int64_t most_ctas() { return std::min<int64_t>(4 * (int64_t)sm_count(), NVFP4_AMAX_PARTIALS); }
+unsigned partial_grid(int64_t n_vec) { return (unsigned)std::min(wanted_ctas(n_vec), most_ctas()); }
+unsigned wide_bit(const void* x) { return (reinterpret_cast<uintptr_t>(x) & 31u) == 0; }
+
 // Launches the resident form if the tensor fits; *done says whether.
 int launch_resident(const void* x, int64_t rows, int64_t cols, float* amax, uint8_t* packed, uint8_t* sf_lin,
                     uint8_t* sf_swz, float* gscale, float* partials, cudaStream_t st, bool* done) {
@@ -721,19 +766,21 @@ int launch_small(const void* x, int64_t rows, int64_t cols, float* amax, uint8_t
 // The maxima of up to three tensors in one launch, each tensor's CTAs in proportion to its size: `job.first` and
 // `job.count` say which of the partial maxima are a tensor's.
 int launch_amax_partials(AmaxJob (&jobs)[3], int n_jobs, float* partials, unsigned* zero, int n_zero, void* stream) {
+  const int64_t most = most_ctas();
   int64_t want = 0;
-  for (int i = 0; i < n_jobs; ++i) want += amax_grid(jobs[i].n / 8);
+  for (int i = 0; i < n_jobs; ++i) want += wanted_ctas(jobs[i].n / 8);
   AmaxArgs<3> a{};
   unsigned next = 0;
   for (int i = 0; i < 3; ++i) {
     a.first[i] = next;
     if (i >= n_jobs) continue;
     const int64_t n_vec = jobs[i].n / 8;
-    int64_t ctas = amax_grid(n_vec);
+    int64_t ctas = wanted_ctas(n_vec);
     // rounded down, and three single CTAs at most on top of that: no more than there is room for
-    if (want > NVFP4_AMAX_PARTIALS) ctas = ctas * (NVFP4_AMAX_PARTIALS - 3) / want + 1;
+    if (want > most) ctas = ctas * (most - 3) / want + 1;
     a.x[i] = static_cast<const uint4*>(jobs[i].x);
     a.n_vec[i] = n_vec;
+    a.wide |= wide_bit(jobs[i].x) << i;
     jobs[i].first = (int)next;
     jobs[i].count = (int)ctas;
     next += (unsigned)ctas;
@@ -741,8 +788,7 @@ int launch_amax_partials(AmaxJob (&jobs)[3], int n_jobs, float* partials, unsign
   a.first[3] = next;
   a.zero = zero;
   a.n_zero = n_zero;
-  return launch_dependent(amax_bf16_kernel<true, 3>, dim3(next), kThreads, 0, 1,
-                          reinterpret_cast<cudaStream_t>(stream), a, (const __nv_bfloat16*)nullptr, 0,
+  return launch_dependent(amax_bf16_kernel<3, false>, dim3(next), kThreads, 0, 1, reinterpret_cast<cudaStream_t>(stream), a,
                           reinterpret_cast<unsigned*>(partials));
 }
 
@@ -764,10 +810,9 @@ int nvfp4_amax_bf16(const void* x, int64_t n, float* amax_dev, void* stream) {
   if (!aligned16(x)) return NVFP4_ERR_BAD_ALIGN;
   const int64_t n_vec = n / 8;
   const int n_tail = (int)(n - n_vec * 8);
-  const unsigned grid = amax_grid(n_vec);
-  const AmaxArgs<1> a{{reinterpret_cast<const uint4*>(x)}, {n_vec}, {0u, grid}, nullptr, 0};
-  amax_bf16_kernel<false, 1><<<grid, kThreads, 0, st>>>(
-      a, reinterpret_cast<const __nv_bfloat16*>(x) + n_vec * 8, n_tail, reinterpret_cast<unsigned*>(amax_dev));
+  amax_slot_kernel<<<amax_grid(n_vec), kThreads, 0, st>>>(
+      reinterpret_cast<const uint4*>(x), n_vec, reinterpret_cast<const __nv_bfloat16*>(x) + n_vec * 8, n_tail,
+      reinterpret_cast<unsigned*>(amax_dev));
   return launch_status();
 }
 
@@ -808,10 +853,12 @@ int nvfp4_amax_quantize_bf16(const void* x, int64_t rows, int64_t cols, float* a
   int threads;
   if (n_blocks > 0 && partials && rows_form(rows, cols, scales_swizzled != nullptr, &threads)) {
     const int64_t n_vec = n_blocks * 2;
-    const unsigned grid = amax_grid(n_vec);
-    const AmaxArgs<1> first{{reinterpret_cast<const uint4*>(x)}, {n_vec}, {0u, grid}, nullptr, 0};
-    rc = launch_dependent(amax_bf16_kernel<true, 1>, dim3(grid), kThreads, 0, 1, st, first,
-                          (const __nv_bfloat16*)nullptr, 0, reinterpret_cast<unsigned*>(partials));
+    const unsigned grid = partial_grid(n_vec);
+    const AmaxArgs<1> first{{reinterpret_cast<const uint4*>(x)}, {n_vec}, {0u, grid}, wide_bit(x), nullptr, 0};
+    rc = n_blocks * 32 > kKeepFrom ? launch_dependent(amax_bf16_kernel<1, true>, dim3(grid), kThreads, 0, 1, st, first,
+                                                      reinterpret_cast<unsigned*>(partials))
+                                   : launch_dependent(amax_bf16_kernel<1, false>, dim3(grid), kThreads, 0, 1, st, first,
+                                                      reinterpret_cast<unsigned*>(partials));
     if (rc != NVFP4_OK) return rc;
     PackArgs a{};
     a.x = reinterpret_cast<const uint4*>(x);
