@@ -1,6 +1,6 @@
 // The Python layer's frequent calls in one native step each: argument checks, allocations, stream and
 // library call.  Through ctypes these cost 11 to 38 us a call (a linear 27, a quantizer 21 to 28, norm + quantize
-// 30 to 38), more than the kernels of a few thousand rows take.
+// 30 to 38, the backward of a linear 45), more than the kernels of a few thousand rows take.
 //
 // Every function returns None for what is not the plain case (other types, devices, layouts or alignments,
 // tensor subclasses, an active dispatch mode, an empty tensor): the Python code that called it then does what it
@@ -111,6 +111,43 @@ std::optional<Packed> quantize(const Tensor& x, bool linear_scales, bool swizzle
   return Packed(rows, cols, data, scales, swz, amax, gscale);
 }
 
+// The same with its maximum known (amax), and into the given buffers (data, scales, swizzled scales, amax, tensor scale, row
+// statistics, partial maxima).
+std::optional<Packed> quantize_into(const Tensor& x, bool linear_scales, bool swizzled_scales, const Maybe& amax_,
+                                    const std::optional<std::vector<Maybe>>& out) {
+  if (!plain(x) || modes() || x.scalar_type() != at::kBFloat16 || x.dim() < 1 || x.numel() == 0 ||
+      x.size(-1) % 16 != 0 || !x.is_contiguous())
+    return {};
+  if (amax_ && (!plain(*amax_) || amax_->scalar_type() != at::kFloat || amax_->numel() != 1 ||
+                amax_->device() != x.device()))
+    return {};
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int64_t cols = x.size(-1), rows = x.numel() / cols;
+  Tensor data, gscale, amax, partials;
+  Maybe scales, swz;
+  if (out) {
+    const auto& o = *out;
+    data = *o[0]; swz = o[2]; gscale = *o[4]; partials = *o[6];
+    if (linear_scales) scales = o[1];
+    amax = amax_ ? *amax_ : *o[3];
+  } else {
+    amax = amax_ ? *amax_ : empty({1}, at::kFloat, x);
+    gscale = empty({1}, at::kFloat, x);
+    data = empty({rows * cols / 2}, at::kByte, x);
+    if (linear_scales) scales = empty({rows * cols / 16}, at::kByte, x);
+    if (swizzled_scales) swz = empty({nvfp4_swizzled_scale_bytes(rows, cols)}, at::kByte, x);
+    if (!amax_) partials = empty({NVFP4_AMAX_PARTIALS}, at::kFloat, x);
+  }
+  if (amax_)
+    check(nvfp4_quantize_bf16(x.data_ptr(), rows, cols, f32(amax), u8(data), u8(scales), u8(swz), f32(gscale), stream_of(x)),
+          "[tensor] quantize");
+  else
+    check(nvfp4_amax_quantize_bf16(x.data_ptr(), rows, cols, f32(amax), u8(data), u8(scales), u8(swz), f32(gscale),
+                                   f32(partials), stream_of(x)),
+          "[tensor] amax+quantize");
+  return Packed(rows, cols, data, scales, swz, amax, gscale);
+}
+
 // The same of norm(x) * weight + bias, modulated; into the given buffers (data, scales, swizzled scales, amax,
 // tensor scale, row statistics, partial maxima) or new ones.
 std::optional<Packed> norm_quantize(const Tensor& x, const Maybe& weight, const Maybe& bias, const Maybe& scale,
@@ -183,6 +220,70 @@ Maybe gemm(const Tensor& a, const Tensor& b, const Tensor& a_scales, const Tenso
   return d;
 }
 
+// The gradients that are wanted of y = x @ w.T + b: dx, dw, db
+std::optional<std::vector<Maybe>> linear_backward(const Tensor& dy, const Tensor& x, const Tensor& w, bool want_dx,
+                                                  bool want_dw, bool want_db) {
+  if (!plain(dy) || !plain(x) || !plain(w) || modes() || (!want_dx && !want_dw) || dy.dim() < 1 || x.dim() < 1 ||
+      w.dim() != 2 || !status_of(dy))
+    return {};
+  const int64_t n = w.size(0), k = w.size(1);
+  if (n == 0 || k == 0 || dy.numel() == 0 || dy.size(-1) != n || x.size(-1) != k) return {};
+  const int64_t m = dy.numel() / n;
+  if (x.numel() != m * k || n % 32 != 0 || k % 8 != 0) return {};
+  for (const Tensor* t : {&dy, &x, &w})
+    if (t->scalar_type() != at::kBFloat16 || t->device() != dy.device() || !t->is_contiguous() || !aligned(*t)) return {};
+  const c10::cuda::CUDAGuard guard(dy.device());
+  Maybe dx, dw, db;
+  if (want_dx) dx = empty(x.sizes(), at::kBFloat16, dy);
+  if (want_dw) dw = empty({n, k}, at::kBFloat16, dy);
+  if (want_db) db = empty({n}, at::kBFloat16, dy);
+  const Tensor ws = empty({nvfp4_linear_backward_workspace_bytes(m, n, k)}, at::kByte, dy);
+  check(nvfp4_linear_backward_bias_bf16(dy.data_ptr(), want_dw ? x.data_ptr() : nullptr, want_dx ? w.data_ptr() : nullptr,
+                                        nullptr, m, n, k, ptr(dx), ptr(dw), ptr(db), ws.data_ptr(), status_of(dy),
+                                        stream_of(dy)),
+        "[linear] backward");
+  return std::vector<Maybe>{dx, dw, db};
+}
+
+// RMSNorm across heads of q and k and the rotary embedding of [L, 3 * heads * head_dim]: q, k
+std::optional<std::tuple<Tensor, Tensor>> qk_norm_rope(const Tensor& qkv, int64_t heads, int64_t head_dim,
+                                                       const Maybe& gain_q, const Maybe& gain_k, double eps,
+                                                       const Tensor& cos_sin) {
+  if (!plain(qkv) || !plain(cos_sin) || modes() || heads <= 0 || head_dim <= 0 || heads > 16384 || head_dim > 16384 ||
+      qkv.dim() != 2 || qkv.scalar_type() != at::kBFloat16 || !qkv.is_contiguous() ||
+      qkv.get_device() != c10::cuda::current_device() || !status_of(qkv))
+    return {};
+  const int64_t L = qkv.size(0), dim = heads * head_dim;
+  if (qkv.size(1) != 3 * dim || cos_sin.dim() != 3 || cos_sin.size(0) != L || cos_sin.size(1) != head_dim / 2 ||
+      cos_sin.size(2) != 2 || !fits(cos_sin, at::kFloat, cos_sin.numel(), qkv) || !fits(gain_q, at::kFloat, dim, qkv) ||
+      !fits(gain_k, at::kFloat, dim, qkv))
+    return {};
+  Tensor q = empty({L, heads, head_dim}, at::kBFloat16, qkv), k = empty({L, heads, head_dim}, at::kBFloat16, qkv);
+  const char* base = static_cast<const char*>(qkv.data_ptr());
+  check(nvfp4_qk_norm_rope_bf16(base, base + 2 * dim, nullptr, 3 * dim, L, (int)heads, (int)head_dim,
+                                static_cast<float*>(ptr(gain_q)), static_cast<float*>(ptr(gain_k)), (float)eps,
+                                f32(cos_sin), q.data_ptr(), k.data_ptr(), nullptr, dim, head_dim, status_of(qkv),
+                                stream_of(qkv)),
+        "qk_norm_rope");
+  return std::make_tuple(q, k);
+}
+
+// RMSNorm of the rows of [L, heads * head_dim], which may lie apart
+Maybe rms_norm(const Tensor& x, int64_t heads, int64_t head_dim, const Maybe& gain, double eps) {
+  if (!plain(x) || modes() || heads <= 0 || head_dim <= 0 || heads > 16384 || head_dim > 16384 || x.dim() != 2 ||
+      x.scalar_type() != at::kBFloat16 || x.get_device() != c10::cuda::current_device() || !status_of(x))
+    return {};
+  const int64_t L = x.size(0), dim = heads * head_dim;
+  if (x.size(1) != dim || x.stride(1) != 1 || x.stride(0) % 8 != 0 || !aligned(x) || !fits(gain, at::kFloat, dim, x))
+    return {};
+  Tensor out = empty({L, heads, head_dim}, at::kBFloat16, x);
+  check(nvfp4_qk_norm_rope_bf16(x.data_ptr(), nullptr, nullptr, x.stride(0), L, (int)heads, (int)head_dim,
+                                static_cast<float*>(ptr(gain)), nullptr, (float)eps, nullptr, out.data_ptr(), nullptr,
+                                nullptr, dim, head_dim, status_of(x), stream_of(x)),
+        "rms_norm");
+  return out;
+}
+
 Maybe attention(const Tensor& q, const Tensor& k, const Tensor& v, const Maybe& amax, const Maybe& out) {
   if (!plain(q) || !plain(k) || !plain(v) || modes() || out || q.dim() != 3 || k.dim() != 3 || v.dim() != 3 ||
       !status_of(q) || q.get_device() != c10::cuda::current_device())
@@ -211,6 +312,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("set_status", &set_status);
   m.def("linear", torch::wrap_pybind_function_no_gil(linear));
   m.def("quantize", torch::wrap_pybind_function_no_gil(quantize));
+  m.def("quantize_into", torch::wrap_pybind_function_no_gil(quantize_into));
+  m.def("linear_backward", torch::wrap_pybind_function_no_gil(linear_backward));
+  m.def("qk_norm_rope", torch::wrap_pybind_function_no_gil(qk_norm_rope));
+  m.def("rms_norm", torch::wrap_pybind_function_no_gil(rms_norm));
   m.def("norm_quantize", torch::wrap_pybind_function_no_gil(norm_quantize));
   m.def("dequantize", torch::wrap_pybind_function_no_gil(dequantize));
   m.def("gemm", torch::wrap_pybind_function_no_gil(gemm));

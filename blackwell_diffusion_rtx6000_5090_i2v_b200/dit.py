@@ -259,6 +259,11 @@ def qk_norm_rope(qkv: torch.Tensor, heads: int, head_dim: int, gain_q: Optional[
     below).  Returns ``(q, k, v)`` as ``[L, heads, head_dim]`` tensors -- v is a view of
     ``qkv`` -- or, with ``packed``, one ``[L, heads, 3*head_dim]`` tensor holding q | k | v per
     head, the layout the head/sequence exchange sends."""
+    if not packed and qkv.is_cuda:
+        N.status_word(qkv.device)
+        made = N.host.qk_norm_rope(qkv, heads, head_dim, gain_q, gain_k, eps, cos_sin)
+        if made is not None:
+            return (*made, qkv[:, 2 * heads * head_dim:].view(qkv.shape[0], heads, head_dim))
     L, three_dim = qkv.shape
     dim = heads * head_dim
     if three_dim != 3 * dim or qkv.dtype != torch.bfloat16 or not qkv.is_contiguous():
@@ -291,6 +296,11 @@ def rms_norm_fused(x: torch.Tensor, heads: int, head_dim: int, gain: Optional[to
     """RMSNorm over the last axis of a bf16 ``[L, heads*head_dim]`` tensor (rows may be a strided
     view, e.g. a column block of a wider matrix) with the same kernel (no rotation); returns a
     contiguous ``[L, heads, head_dim]``."""
+    if x.is_cuda:
+        N.status_word(x.device)
+        out = N.host.rms_norm(x, heads, head_dim, gain, eps)
+        if out is not None:
+            return out
     L, dim = x.shape
     if dim != heads * head_dim or x.dtype != torch.bfloat16 or x.stride(1) != 1 or \
             x.stride(0) % 8 != 0 or x.data_ptr() % 16 != 0:
@@ -476,7 +486,7 @@ class WanBlock:
         kv = (self.cross_kv.nvfp4(_record_amax(self.cross_kv, FP4Tensor.from_bfloat16(
             ctx, linear_scales=_want_linear_scales())))
               if mode == "nvfp4" else self.cross_kv.dequant(ctx, reorder=mode == "dequant_reordered"))
-        return self._split_text_kv(kv)
+        return self._split_text_kv(kv, fused=mode == "nvfp4")
 
     def _split_text_kv(self, kv: torch.Tensor, fused: bool = False):
         """``[C, 2*dim]`` projection of the text context -> normalised k and v, ``[C, heads, D]``.

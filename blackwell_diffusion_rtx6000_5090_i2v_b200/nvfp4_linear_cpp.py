@@ -246,6 +246,15 @@ def backward(grad_output: torch.Tensor, input: torch.Tensor, weight: torch.Tenso
     GEMMs run through the same FP4 path.  The reference's weight-gradient call
     passes operands whose inner dimensions disagree (:187); the product meant
     there, ``grad_output.T @ input``, is what is computed here."""
+    if grad_output.is_cuda:
+        N.status_word(grad_output.device)
+    # a backward that is itself differentiated keeps the bias gradient's sum as an operation of torch
+    own_sum = needs_bias_grad and not (grad_output.requires_grad and torch.is_grad_enabled())
+    made = N.host.linear_backward(grad_output, input, weight, needs_input_grad, needs_weight_grad, own_sum)
+    if made is not None:
+        if needs_bias_grad and not own_sum:
+            made[2] = grad_output.reshape(-1, weight.size(0)).sum(0)
+        return made
     in_features = input.size(-1)
     out_features = weight.size(0)
     x2 = input.reshape(-1, in_features)
@@ -271,7 +280,7 @@ def backward(grad_output: torch.Tensor, input: torch.Tensor, weight: torch.Tenso
         with N.device_guard(dev):
             ws = torch.empty(N.lib.nvfp4_linear_backward_workspace_bytes(m, out_features, k),
                              dtype=torch.uint8, device=dev)
-            if needs_bias_grad:
+            if own_sum:
                 grad_bias = torch.empty(out_features, dtype=torch.bfloat16, device=dev)
             # the maximum of the weight is taken here, not from the forward's packed copy: a write
             # through weight.data would leave that one behind

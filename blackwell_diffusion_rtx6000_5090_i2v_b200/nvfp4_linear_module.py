@@ -28,9 +28,9 @@ class NVFP4LinearFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_output: Tensor):
         input, weight, scale_input, scale_weight = ctx.saved_tensors
-        scale_grad_output = torch.ones_like(scale_input)
+        # (a scale of the gradient is reserved and ignored, like the others)
         grad_input, grad_weight, grad_bias = nvfp4_linear_cpp.backward(
-            grad_output, input, weight, scale_input, scale_weight, scale_grad_output,
+            grad_output, input, weight, scale_input, scale_weight, scale_input,
             ctx.needs_input_grad[0], ctx.needs_input_grad[1], ctx.needs_bias_grad)
         return grad_input, grad_weight, grad_bias, None, None
 
