@@ -213,6 +213,19 @@ __device__ __forceinline__ uint4 load_u32x4_once(const void* p) {
   return v;
 }
 
+// The maximum of this thread's share of a CTA's partial maxima (bits of non-negative floats): four at a time, all asked for
+// before the first is needed.  One behind the other they were four trips to L2 ahead of a packing kernel's first block.
+__device__ __forceinline__ unsigned max_of_partials(const unsigned* partial, int n) {
+  unsigned m = 0u;
+  for (int i = threadIdx.x; i < n; i += 4 * blockDim.x) {
+    unsigned v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = load_u32(partial + min(i + j * (int)blockDim.x, n - 1));
+    m = max(max(m, max(v[0], v[1])), max(v[2], v[3]));
+  }
+  return m;
+}
+
 // 32 bytes of x that are read once: one 256-bit load where the address allows, else two of 128.
 __device__ __forceinline__ void load_block_once(const uint4* src, bool wide, uint32_t (&x)[8]) {
   if (wide) {

@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(kPackThreads, 4) pack_rows_kernel(const PackAr
   float amax_g;
   if (p.partial) {
     unsigned m = 0u;
-    for (int i = threadIdx.x; i < p.n_partial; i += blockDim.x) m = max(m, load_u32(p.partial + i));
+    m = max_of_partials(p.partial, p.n_partial);
     m = __reduce_max_sync(0xffffffffu, m);
     if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = m;
     __syncthreads();

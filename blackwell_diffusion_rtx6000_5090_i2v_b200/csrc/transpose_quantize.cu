@@ -92,8 +92,7 @@ __global__ void __launch_bounds__(kThreads, kJobs == 1 ? 4 : 3) quantize_transpo
     if (kJobs > 1 && p.first[k] == p.first[k + 1]) continue;
     float amax_g;
     if (kJobs > 1 && q.n_partial > 0) {
-      unsigned m = 0u;
-      for (int i = threadIdx.x; i < q.n_partial; i += kThreads) m = max(m, load_u32(p.partial + q.first_partial + i));
+      unsigned m = max_of_partials(p.partial + q.first_partial, q.n_partial);
       m = __reduce_max_sync(0xffffffffu, m);
       if (lane == 0) warp_max[threadIdx.x >> 5] = m;
       __syncthreads();
