@@ -132,7 +132,7 @@ int nvfp4_linear_bf16(const void* x_bf16, int64_t M, int64_t K, const uint8_t* w
   uint8_t* scales = packed + (M * K / 2 + 255) / 256 * 256;
   float* amax = reinterpret_cast<float*>(scales + sf_swizzled_bytes(M, K));
   float* partials = amax + 64;
-  const int rc = nvfp4_amax_quantize_bf16(x_bf16, M, K, amax, packed, nullptr, scales, amax + 1, partials, stream);
+  const int rc = amax_quantize(x_bf16, M, K, amax, packed, nullptr, scales, amax + 1, partials, false, stream);
   if (rc != NVFP4_OK) return rc;
   return nvfp4_gemm(packed, w_packed, scales, w_scales_swizzled, amax + 1, w_global_scale_dev, M, N, K, 1.0f,
                     residual_bf16 ? 1.0f : 0.0f, residual_bf16, bias_bf16, gate_f32, act, y_bf16, nullptr,

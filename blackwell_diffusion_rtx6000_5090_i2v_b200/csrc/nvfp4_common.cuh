@@ -277,6 +277,10 @@ int check_device_sm100();                 // NVFP4_OK or NVFP4_ERR_UNSUPPORTED_A
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 int sm_count();                           // SMs of the current device (cached per device)
 
+// nvfp4_amax_quantize_bf16, and whether nothing is known to follow it on the stream.
+int amax_quantize(const void* x, int64_t rows, int64_t cols, float* amax_dev, uint8_t* packed, uint8_t* scales_linear,
+                  uint8_t* scales_swizzled, float* global_scale_dev, float* partials, bool alone, void* stream);
+
 // One tensor of launch_amax_partials(): n a multiple of 8, 16-byte aligned.  `first`, `count` are filled in.
 struct AmaxJob {
   const void* x;

@@ -219,6 +219,7 @@ quantize_bf16_kernel(const uint4* __restrict__ x, uint32_t n_blocks, uint32_t kb
 // before); the pad rows and K-blocks of the swizzled layout are written as zeros here instead of
 // by a memset ahead of the kernel.
 constexpr int kPackThreads = 192;
+constexpr int kPackWide = 320;       // the wider of the two CTAs
 constexpr int kRows = 4;
 
 struct PackArgs {
@@ -239,9 +240,12 @@ struct PackArgs {
   int word_swz;               // sf_swz starts on a 4-byte boundary
 };
 
-__global__ void __launch_bounds__(kPackThreads, 4) pack_rows_kernel(const PackArgs p) {
+// kMax: most threads of a CTA, kPackThreads or kPackWide.
+constexpr int pack_ctas(int max) { return max == kPackThreads ? 4 : 3; }
+template <int kMax>
+__global__ void __launch_bounds__(kMax, pack_ctas(kMax)) pack_rows_kernel(const PackArgs p) {
   __shared__ float enc_tab[128];
-  __shared__ unsigned warp_max[kPackThreads / 32];
+  __shared__ unsigned warp_max[kMax / 32];
   const int u = threadIdx.x;
   const bool live = u < p.units;
   const bool in_layout = u < (int)p.k_atoms * 4;
@@ -612,17 +616,16 @@ int zero_swizzle_padding(uint8_t* swz, int64_t rows, int64_t cols, cudaStream_t 
   return NVFP4_OK;
 }
 
-// The rows form takes rows that one CTA of kPackThreads spans with at least three quarters of its threads
-// (1152 to 3072 columns), and enough of them for kRows at a time: [27280, 3072] amax + pack 77.8 us flat with
-// its two memsets, 71.7 rows.  Much wider rows are better off in the flat form, whose CTAs read one contiguous
-// piece each ([27280, 14336] 291 us, 302-350 with five CTAs side by side on a row).  Where the line should
-// lie in between is open: CTAs of 320 threads would take 4096 and 5120 columns in 98 and 125 us instead of 104
-// and 127 ([32760, .], 16 instead of 21 and 18 instead of 23 at 4095 rows), the memsets among it, but 3072
-// in 77 instead of 74.
+// The rows form takes rows that one CTA spans with at least three quarters of its threads (1152 to 5120 columns), and
+// enough of them for kRows at a time: [27280, 3072] amax + pack 77.8 us flat with its two memsets, 60.1 rows.  Rows of more
+// than 3072 columns have a wider CTA of their own kernel, since three of 320 threads an SM instead of four of 192 cost the
+// narrower ones ([32760, 3072] 77 instead of 74): through the public call flat and rows [15000, 4096] 55.9 and 46.8, [32760,
+// 4096] 108 and 97, [16000, 5120] 70.2 and 58.7.  Much wider rows are better off in the flat form, whose CTAs read one
+// contiguous piece each ([27280, 14336] 291 us, 302-350 with five CTAs side by side on a row).
 bool rows_form(int64_t rows, int64_t cols, bool swz, int* threads) {
   const int64_t units = swz ? sf_k_atoms(cols) * 4 : cols / kBlock;
   *threads = (int)((units + 31) / 32 * 32);
-  return rows >= 32 && units <= kPackThreads && *threads >= 96 && cols / kBlock * 4 >= (int64_t)*threads * 3;
+  return rows >= 32 && units <= kPackWide && *threads >= 96 && cols / kBlock * 4 >= (int64_t)*threads * 3;
 }
 
 int check_quantize(const void* x, int64_t rows, int64_t cols, const uint8_t* packed) {
@@ -637,13 +640,17 @@ int check_quantize(const void* x, int64_t rows, int64_t cols, const uint8_t* pac
   return check_device_sm100();
 }
 
-int launch_rows(const PackArgs& a, int threads, cudaStream_t st) {
+template <int kMax>
+int launch_rows_of(const PackArgs& a, int threads, cudaStream_t st) {
   const int64_t all_rows = a.sf_swz ? sf_row_tiles(a.rows) * 128 : a.rows;
   const int64_t groups = (all_rows + kRows - 1) / kRows;
-  // CTAs per SM by the launch bound's registers: 4 of kPackThreads, more of narrower ones
-  const int64_t resident = (int64_t)sm_count() * (4 * kPackThreads / threads);
-  return launch_dependent(pack_rows_kernel, dim3((unsigned)(groups < resident ? groups : resident)),
+  // CTAs per SM by the launch bound's registers, more of narrower ones
+  const int64_t resident = (int64_t)sm_count() * (pack_ctas(kMax) * kMax / threads);
+  return launch_dependent(pack_rows_kernel<kMax>, dim3((unsigned)(groups < resident ? groups : resident)),
                           (unsigned)threads, 0, 1, st, a);
+}
+int launch_rows(const PackArgs& a, int threads, cudaStream_t st) {
+  return threads <= kPackThreads ? launch_rows_of<kPackThreads>(a, threads, st) : launch_rows_of<kPackWide>(a, threads, st);
 }
 
 int quantize_impl(const void* x, int64_t rows, int64_t cols, const float* amax_dev, float amax_val,
@@ -792,6 +799,76 @@ int launch_amax_partials(AmaxJob (&jobs)[3], int n_jobs, float* partials, unsign
                           reinterpret_cast<unsigned*>(partials));
 }
 
+// Wide rows in up to this many blocks are packed in one launch where no GEMM follows (amax_quantize).
+constexpr int64_t kAloneBlocks = 480 << 10;
+
+// `alone`: nothing is known to follow on the stream.
+int amax_quantize(const void* x, int64_t rows, int64_t cols, float* amax_dev, uint8_t* packed, uint8_t* scales_linear,
+                  uint8_t* scales_swizzled, float* global_scale_dev, float* partials, bool alone, void* stream) {
+  int rc = check_quantize(x, rows, cols, packed);
+  if (rc != NVFP4_OK) return rc;
+  if (!amax_dev) return NVFP4_ERR_BAD_ARG;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const int64_t n_blocks = rows * cols / kBlock;
+  const bool small_fits = n_blocks > 0 && n_blocks <= kSmallMax && aligned16(scales_swizzled) &&
+                          (!scales_swizzled || sf_swizzled_bytes(rows, cols) <= kSmallPad);
+  auto small = [&]() {
+    // as few blocks per thread as the cluster allows: latency is what counts here
+    int ctas = 1;
+    while (ctas < kSmallCtas && n_blocks > (int64_t)ctas * kSmallThreads) ctas *= 2;
+    const int64_t per = (n_blocks + (int64_t)ctas * kSmallThreads - 1) / ((int64_t)ctas * kSmallThreads);
+#define NVFP4_SMALL(B) \
+  launch_small<B>(x, rows, cols, amax_dev, packed, scales_linear, scales_swizzled, global_scale_dev, ctas, st)
+    return per <= 1 ? NVFP4_SMALL(1) : per <= 2 ? NVFP4_SMALL(2) : per <= 4 ? NVFP4_SMALL(4) : NVFP4_SMALL(8);
+#undef NVFP4_SMALL
+  };
+  if (small_fits && n_blocks <= kSmallBest) return small();
+  int threads;
+  if (n_blocks > 0 && partials && rows_form(rows, cols, scales_swizzled != nullptr, &threads) &&
+      !(alone && threads > kPackThreads && n_blocks <= kAloneBlocks)) {
+    const int64_t n_vec = n_blocks * 2;
+    const unsigned grid = partial_grid(n_vec);
+    const AmaxArgs<1> first{{reinterpret_cast<const uint4*>(x)}, {n_vec}, {0u, grid}, wide_bit(x), nullptr, 0};
+    rc = n_blocks * 32 > kKeepFrom ? launch_dependent(amax_bf16_kernel<1, true>, dim3(grid), kThreads, 0, 1, st, first,
+                                                      reinterpret_cast<unsigned*>(partials))
+                                   : launch_dependent(amax_bf16_kernel<1, false>, dim3(grid), kThreads, 0, 1, st, first,
+                                                      reinterpret_cast<unsigned*>(partials));
+    if (rc != NVFP4_OK) return rc;
+    PackArgs a{};
+    a.x = reinterpret_cast<const uint4*>(x);
+    a.rows = rows;
+    a.units = (int)(cols / kBlock);
+    a.partial = reinterpret_cast<const unsigned*>(partials);
+    a.n_partial = (int)grid;
+    a.amax_out = amax_dev;
+    a.packed = reinterpret_cast<uint2*>(packed);
+    a.sf_lin = scales_linear;
+    a.sf_swz = scales_swizzled;
+    a.k_atoms = (uint32_t)sf_k_atoms(cols);
+    a.gscale_out = global_scale_dev;
+    a.wide_x = (reinterpret_cast<uintptr_t>(x) & 31u) == 0;
+    a.word_swz = (reinterpret_cast<uintptr_t>(scales_swizzled) & 3u) == 0;
+    return launch_rows(a, threads, st);
+  }
+  // Widths that the rows form does not take: the resident form where the tensor fits.  Not ahead of the rows
+  // form, whose two kernels overlap what comes before and each other: us, resident and rows, [4095, 4096] 23.1 and 15.9,
+  // [4095, 5120] 23.1 and 16.6 (both bound by the host from there down); with a GEMM behind it 512 x 3072 x 4096 (M, N, K) 18.2
+  // and 15.8, 900 x 5120 x 5120 29.2 and 26.8, 2500 x 5120 x 5120 46.7 and 42.4, 300 x 15360 x 5120 29.2 and 27.6.  But a few rows
+  // alone are a matter of launches: [512, 4096] 14.4 and 16.0, [1500, 5120] 14.8 and 15.8 through the public call.
+  if (n_blocks > 0 && partials && aligned16(scales_swizzled) &&
+      (!scales_swizzled || sf_swizzled_bytes(rows, cols) <= n_blocks * 4)) {
+    bool done = false;
+    rc = launch_resident(x, rows, cols, amax_dev, packed, scales_linear, scales_swizzled, global_scale_dev, partials, st,
+                         &done);
+    if (rc != NVFP4_OK || done) return rc;
+  }
+  if (small_fits) return small();
+  rc = nvfp4_amax_bf16(x, rows * cols, amax_dev, stream);
+  if (rc != NVFP4_OK) return rc;
+  return quantize_impl(x, rows, cols, amax_dev, 0.0f, packed, scales_linear, scales_swizzled,
+                       global_scale_dev, stream);
+}
+
 }  // namespace nvfp4
 
 using namespace nvfp4;
@@ -832,66 +909,8 @@ int nvfp4_quantize_bf16(const void* x, int64_t rows, int64_t cols, const float* 
 int nvfp4_amax_quantize_bf16(const void* x, int64_t rows, int64_t cols, float* amax_dev, uint8_t* packed,
                              uint8_t* scales_linear, uint8_t* scales_swizzled, float* global_scale_dev,
                              float* partials, void* stream) {
-  int rc = check_quantize(x, rows, cols, packed);
-  if (rc != NVFP4_OK) return rc;
-  if (!amax_dev) return NVFP4_ERR_BAD_ARG;
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const int64_t n_blocks = rows * cols / kBlock;
-  const bool small_fits = n_blocks > 0 && n_blocks <= kSmallMax && aligned16(scales_swizzled) &&
-                          (!scales_swizzled || sf_swizzled_bytes(rows, cols) <= kSmallPad);
-  auto small = [&]() {
-    // as few blocks per thread as the cluster allows: latency is what counts here
-    int ctas = 1;
-    while (ctas < kSmallCtas && n_blocks > (int64_t)ctas * kSmallThreads) ctas *= 2;
-    const int64_t per = (n_blocks + (int64_t)ctas * kSmallThreads - 1) / ((int64_t)ctas * kSmallThreads);
-#define NVFP4_SMALL(B) \
-  launch_small<B>(x, rows, cols, amax_dev, packed, scales_linear, scales_swizzled, global_scale_dev, ctas, st)
-    return per <= 1 ? NVFP4_SMALL(1) : per <= 2 ? NVFP4_SMALL(2) : per <= 4 ? NVFP4_SMALL(4) : NVFP4_SMALL(8);
-#undef NVFP4_SMALL
-  };
-  if (small_fits && n_blocks <= kSmallBest) return small();
-  int threads;
-  if (n_blocks > 0 && partials && rows_form(rows, cols, scales_swizzled != nullptr, &threads)) {
-    const int64_t n_vec = n_blocks * 2;
-    const unsigned grid = partial_grid(n_vec);
-    const AmaxArgs<1> first{{reinterpret_cast<const uint4*>(x)}, {n_vec}, {0u, grid}, wide_bit(x), nullptr, 0};
-    rc = n_blocks * 32 > kKeepFrom ? launch_dependent(amax_bf16_kernel<1, true>, dim3(grid), kThreads, 0, 1, st, first,
-                                                      reinterpret_cast<unsigned*>(partials))
-                                   : launch_dependent(amax_bf16_kernel<1, false>, dim3(grid), kThreads, 0, 1, st, first,
-                                                      reinterpret_cast<unsigned*>(partials));
-    if (rc != NVFP4_OK) return rc;
-    PackArgs a{};
-    a.x = reinterpret_cast<const uint4*>(x);
-    a.rows = rows;
-    a.units = (int)(cols / kBlock);
-    a.partial = reinterpret_cast<const unsigned*>(partials);
-    a.n_partial = (int)grid;
-    a.amax_out = amax_dev;
-    a.packed = reinterpret_cast<uint2*>(packed);
-    a.sf_lin = scales_linear;
-    a.sf_swz = scales_swizzled;
-    a.k_atoms = (uint32_t)sf_k_atoms(cols);
-    a.gscale_out = global_scale_dev;
-    a.wide_x = (reinterpret_cast<uintptr_t>(x) & 31u) == 0;
-    a.word_swz = (reinterpret_cast<uintptr_t>(scales_swizzled) & 3u) == 0;
-    return launch_rows(a, threads, st);
-  }
-  // Widths that the rows form does not take: the resident form where the tensor fits.  Not ahead of the rows
-  // form, whose two kernels overlap what comes before and each other: flat with its memsets, rows, resident us
-  // [512, 4096] 9.3, -, 6.6; [1490, 4096] 14.5, -, 10.5; [2500, 5120] 19.9, -, 16.2; [900, 14336] 20.1, -, 16.4;
-  // [1024, 3072] -, 7.6, 8.6; [4096, 3072] -, 16.2, 16.2, and with the GEMM behind it 37.7 and 41.0.
-  if (n_blocks > 0 && partials && aligned16(scales_swizzled) &&
-      (!scales_swizzled || sf_swizzled_bytes(rows, cols) <= n_blocks * 4)) {
-    bool done = false;
-    rc = launch_resident(x, rows, cols, amax_dev, packed, scales_linear, scales_swizzled, global_scale_dev, partials, st,
-                         &done);
-    if (rc != NVFP4_OK || done) return rc;
-  }
-  if (small_fits) return small();
-  rc = nvfp4_amax_bf16(x, rows * cols, amax_dev, stream);
-  if (rc != NVFP4_OK) return rc;
-  return quantize_impl(x, rows, cols, amax_dev, 0.0f, packed, scales_linear, scales_swizzled,
-                       global_scale_dev, stream);
+  return amax_quantize(x, rows, cols, amax_dev, packed, scales_linear, scales_swizzled, global_scale_dev, partials, true,
+                       stream);
 }
 
 int nvfp4_quantize_bf16_amax(const void* x, uint8_t* packed, uint8_t* scales, int64_t n,

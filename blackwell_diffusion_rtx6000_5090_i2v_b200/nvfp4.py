@@ -137,9 +137,13 @@ class FP4Tensor:
         self._device = input.device
         n = input.numel()
         self._numel = n
-        if amax_hook is None and (out is None or out.holds(input, linear_scales)):
-            made = (N.host.quantize(input, linear_scales, swizzled_scales) if out is None and amax is None else
-                    N.host.quantize_into(input, linear_scales, swizzled_scales, amax, None if out is None else out.tensors))
+        if amax_hook is None:
+            if out is None and amax is None:
+                made = N.host.quantize(input, linear_scales, swizzled_scales)
+            elif out is None or out.holds(input, linear_scales):
+                made = N.host.quantize_into(input, linear_scales, swizzled_scales, amax, None if out is None else out.tensors)
+            else:
+                made = None
             if made is not None:
                 (self._rows, self._cols, self._data, self._scales, self._scales_swz, self._amax,
                  self._gscale) = made
