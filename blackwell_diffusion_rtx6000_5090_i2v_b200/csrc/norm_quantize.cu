@@ -257,6 +257,21 @@ __device__ __forceinline__ uint32_t normalize16(uint32_t a2, const uint32_t (&xp
 
 // kWhole: both vectors of every kind are given and every thread has blocks (T * kJ * 16 == cols), so that nothing of that
 // is asked for each pair of elements or block.
+// The maximum of m and |h| of a block, h before its rounding to bf16: rounding keeps the order, so that the rounded
+// maximum is the maximum of the rounded (NaNs are passed over by both).  One three-operand instruction a pair.
+template <bool kAffine, bool kMod>
+__device__ __forceinline__ float max_normed16(float m, const uint32_t (&xp)[8], float mean, float2 r2, const float2 (&cw)[8],
+                                              const float2 (&cb)[8], const float2 (&cs)[8], const float2 (&ct)[8]) {
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    float2 y = f2_mul(bf16x2_sub(xp[e], mean), r2);
+    if (kAffine) y = f2_add(f2_mul(y, cw[e]), cb[e]);
+    if (kMod) y = f2_add(f2_mul(y, cs[e]), ct[e]);
+    asm("max.abs.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(y.x), "f"(y.y));
+  }
+  return m;
+}
+
 template <bool kQuantize, int kJ, bool kAffine, bool kMod, bool kWhole>
 __global__ void __launch_bounds__(kMaxThreads)
 norm_mod_kernel(const NormArgs p) {
@@ -347,6 +362,10 @@ norm_mod_kernel(const NormArgs p) {
   }
 
   uint32_t amax_t = 0u;                 // bf16x2 running max of |h| (sweep 1)
+  float amax_f = 0.0f;                  // the same where max_normed16 takes it
+  // With one block a thread, no h wanted (with_variant): [27280, 3072] with all four vectors, both sweeps, 123.0 -> 116.9 us.
+  // With two it gains or loses by the width ([32760, 5120] 157.3 -> 152.7, [27280, 3072] affine 82.2 -> 83.1).
+  constexpr bool kMaxOnly = !kQuantize && kWhole && kJ == 1;
   const float cols_f = (float)p.cols, cols_inv = __fdiv_rn(1.0f, cols_f);
 
   // sweep 2 asks for a group's row statistics one group ahead: the load would otherwise sit
@@ -476,6 +495,12 @@ norm_mod_kernel(const NormArgs p) {
       for (int j = 0; j < kJ; ++j) {
         const int u = threadIdx.x + j * T;
         const bool on = live[j] && row_ok[r];
+        if constexpr (kMaxOnly) {
+          if (on)
+            amax_f = max_normed16<kAffine, kMod>(amax_f, xp[r][j], mean[r], r2, cw[kAffine ? j : 0], cb[kAffine ? j : 0],
+                                                 cs[kMod ? j : 0], ct[kMod ? j : 0]);
+          continue;
+        }
         uint32_t hp[8];
         const uint32_t a2 = normalize16<kAffine, kMod>(
             kQuantize ? 0u : amax_t, xp[r][j], m2, r2, cw[kAffine ? j : 0], cb[kAffine ? j : 0], cs[kMod ? j : 0],
@@ -515,8 +540,9 @@ norm_mod_kernel(const NormArgs p) {
   }
 
   if (!kQuantize) {
-    const float amax_f = fmaxf(fabsf(bf16lo_to_f32(amax_t)), fabsf(bf16hi_to_f32(amax_t)));
-    const unsigned bits = __reduce_max_sync(0xffffffffu, __float_as_uint(amax_f));
+    const float amax = kMaxOnly ? __bfloat162float(__float2bfloat16(amax_f))
+                              : fmaxf(fabsf(bf16lo_to_f32(amax_t)), fabsf(bf16hi_to_f32(amax_t)));
+    const unsigned bits = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));
     __syncthreads();
     if ((threadIdx.x & 31) == 0) red_max[threadIdx.x >> 5] = __uint_as_float(bits);
     __syncthreads();
@@ -857,7 +883,7 @@ int with_variant(const NormArgs& a, int* threads, F&& f) {
   int J;
   const bool affine = a.w || a.b, mod = a.scale || a.shift;
   shape_for(a.cols / 16, affine + mod, &J, threads);
-  const bool whole = (!affine || (a.w && a.b)) && (!mod || (a.scale && a.shift)) && *threads * J * 16 == a.cols;
+  const bool whole = (!affine || (a.w && a.b)) && (!mod || (a.scale && a.shift)) && *threads * J * 16 == a.cols && (J == 2 || !a.h_out);
   auto go = [&](auto j, auto with_affine, auto with_mod) {
     return whole ? f(j, with_affine, with_mod, std::true_type()) : f(j, with_affine, with_mod, std::false_type());
   };
