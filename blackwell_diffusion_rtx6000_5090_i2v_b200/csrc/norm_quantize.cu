@@ -30,8 +30,8 @@
 // 128-entry table per tensor); scale offsets split into a per-row and a per-thread part.
 // What is known of a call is a template parameter (kWhole), the widening of x is part of its subtraction, |h| and its
 // maximum are one instruction, and the means' divisions are three operations.  Both sweeps, us, before and after:
-// [27280, 3072] modulation 96.4 -> 82.1, affine 96.4 -> 81.9, all four vectors 147 -> 123, [32760, 5120] modulation 186 -> 157,
-// [12000, 6384] 152 -> 122; 31 M -> 25 M instructions a sweep.
+// [27280, 3072] modulation 96.4 -> 81.7, affine 96.4 -> 80.6, all four vectors 147 -> 117, [32760, 5120] modulation 186 -> 156,
+// [12000, 6384] 152 -> 122; 31 M -> 24 M and 28 M instructions.
 // Sweep 1 leaves mean and rstd per row in a small stats buffer so that sweep 2, which needs
 // no reduction at all, repeats exactly the same arithmetic.
 //
@@ -231,7 +231,9 @@ __device__ __forceinline__ float2 bf16x2_sub(uint32_t w, float m) {
 }
 
 // h for one 16-element block as 8 packed bf16 pairs, and the running bf16x2 max of |h| and a2, whose signs mean nothing.
-template <bool kAffine, bool kMod>
+// kMixed: widening and mean in one subtraction a lane (sweep 2 has fewer instructions the other way, but with all four vectors:
+// [27280, 3072] affine 82.0 -> 80.6 us, modulation 82.1 -> 81.7, all four 116.9 -> 117.1).
+template <bool kAffine, bool kMod, bool kMixed>
 __device__ __forceinline__ uint32_t normalize16(uint32_t a2, const uint32_t (&xp)[8], float2 m2, float2 r2,
                                                 const float2 (&cw)[8], const float2 (&cb)[8],
                                                 const float2 (&cs)[8], const float2 (&ct)[8],
@@ -239,7 +241,7 @@ __device__ __forceinline__ uint32_t normalize16(uint32_t a2, const uint32_t (&xp
                                                 uint32_t (&hp)[8]) {
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
-    float2 y = f2_mul(bf16x2_sub(xp[e], m2.x), r2);
+    float2 y = f2_mul(kMixed ? bf16x2_sub(xp[e], m2.x) : f2_sub(bf16x2_to_f2(xp[e]), m2), r2);
     if (kAffine) {
       if (has_w) y = f2_mul(y, cw[e]);
       if (has_b) y = f2_add(y, cb[e]);
@@ -502,7 +504,7 @@ norm_mod_kernel(const NormArgs p) {
           continue;
         }
         uint32_t hp[8];
-        const uint32_t a2 = normalize16<kAffine, kMod>(
+        const uint32_t a2 = normalize16<kAffine, kMod, !kQuantize || (kAffine && kMod)>(
             kQuantize ? 0u : amax_t, xp[r][j], m2, r2, cw[kAffine ? j : 0], cb[kAffine ? j : 0], cs[kMod ? j : 0],
             ct[kMod ? j : 0], has_w, has_b, has_s, has_t, hp);
         if (!kQuantize) {
@@ -689,7 +691,7 @@ norm_mod_resident_kernel(const NormArgs p, int per_cta, unsigned* partial) {
       for (int j = 0; j < kJ; ++j) {
         const int u = threadIdx.x + j * T;
         uint32_t hp[8];
-        const uint32_t a2 = normalize16<kAffine, kMod>(
+        const uint32_t a2 = normalize16<kAffine, kMod, true>(
             amax_t, xp[r][j], m2, r2, cw[kAffine ? j : 0], cb[kAffine ? j : 0], cs[kMod ? j : 0], ct[kMod ? j : 0], has_w,
             has_b, has_s, has_t, hp);
         if (live[j] && row_ok[r]) {
