@@ -10,6 +10,7 @@
 // stream's queue is full and an allocation may reach the driver, and neither needs the interpreter.  Their errors are
 // torch's (an allocation that does not fit raises torch.OutOfMemoryError).
 #include <ATen/TensorSubclassLikeUtils.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -220,7 +221,13 @@ Maybe gemm(const Tensor& a, const Tensor& b, const Tensor& a_scales, const Tenso
   return d;
 }
 
-// The gradients that are wanted of y = x @ w.T + b: dx, dw, db
+// Whether something follows what is done to t: a graph being recorded, a forward-mode tangent, a trace.
+bool followed(const Tensor& t) {
+  return (t.requires_grad() && at::GradMode::is_enabled()) || t._fw_grad(0).defined() ||
+         c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::Tracer);
+}
+
+// The gradients that are wanted of y = x @ w.T + b: dx, dw, db (not db where dy is followed: it stays torch's sum)
 std::optional<std::vector<Maybe>> linear_backward(const Tensor& dy, const Tensor& x, const Tensor& w, bool want_dx,
                                                   bool want_dw, bool want_db) {
   if (!plain(dy) || !plain(x) || !plain(w) || modes() || (!want_dx && !want_dw) || dy.dim() < 1 || x.dim() < 1 ||
@@ -236,7 +243,7 @@ std::optional<std::vector<Maybe>> linear_backward(const Tensor& dy, const Tensor
   Maybe dx, dw, db;
   if (want_dx) dx = empty(x.sizes(), at::kBFloat16, dy);
   if (want_dw) dw = empty({n, k}, at::kBFloat16, dy);
-  if (want_db) db = empty({n}, at::kBFloat16, dy);
+  if (want_db && !followed(dy)) db = empty({n}, at::kBFloat16, dy);
   const Tensor ws = empty({nvfp4_linear_backward_workspace_bytes(m, n, k)}, at::kByte, dy);
   check(nvfp4_linear_backward_bias_bf16(dy.data_ptr(), want_dw ? x.data_ptr() : nullptr, want_dx ? w.data_ptr() : nullptr,
                                         nullptr, m, n, k, ptr(dx), ptr(dw), ptr(db), ws.data_ptr(), status_of(dy),

@@ -18,6 +18,8 @@ import weakref
 from typing import List, Optional, Tuple
 
 import torch
+from torch.autograd.forward_ad import unpack_dual
+from torch.utils._python_dispatch import is_in_torch_dispatch_mode
 
 from . import _native as N
 from .nvfp4 import FP4Tensor, fp4_gemm
@@ -238,6 +240,13 @@ def forward(input: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor,
     return linear(input, weight, bias)
 
 
+def _followed(t: torch.Tensor) -> bool:
+    """Whether something follows what is done to ``t`` (a graph being recorded, a forward-mode tangent, a trace, a
+    dispatch mode), so that a sum over it stays an operation of torch."""
+    return (t.requires_grad and torch.is_grad_enabled() or torch.jit.is_tracing() or is_in_torch_dispatch_mode()
+            or unpack_dual(t).tangent is not None)
+
+
 def backward(grad_output: torch.Tensor, input: torch.Tensor, weight: torch.Tensor,
              scale_input: torch.Tensor, scale_weight: torch.Tensor,
              scale_grad_output: torch.Tensor, needs_input_grad: bool, needs_weight_grad: bool,
@@ -248,11 +257,9 @@ def backward(grad_output: torch.Tensor, input: torch.Tensor, weight: torch.Tenso
     there, ``grad_output.T @ input``, is what is computed here."""
     if grad_output.is_cuda:
         N.status_word(grad_output.device)
-    # a backward that is itself differentiated keeps the bias gradient's sum as an operation of torch
-    own_sum = needs_bias_grad and not (grad_output.requires_grad and torch.is_grad_enabled())
-    made = N.host.linear_backward(grad_output, input, weight, needs_input_grad, needs_weight_grad, own_sum)
+    made = N.host.linear_backward(grad_output, input, weight, needs_input_grad, needs_weight_grad, needs_bias_grad)
     if made is not None:
-        if needs_bias_grad and not own_sum:
+        if needs_bias_grad and made[2] is None:
             made[2] = grad_output.reshape(-1, weight.size(0)).sum(0)
         return made
     in_features = input.size(-1)
@@ -280,7 +287,7 @@ def backward(grad_output: torch.Tensor, input: torch.Tensor, weight: torch.Tenso
         with N.device_guard(dev):
             ws = torch.empty(N.lib.nvfp4_linear_backward_workspace_bytes(m, out_features, k),
                              dtype=torch.uint8, device=dev)
-            if own_sum:
+            if needs_bias_grad and not _followed(go):
                 grad_bias = torch.empty(out_features, dtype=torch.bfloat16, device=dev)
             # the maximum of the weight is taken here, not from the forward's packed copy: a write
             # through weight.data would leave that one behind
