@@ -787,25 +787,28 @@ int launch_variant(const NormArgs& a, int threads, cudaStream_t st) {
   auto kernel = norm_mod_kernel<kQuantize, kJ, kAffine, kMod, kWhole>;
   constexpr int kR = RowsPerIter<kJ>::value;
   const size_t smem = (size_t)kStages * kR * a.cols * 2;
-  // (dynamic shared memory limit, CTAs per SM) of the last geometry this variant saw on each
-  // device: a model calls it with one row width over and over
-  struct Geometry { size_t smem; int threads; int per_sm; };
-  static Geometry cached[64];
   int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) dev = 0;
-  Geometry& c = cached[dev];
-  if (c.per_sm < 1 || c.smem != smem || c.threads != threads) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return NVFP4_ERR_BAD_ARG;
+  // One limit for all widths: one that followed the width could be lowered by another thread between this thread's
+  // question and its launch, which is then refused.
+  static std::atomic<bool> allowed[64];
+  if (!allowed[dev].load(std::memory_order_acquire)) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStages * kR * kJ * 16 * kMaxThreads * 2) !=
         cudaSuccess)
       return NVFP4_ERR_LAUNCH_FAILED;
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem) != cudaSuccess ||
-        n < 1)
-      return NVFP4_ERR_LAUNCH_FAILED;
-    c = Geometry{smem, threads, n};
+    allowed[dev].store(true, std::memory_order_release);
   }
-  const int per_sm = c.per_sm;
+  // CTAs that an SM holds, for the last geometry of this variant in this thread: a model calls it with one row width over
+  // and over
+  struct Geometry { int dev, cols, threads, per_sm; };
+  static thread_local Geometry last{};
+  if (last.per_sm < 1 || last.dev != dev || last.cols != a.cols || last.threads != threads) {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem) != cudaSuccess || n < 1)
+      return NVFP4_ERR_LAUNCH_FAILED;
+    last = {dev, a.cols, threads, n};
+  }
+  const int per_sm = last.per_sm;
   const int64_t groups = (a.rows + kR - 1) / kR;
   const int64_t resident = (int64_t)sm_count() * per_sm;
   const unsigned grid = (unsigned)(groups < resident ? groups : resident);
