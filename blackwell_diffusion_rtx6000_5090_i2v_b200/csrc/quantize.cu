@@ -664,9 +664,16 @@ int quantize_impl(const void* x, int64_t rows, int64_t cols, const float* amax_d
   // form (its table, a CTA's idle lanes) pays only for long tensors and nearly full CTAs.  Replayed from a
   // graph, us flat and rows: [256, 3072] 2.4 and 2.9, [4096, 3072] 6.1 and 6.1, [16384, 3072] 19.9 and
   // 18.8, [16384, 1280] 8.9 and 9.2; with a pad, and so a memset, [170, 3072] 3.9 and 2.8.
+  // The wider CTAs pay only with a pad, and those of more than 224 threads (3584 columns) not for long tensors: flat and rows,
+  // with a pad [32, 5120] 3.5 and 2.9, [1000, 4096] 4.6 and 3.4, [4095, 5120] 11.3 and 10.3, [8191, 5120] 18.8 and 17.7, [10001, 5120]
+  // 22.9 and 23.1, [32760, 5120] 67.2 and 70.3, but [32760, 3280] 45.4 and 44.9; without [4096, 4096] 7.7 and 7.9, [16384, 5120]
+  // 34.1 and 35.4, linear scales only [4096, 5120] 8.0 and 9.4.
   const bool pads = sf_swz && (rows % 256 != 0 || cols / kBlock % kSfKbPad != 0);
-  if (rows_form(rows, cols, sf_swz != nullptr, &threads) &&
-      (pads || (n_blocks >= (1 << 20) && cols / kBlock * 8 >= (int64_t)threads * 7))) {
+  const auto pays = [&] {
+    if (threads > kPackThreads) return pads && (threads <= 224 || n_blocks <= 3 << 20);
+    return pads || (n_blocks >= (1 << 20) && cols / kBlock * 8 >= (int64_t)threads * 7);
+  };
+  if (rows_form(rows, cols, sf_swz != nullptr, &threads) && pays()) {
     PackArgs a{};
     a.x = reinterpret_cast<const uint4*>(x);
     a.rows = rows;
