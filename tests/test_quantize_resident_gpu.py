@@ -33,7 +33,8 @@ def _run(one, x, rows, cols, linear=True, swizzled=True, shift=0, part=None, che
     (128, 4096), (129, 4096), (1, 262160), (300, 272),
     (296, 8192), (296, 8208),                            # one block a thread of the grid, and a few over
     (1480, 9840), (1776, 8192), (1776, 8208),            # the last that fits, and the first that does not
-    (700, 14336), (2500, 5120), (100, 13824),
+    (700, 14336), (1700, 8192), (900, 14336), (100, 13824),
+    (1536, 5120), (1537, 5120), (2500, 5120),            # rows of a CTA's width: the last that take one launch, and rows
 ])
 def test_forms_agree_at_their_edges(rows, cols):
     g = torch.Generator(device="cuda").manual_seed(rows + cols)
@@ -54,7 +55,7 @@ def test_buffers_a_caller_may_give(form, offset):
 @pytest.mark.parametrize("graph", [False, True])
 @pytest.mark.parametrize("rows,cols,ctas", [
     (64, 4096, 0),                          # the one-cluster form
-    (128, 4096, 64), (600, 4096, 150), (700, 14336, 245), (1776, 8192, 296),
+    (128, 4096, 64), (600, 4096, 150), (1536, 5120, 240), (700, 14336, 245), (900, 14336, 263), (1700, 8192, 284), (1776, 8192, 296),
     (1480, 9840, 0), (1776, 8208, 0), (27280, 14336, 0),    # more than the shared memory holds: the maximum in a pass of its own
 ])
 def test_which_form_is_taken(rows, cols, ctas, graph):
@@ -98,11 +99,18 @@ def test_beside_other_kernels_that_want_the_whole_gpu():
     """Two one-launch quantizers, a one-launch norm and an attention on a stream each: the grids that meet share
     the GPU with one another and with a kernel that does not."""
     from blackwell_diffusion_rtx6000_5090_i2v_b200 import _native as N, dit
-    from blackwell_diffusion_rtx6000_5090_i2v_b200.nvfp4 import FP4Tensor
-    xs = [torch.randn(n, 5120, device="cuda").bfloat16() for n in (2500, 2600)]
+    from blackwell_diffusion_rtx6000_5090_i2v_b200.nvfp4 import FP4Tensor, PackedBuffers
+    sizes = {(1700, 8192): 284, (900, 14336): 263}       # and the CTAs of their one launch
+    xs = [torch.randn(s, device="cuda").bfloat16() for s in sizes]
     y = torch.randn(4096, 3072, device="cuda").bfloat16()
     heads = y.view(4096, 24, 128)
-    calls = [lambda: FP4Tensor.from_bfloat16(xs[0]), lambda: FP4Tensor.from_bfloat16(xs[1]),
+    partials = [[], []]
+
+    def quantize(i):
+        out = PackedBuffers(*xs[i].shape, "cuda", linear_scales=True)
+        partials[i].append(out.partials.fill_(float("nan")))
+        return FP4Tensor.from_bfloat16(xs[i], out=out)
+    calls = [lambda: quantize(0), lambda: quantize(1),
              lambda: FP4Tensor.from_norm_mod(y), lambda: dit.attention_native(heads, heads, heads)]
     want = [c() for c in calls]
     streams = [torch.cuda.Stream() for _ in calls]
@@ -121,3 +129,6 @@ def test_beside_other_kernels_that_want_the_whole_gpu():
         else:
             assert torch.equal(t._data, w._data) and torch.equal(t._scales_swz, w._scales_swz)
             assert torch.equal(t._gscale, w._gscale)
+    # that each quantizer was one launch: its CTAs alone leave partial maxima
+    for parts, ctas in zip(partials, sizes.values()):
+        assert len(parts) == 31 and all(int((~torch.isnan(p)).sum()) == ctas for p in parts)
