@@ -135,8 +135,8 @@ def test_where_the_rows_fit(rows, cols, kind, one, graph):
     assert _one_launch(rows, cols, kind, graph) == one
 
 
-@pytest.mark.parametrize("rows,cols", [(300, 3072), (64, 10240), (1900, 272)])
-@pytest.mark.parametrize("kind", [0, 2])
+@pytest.mark.parametrize("rows,cols", [(300, 3072), (257, 5120), (70, 1536), (64, 10240), (1900, 272)])
+@pytest.mark.parametrize("kind", [0, 2, 3])
 @pytest.mark.parametrize("rms", [0, 1])
 @pytest.mark.parametrize("what", ["inf", "-inf", "nan", "nan row", "largest", "all nan"])
 def test_special_values(rows, cols, kind, rms, what):
