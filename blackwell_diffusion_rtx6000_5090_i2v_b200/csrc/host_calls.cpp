@@ -1,5 +1,5 @@
 // The Python layer's frequent calls in one native step each: argument checks, allocations, stream and
-// library call.  Through ctypes these cost 11 to 38 us a call (a linear 27, a quantizer 21 to 28, norm + quantize
+// library call.  Through ctypes these cost 11 to 45 us a call (a linear 27, a quantizer 21 to 28, norm + quantize
 // 30 to 38, the backward of a linear 45), more than the kernels of a few thousand rows take.
 //
 // Every function returns None for what is not the plain case (other types, devices, layouts or alignments,

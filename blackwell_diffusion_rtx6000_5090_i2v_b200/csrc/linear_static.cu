@@ -145,7 +145,8 @@ int64_t nvfp4_linear_backward_workspace_bytes(int64_t M, int64_t N, int64_t K) {
 
 // Four launches: the maxima of all operands, all operands packed (and the bias gradient), the two products.  The
 // kernels of [2048, 3072] x 3072 take 60 us so, and took 89 as a launch or two per operand, memsets and torch's
-// sum; the training pass, which waits for its fifteen launches from Python, 168 -> 138 us.
+// sum; the training pass, which waits for the host, 168 -> 138 us, and 110 with the native call in front.
+// (dy's maximum is taken whatever is wanted, so with db alone for nothing: no caller in this package asks for that.)
 int nvfp4_linear_backward_bias_bf16(const void* dy_bf16, const void* x_bf16, const void* w_bf16,
                                     const float* w_amax_dev, int64_t M, int64_t N, int64_t K, void* dx_bf16,
                                     void* dw_bf16, void* db_bf16, void* workspace, int* status_dev, void* stream) {

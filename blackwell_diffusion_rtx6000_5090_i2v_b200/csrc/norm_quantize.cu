@@ -257,8 +257,6 @@ __device__ __forceinline__ uint32_t normalize16(uint32_t a2, const uint32_t (&xp
   return a2;
 }
 
-// kWhole: both vectors of every kind are given and every thread has blocks (T * kJ * 16 == cols), so that nothing of that
-// is asked for each pair of elements or block.
 // The maximum of m and |h| of a block, h before its rounding to bf16: rounding keeps the order, so that the rounded
 // maximum is the maximum of the rounded (NaNs are passed over by both).  One three-operand instruction a pair.
 template <bool kAffine, bool kMod>
@@ -274,6 +272,8 @@ __device__ __forceinline__ float max_normed16(float m, const uint32_t (&xp)[8], 
   return m;
 }
 
+// kWhole: both vectors of every kind are given and every thread has blocks (T * kJ * 16 == cols), so that nothing of that
+// is asked for each pair of elements or block.
 template <bool kQuantize, int kJ, bool kAffine, bool kMod, bool kWhole>
 __global__ void __launch_bounds__(kMaxThreads)
 norm_mod_kernel(const NormArgs p) {

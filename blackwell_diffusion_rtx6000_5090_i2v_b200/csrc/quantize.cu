@@ -816,10 +816,11 @@ int launch_amax_partials(AmaxJob (&jobs)[3], int n_jobs, float* partials, unsign
                           reinterpret_cast<unsigned*>(partials));
 }
 
-// Wide rows in up to this many blocks are packed in one launch where no GEMM follows (amax_quantize).
+// Wide rows in up to this many blocks are packed in one launch where the caller says nothing of what follows
+// (amax_quantize): the public entry cannot know, nvfp4_linear_bf16 does.
 constexpr int64_t kAloneBlocks = 480 << 10;
 
-// `alone`: nothing is known to follow on the stream.
+// `alone`: nothing is known to follow on the stream (something may: a program that quantizes and multiplies in two calls).
 int amax_quantize(const void* x, int64_t rows, int64_t cols, float* amax_dev, uint8_t* packed, uint8_t* scales_linear,
                   uint8_t* scales_swizzled, float* global_scale_dev, float* partials, bool alone, void* stream) {
   int rc = check_quantize(x, rows, cols, packed);
@@ -867,11 +868,12 @@ int amax_quantize(const void* x, int64_t rows, int64_t cols, float* amax_dev, ui
     a.word_swz = (reinterpret_cast<uintptr_t>(scales_swizzled) & 3u) == 0;
     return launch_rows(a, threads, st);
   }
-  // Widths that the rows form does not take: the resident form where the tensor fits.  Not ahead of the rows
-  // form, whose two kernels overlap what comes before and each other: us, resident and rows, [4095, 4096] 23.1 and 15.9,
-  // [4095, 5120] 23.1 and 16.6 (both bound by the host from there down); with a GEMM behind it 512 x 3072 x 4096 (M, N, K) 18.2
-  // and 15.8, 900 x 5120 x 5120 29.2 and 26.8, 2500 x 5120 x 5120 46.7 and 42.4, 300 x 15360 x 5120 29.2 and 27.6.  But a few rows
-  // alone are a matter of launches: [512, 4096] 14.4 and 16.0, [1500, 5120] 14.8 and 15.8 through the public call.
+  // What the rows form does not take: the resident form where the tensor fits.  Not ahead of the rows form, whose two
+  // kernels overlap what comes before and each other: us, resident and rows, [4095, 4096] 23.1 and 15.9, [4095, 5120] 23.1 and 16.6
+  // (both bound by the host from there down); with a GEMM behind it 512 x 3072 x 4096 (M, N, K) 18.2 and 15.8, 900 x 5120 x 5120 29.2
+  // and 26.8, 2500 x 5120 x 5120 46.7 and 42.4, 300 x 15360 x 5120 29.2 and 27.6.  But a few wide rows of a caller that says
+  // nothing of a GEMM are a matter of launches: through the public call [512, 4096] 14.4 and 16.0, [1500, 5120] 14.8 and 15.8.
+  // (Where that caller has a GEMM follow all the same, and no host time to save, it pays the difference above.)
   if (n_blocks > 0 && partials && aligned16(scales_swizzled) &&
       (!scales_swizzled || sf_swizzled_bytes(rows, cols) <= n_blocks * 4)) {
     bool done = false;

@@ -2,11 +2,12 @@
 
     python -m blackwell_diffusion_rtx6000_5090_i2v_b200.profile_case gemm --m 8192 --n 9216 --k 3072
     python -m blackwell_diffusion_rtx6000_5090_i2v_b200.profile_case quantize --m 27280 --k 3072
-    python -m blackwell_diffusion_rtx6000_5090_i2v_b200.profile_case amax_quantize --m 2500 --k 5120
+    python -m blackwell_diffusion_rtx6000_5090_i2v_b200.profile_case amax_quantize --m 1700 --k 8192
     python -m blackwell_diffusion_rtx6000_5090_i2v_b200.profile_case norm --m 27280 --k 3072
     python -m blackwell_diffusion_rtx6000_5090_i2v_b200.profile_case rope --m 27280 --k 3072
     python -m blackwell_diffusion_rtx6000_5090_i2v_b200.profile_case return --m 32760 --k 5120
     python -m blackwell_diffusion_rtx6000_5090_i2v_b200.profile_case attention --m 27280 --k 3072
+    python -m blackwell_diffusion_rtx6000_5090_i2v_b200.profile_case backward --m 2048 --n 3072 --k 3072
 
 Each case holds well under a few GB on the device, launches the kernel
 ``--iters`` times after ``--warmup`` launches, and prints the CUDA-event time.
@@ -37,7 +38,8 @@ def _time(fn, warmup, iters):
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("kernel", choices=["gemm", "quantize", "amax", "amax_quantize", "norm", "rope", "return", "attention"])
+    ap.add_argument("kernel", choices=["gemm", "quantize", "amax", "amax_quantize", "norm", "rope", "return", "attention",
+                                       "backward"])
     ap.add_argument("--tiling", choices=["auto", "uniform", "alternating"], default="auto")
     ap.add_argument("--m", type=int, default=8192)
     ap.add_argument("--n", type=int, default=9216)
@@ -129,6 +131,14 @@ def main():
         n = a.m * a.k
         print(f"norm+mod+quantize [{a.m}, {a.k}]: {ms:.4f} ms, algorithmic {2.5625 * n / ms / 1e6:.1f} "
               f"GB/s, moved {4.5625 * n / ms / 1e6:.1f} GB/s")
+    elif a.kernel == "backward":
+        from . import nvfp4_linear_cpp
+        w = outlier_weight_bf16((a.n, a.k), 8, device="cuda")
+        dy = student_t_bf16((a.m, a.n), 9, scale=1e-3, device="cuda")
+        one = torch.ones(1, device="cuda")
+        ms = _time(lambda: nvfp4_linear_cpp.backward(dy, x, w, one, one, one, True, True, True), a.warmup, a.iters)
+        N.check_status()
+        print(f"backward M={a.m} N={a.n} K={a.k}: {ms:.4f} ms, {4.0 * a.m * a.n * a.k / ms / 1e9:.1f} TFLOP/s")
     elif a.kernel == "amax_quantize":
         ms = _time(lambda: FP4Tensor.from_bfloat16(x, linear_scales=False), a.warmup, a.iters)
         print(f"amax+quantize [{a.m}, {a.k}]: {ms:.4f} ms, algorithmic {2.5625 * a.m * a.k / ms / 1e6:.1f} GB/s")

@@ -81,10 +81,10 @@ NVFP4_API int nvfp4_quantize_bf16(const void* x_bf16, int64_t rows, int64_t cols
 
 /* nvfp4_amax_bf16 and nvfp4_quantize_bf16 in one call, with the same results: amax_dev receives
  * max|x|.  One kernel for tensors of up to 262144 elements (524288 where no other form applies) and, given
- * partials, of up to some 14.5 million where rows are longer than 3072 elements (and at some shorter ones); the latter is a
- * cooperative launch: what that means beside other streams stands with nvfp4_norm_mod_bf16 below.  partials
- * (nullable): device scratch of NVFP4_AMAX_PARTIALS floats, used by this call alone; without it the maximum takes a
- * memset and a pass of its own. */
+ * partials, of up to 7.8 million where rows have 3088 to 5120 elements, of up to some 14.5 million where they are longer
+ * (and at some shorter ones); the latter two are a cooperative launch: what that means beside other streams stands with
+ * nvfp4_norm_mod_bf16 below.  partials (nullable): device scratch of NVFP4_AMAX_PARTIALS floats, used by this call
+ * alone; without it the maximum takes a memset and a pass of its own. */
 #define NVFP4_AMAX_PARTIALS 1184
 NVFP4_API int nvfp4_amax_quantize_bf16(const void* x_bf16, int64_t rows, int64_t cols, float* amax_dev,
                              uint8_t* packed, uint8_t* scales_linear, uint8_t* scales_swizzled,
